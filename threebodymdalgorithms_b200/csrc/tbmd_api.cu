@@ -4,6 +4,7 @@
 // replayed; per-step triplet counts are recorded on the device and read back once per call.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <cstdarg>
@@ -93,6 +94,13 @@ struct tbmd_ctx {
     int64_t total_items = 0;
     DevBuf partial;
     int sweep_grid = 0;
+    // no-cutoff forces of the mixed form as a product of pair tensors: the systems the plan was made
+    // for (their particle offsets), its tables on the device, panel, tile results, split positions
+    std::vector<int64_t> pt_off;
+    PtPlan pt;
+    PtDev pt_dev{};
+    DevBuf pt_tab, pt_panel, pt_slots, pt_pos;
+    int sms = 0;
 
     // P3BCA
     bool domain_set = false;
@@ -183,6 +191,8 @@ static double *energy_ptr(tbmd_ctx *c) { return c->scalars.as<double>(); }
 static unsigned long long *count_ptr(tbmd_ctx *c) { return (unsigned long long *)(c->scalars.as<char>() + 8); }
 static unsigned int *step_ptr(tbmd_ctx *c) { return (unsigned int *)(c->scalars.as<char>() + 16); }
 static unsigned int *sweep_counter(tbmd_ctx *c) { return (unsigned int *)(c->scalars.as<char>() + 24); }
+
+static unsigned int *pairs_err(tbmd_ctx *c) { return (unsigned int *)(c->scalars.as<char>() + 48); }
 
 static int sweep_R(const tbmd_ctx *ctx)
 {
@@ -288,6 +298,48 @@ static SweepWork single_sweep(tbmd_ctx *ctx)
     return SweepWork{ctx->prefix.as<int64_t>(), ctx->nblocks, ctx->total_items, sweep_counter(ctx), 1,
                      (const int64_t *)t, (const int64_t *)(t + 16), (const int64_t *)(t + 32),
                      (const int32_t *)(t + 40), ctx->prefix_kseg};
+}
+
+// Whether the no-cutoff forces of a system (or the largest of a batch) go through the pair-tensor product
+// (tbmd_pairs.cu) instead of a sweep: the mixed form's forces.  At n = 128 both take about 50 us on the
+// device (46 against 54), from there on the product is faster (n = 1000: 0.22 against 0.94 ms, 8192: 81
+// against 240 ms for AUTA and 541 for NATA); above 65,536 its panel and tile results would pass 4 GB.
+constexpr int64_t kPairsMin = 128, kPairsMax = 65536;
+static bool use_pairs(const tbmd_ctx *ctx, int64_t n, bool dual)
+{
+    return mixed(ctx) && !dual && n >= kPairsMin && n <= kPairsMax;
+}
+
+// Plan, tables and workspaces of the pair-tensor product for systems at offsets off[0 .. nsys].  The
+// panel and the tile results of one launch stay within 1 GB (one range of k where that takes more).
+static tbmd_status ensure_pairs(tbmd_ctx *ctx, const int64_t *off, int nsys)
+{
+    if (ctx->pt_off.size() == (size_t)nsys + 1 && std::memcmp(ctx->pt_off.data(), off, sizeof(int64_t) * (nsys + 1)) == 0)
+        return TBMD_OK;
+    // the tables are rewritten: a launch on a caller's stream may still read the old ones
+    CK(cudaDeviceSynchronize());
+    ctx->pt_off.clear();
+    invalidate_graph(ctx);
+    if (!ctx->sms) CK(cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device));
+    CK(pt_init());
+    pt_plan(off, nsys, ctx->sms, (size_t)1 << 30, ctx->pt);
+    const PtPlan &p = ctx->pt;
+    const size_t b_seg = sizeof(PtSeg) * p.segs.size(), b_sys = sizeof(PtSys) * p.sys.size(),
+                 b_til = sizeof(unsigned int) * p.tiles.size();
+    CK(ctx->pt_tab.ensure(b_seg + b_sys + b_til));
+    CK(ctx->pt_panel.ensure(p.mem));
+    CK(ctx->pt_slots.ensure(p.slots * pt_slot_bytes()));
+    CK(ctx->pt_pos.ensure(sizeof(float4) * 2 * (size_t)off[nsys]));
+    char *t = ctx->pt_tab.as<char>();
+    CK(cudaMemcpyAsync(t, p.segs.data(), b_seg, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(t + b_seg, p.sys.data(), b_sys, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(t + b_seg + b_sys, p.tiles.data(), b_til, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    ctx->pt_dev = PtDev{(const PtSeg *)t, (const PtSys *)(t + b_seg), (const unsigned int *)(t + b_seg + b_sys),
+                        ctx->pt_panel.as<unsigned char>(), ctx->pt_slots.as<double>(), ctx->pt_pos.as<float4>(),
+                        ctx->pt_pos.as<float4>() + off[nsys], pairs_err(ctx)};
+    ctx->pt_off.assign(off, off + nsys + 1);
+    return TBMD_OK;
 }
 
 // Cell grid for the current domain and cutoff (oracle tbo_cell_dims).
@@ -450,6 +502,10 @@ static tbmd_status prepare(tbmd_ctx *ctx, int64_t n, bool dual, bool energy)
     tbmd_status s = ensure_scalars(ctx);
     if (s != TBMD_OK) return s;
     if (is_p3bca_cut(ctx)) return ensure_cells(ctx, n, dual, energy);
+    if (use_pairs(ctx, n, dual)) {
+        const int64_t off[2] = {0, n};
+        return ensure_pairs(ctx, off, 1);
+    }
     const int alg = dual ? TBMD_AUTA : (ctx->cfg.algorithm == TBMD_NATA ? TBMD_NATA : TBMD_AUTA);
     const int R = dual ? (mixed(ctx) ? 2 : 1) : sweep_R(ctx);
     return ensure_sweep(ctx, alg, n, R, dual);
@@ -483,6 +539,16 @@ static tbmd_status enqueue_forces(tbmd_ctx *ctx, int64_t n, Pos pos, Out out, bo
         return TBMD_OK;
     }
     phase_mark(ctx, st, PH_TRIPLETS, *nl);
+    if (use_pairs(ctx, n, dual)) {
+        CK(launch_pairs(pos, out, ctx->pt, ctx->pt_dev, energy, nu, ctx->sms, st, nl));
+        phase_mark(ctx, st, PH_UPDATE, *nl);
+        if (count) {
+            k_add_u64<<<1, 1, 0, st>>>(count, choose3(n));
+            CK(cudaGetLastError());
+            *nl += 1;
+        }
+        return TBMD_OK;
+    }
     SweepWork w = single_sweep(ctx);
     CK(cudaMemsetAsync(w.counter, 0, sizeof(unsigned int), st));
     if (ctx->cfg.algorithm == TBMD_NATA && !dual) {
@@ -699,7 +765,8 @@ void tbmd_destroy(tbmd_ctx *ctx)
     for (DevBuf *b : {&ctx->state, &ctx->snapshot, &ctx->scalars, &ctx->step_counts, &ctx->prefix, &ctx->partial,
                       &ctx->cell_n, &ctx->cell_c, &ctx->nbr_buf, &ctx->dirs, &ctx->hvp, &ctx->gset_single,
                       &ctx->sweep_sys, &ctx->bpos, &ctx->bout, &ctx->bsys, &ctx->bprefix, &ctx->ncell_tab,
-                      &ctx->staging, &ctx->long_buf, &ctx->gen_buf, &ctx->bext})
+                      &ctx->staging, &ctx->long_buf, &ctx->gen_buf, &ctx->bext, &ctx->pt_tab, &ctx->pt_panel,
+                      &ctx->pt_slots, &ctx->pt_pos})
         b->release();
     if (ctx->hpin) cudaFreeHost(ctx->hpin);
     if (ctx->copy_stream) {
@@ -954,14 +1021,15 @@ struct CapSeen {
     int32_t max_count;
     uint32_t pad[3];
     uint32_t long_max;
+    uint32_t pairs_err;  // a pair-tensor launch gave up waiting
 };
-static_assert(sizeof(CapSeen) == 20, "scalars 28..48");
+static_assert(sizeof(CapSeen) == 24, "scalars 28..52");
 
 static cudaError_t reset_cap_flags(tbmd_ctx *ctx, cudaStream_t st)
 {
     cudaError_t e = cudaMemsetAsync(ctx->scalars.as<char>() + 28, 0, 4, st);
     if (e != cudaSuccess) return e;
-    return cudaMemsetAsync(ctx->scalars.as<char>() + 44, 0, 4, st);
+    return cudaMemsetAsync(ctx->scalars.as<char>() + 44, 0, 8, st);
 }
 
 static cudaError_t read_cap_flags(tbmd_ctx *ctx, cudaStream_t st, CapSeen *seen)
@@ -1061,6 +1129,7 @@ static tbmd_status run_steps(tbmd_ctx *ctx, int32_t iterations, uint64_t *counts
         if (ho) CK(cudaStreamSynchronize(ctx->copy_stream));
         const CapSeen seen = *hseen;
         phase_resolve(ctx);
+        if (seen.pairs_err) return fail(ctx, TBMD_TIMEOUT, "a wait inside the pair-tensor kernel ran out");
         if (cut && grow_caps(ctx, seen)) {
             CK(cudaMemcpyAsync(ctx->s[0], ctx->snapshot.p, sizeof(double) * 9 * n, cudaMemcpyDeviceToDevice,
                                ctx->stream));
@@ -1174,7 +1243,10 @@ tbmd_status tbmd_forces(tbmd_ctx *ctx, double *fx, double *fy, double *fz, doubl
     if (fz) CK(cudaMemcpyAsync(fz, ctx->s[12], sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(&e, energy_ptr(ctx), sizeof e, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(&c, count_ptr(ctx), sizeof c, cudaMemcpyDeviceToHost, ctx->stream));
+    CapSeen seen{};
+    CK(read_cap_flags(ctx, ctx->stream, &seen));
     CK(cudaStreamSynchronize(ctx->stream));
+    if (seen.pairs_err) return fail(ctx, TBMD_TIMEOUT, "a wait inside the pair-tensor kernel ran out");
     if (energy) *energy = e;
     if (triplets) *triplets = c;
     return TBMD_OK;
@@ -1419,6 +1491,8 @@ extern "C" tbmd_status tbmd_autotune(tbmd_ctx *ctx, const char *cache_path)
     std::vector<std::pair<int, int>> cand;
     if (is_p3bca_cut(ctx)) {
         for (int w : {2, 4, 8}) cand.push_back({R, w});
+    } else if (use_pairs(ctx, ctx->n, false)) {
+        cand.push_back({R, warps});  // the pair-tensor product has no variants
     } else {
         for (int r : {1, 2, 4}) cand.push_back({r, warps});
     }
@@ -1537,6 +1611,8 @@ static tbmd_status batch_eval(tbmd_ctx *ctx, int32_t nsys, const int64_t *offset
     const Out out{O, O + N, O + 2 * N, O + 3 * N, O + 4 * N, O + 5 * N};
     res.counts.assign(nsys, 0);
     int nl = 0;
+    int64_t nmax = 0;
+    for (int s = 0; s < nsys; ++s) nmax = std::max(nmax, offsets[s + 1] - offsets[s]);
 
     if (is_p3bca_cut(ctx)) {
         // per-system grids: the given box, or the reference's domain rule on that system's positions
@@ -1625,6 +1701,16 @@ static tbmd_status batch_eval(tbmd_ctx *ctx, int32_t nsys, const int64_t *offset
         CK(cudaMemcpyAsync(c.data(), CNT, sizeof(unsigned long long) * nsys, cudaMemcpyDeviceToHost, sm));
         CK(cudaStreamSynchronize(sm));
         for (int s = 0; s < nsys; ++s) res.counts[s] = c[s];
+    } else if (!dual && mx && N >= kPairsMin && nmax <= kPairsMax) {
+        CK(reset_cap_flags(ctx, sm));
+        st = ensure_pairs(ctx, offsets, nsys);
+        if (st != TBMD_OK) return st;
+        CK(launch_pairs(pos, out, ctx->pt, ctx->pt_dev, E, nu, ctx->sms, sm, &nl));
+        CapSeen seen{};
+        CK(read_cap_flags(ctx, sm, &seen));
+        CK(cudaStreamSynchronize(sm));
+        if (seen.pairs_err) return fail(ctx, TBMD_TIMEOUT, "a wait inside the pair-tensor kernel ran out");
+        for (int s = 0; s < nsys; ++s) res.counts[s] = choose3(offsets[s + 1] - offsets[s]);
     } else {
         // one sweep over all systems (AUTA work items; NATA gives the same forces)
         const int R = dual ? (mx ? 2 : 1) : (mx ? ctx->R_auta : ctx->R_fp64);

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "at_math.cuh"
 
 namespace tbmd {
@@ -329,6 +331,52 @@ cudaError_t launch_auta(bool mixed, bool dual, int R, bool energy, int64_t n, Po
 cudaError_t launch_nata(bool mixed, bool dual, int R, bool energy, int64_t n, Pos pos, Out out, double *energy_out,
                         double nu, SweepWork work, double *partial, int grid, cudaStream_t st);
 cudaError_t launch_nata_reduce(bool dual, int64_t n, int nblocks, const double *partial, Out out, cudaStream_t st);
+
+// No-cutoff forces of the mixed form as a product of pair tensors (tbmd_pairs.cu).  A segment is one
+// system's range of k; an item is one tile of one segment.  Offsets are within the group (one launch).
+struct PtSeg {
+    int64_t mem;    // bytes into the panel
+    int64_t item0;  // first item
+    int64_t slot0;  // first tile result
+    int32_t part0, n;   // the system's first particle and size
+    int32_t k0, nslab;  // first particle of the range, its slabs of 32 matrix columns
+    int32_t tab;        // first entry of the system's tile order
+    int32_t gen0;       // first block of the panel kernel
+};
+struct PtSys {
+    int64_t part0, slot0;
+    int32_t n, nb2, nseg, index;  // size, column blocks, segments in this group, system
+    int32_t add;                  // 1: an earlier group holds the system's first segments
+    int32_t pad;
+};
+struct PtGroup {
+    int seg0, nsegs, sys0, nsys;
+    size_t mem;
+    int64_t items, slots;
+    int gen;
+};
+struct PtPlan {
+    std::vector<PtSeg> segs;
+    std::vector<PtSys> sys;
+    std::vector<unsigned int> tiles;
+    std::vector<PtGroup> groups;
+    size_t mem = 0, slots = 0;  // largest group's panel bytes and tile results
+};
+struct PtDev {
+    const PtSeg *segs;
+    const PtSys *sys;
+    const unsigned int *tiles;
+    unsigned char *panel;
+    double *slots;
+    float4 *qhi, *qlo;  // split positions
+    unsigned int *err;  // set by a launch that gave up waiting
+};
+void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, PtPlan &plan);
+size_t pt_slot_bytes();
+cudaError_t pt_init();
+// forces overwritten; energy (one accumulator per system, may be NULL) added to
+cudaError_t launch_pairs(Pos pos, Out out, const PtPlan &plan, const PtDev &d, double *energy,
+                         double nu, int sms, cudaStream_t st, int *launches);
 
 // P3BCA pipeline
 // Half-list chunk of the P3BCA triplet kernel: lists of at most P3_CHUNK entries are one work item,

@@ -1,0 +1,701 @@
+// No-cutoff forces and energy of the mixed form as a matrix product on the tensor cores.
+//
+// With the pair tensors T_ij = (3 r r^T - r^2) / r^5 (r = x_j - x_i, symmetric, traceless, T_ii = 0) the
+// Axilrod-Teller energy of a triplet is -nu/3 tr(T_ij T_jk T_ki), so over all triplets
+//   E   = -nu/18 tr(T^3)                             (T: the symmetric 3n x 3n matrix of the 3x3 blocks)
+//   f_i = +dE/dx_i = nu/3 sum_j (G_ij : dT_ij/dr),   G = T T,   G_ij = sum_k T_ik T_kj
+// which is the same sum over i < j < k as the pairwise sweeps (the blocks T_ii = 0 leave out repeated
+// indices).  G is a dense product of 27 n^3 FLOP over i < j; the rest is O(n^2).
+//
+//   k_pt_split   positions relative to the system's first particle as FP32 hi + lo parts
+//   k_pt_panel   T for a range of k, formed in FP64 and split exactly into three bfloat16 (h + m + l holds
+//                26 bits), written in the layout the matrix unit reads from shared memory
+//   k_pt_gemm    tiles of G (42 x 84 particles) by tcgen05.mma, contracted with dT/dr in the same kernel
+//   k_pt_reduce  each particle's force from its tiles, in a fixed order (deterministic)
+//
+// Bound: the tensor cores at the power cap for large n (n = 8192: 9.4e13 FLOP of bf16 in 81 ms, 1.16 PFLOP/s
+// of 1.36 sustained by cuBLAS; AUTA's FP32 sweep took 240 ms, NATA's 541), the operands' way from L2 for
+// medium n (a slab of 72 KB in 2,100 cycles, 1,536 of them product; n = 4096: 9.5 ms against 31.5 and 79).
+// A tile of 128 x 256 is the largest whose FP32 sums fit the registers (128 a thread in eight warps) beside
+// two accumulators of 256 TMEM columns, one filling while the other is added up.
+//
+// Accuracy.  Six products of the splits are kept (hh, hm, mh, mm, hl, lh; the rest is below 2^-26), each
+// exact in FP32.  The tensor core adds into an FP32 accumulator that it truncates, so an accumulator only
+// lives for 32 columns of T: the ten small products go first, the two hh steps last, and the tile is then
+// added to FP32 registers with rounding.  After 256 particles at most the registers are contracted and the
+// forces go on in FP64.  Relative L2 error of the forces against FP64, thermal lattices of 512 .. 8192
+// particles: 2.0e-7 .. 2.6e-7 (the FP32 sweeps: 2.3e-7 .. 2.6e-7).  No step subtracts nearly equal numbers: a pair's force needs no difference of
+// large terms even where two of the three particles nearly coincide.
+#include <cuda_bf16.h>
+
+#include <algorithm>
+
+#include "tbmd_internal.cuh"
+
+namespace tbmd {
+
+constexpr int PT_PART = 42;                 // particles of a row block: 126 of 128 matrix rows
+constexpr int PT_ROWS = 128;
+constexpr int PT_SLAB_K = 32;               // matrix columns of one slab (one pipeline stage)
+constexpr int PT_SPLIT_BYTES = PT_ROWS * PT_SLAB_K * 2;  // one split of a row block's slab: 8 KB
+constexpr int PT_BLOCK_BYTES = 3 * PT_SPLIT_BYTES;       // all three: 24 KB, contiguous in the panel
+constexpr int PT_STAGE_BYTES = 3 * PT_BLOCK_BYTES;       // one row block (A) and two (B)
+constexpr int PT_STAGES = 3;
+constexpr int PT_WARPS = 12;                // 8 accumulate and contract, 1 loads, 1 issues the products, 2 idle
+constexpr int PT_SLOT = 3 * PT_PART * 3 + 2;  // doubles of a tile's results: f_i, f_j (two blocks), energy, pad
+
+struct PtShared {
+    unsigned char stage[PT_STAGES][PT_STAGE_BYTES];
+    double fi[2][PT_ROWS][3];
+    float fj[8][PT_ROWS];
+    double e[8];
+    unsigned long long full[PT_STAGES], empty[PT_STAGES], acc_full[2], acc_empty[2], drained;
+    unsigned int tmem;
+    int dead;
+};
+
+__device__ __forceinline__ unsigned int smem_u32(const void *p) { return (unsigned int)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void bar_init(unsigned long long *b, unsigned int count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(unsigned long long *b)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
+}
+__device__ __forceinline__ void bar_expect(unsigned long long *b, unsigned int bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool bar_try(unsigned long long *b, unsigned int parity)
+{
+    unsigned int ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(b)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ unsigned long long now_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+// Every wait ends: after two seconds it marks the block dead and the launch failed (*err); from then on
+// waits return at once, no copy or product is issued, and the loops run out.
+__device__ __forceinline__ bool bar_wait(unsigned long long *b, unsigned int parity, PtShared &S, unsigned int *err)
+{
+    if (bar_try(b, parity)) return true;
+    const unsigned long long t0 = now_ns();
+    for (unsigned int n = 1;; ++n) {
+        if (bar_try(b, parity)) return true;
+        if ((n & 63u) == 0u) {
+            if (*(volatile int *)&S.dead) return false;
+            if (now_ns() - t0 > 2000000000ull) {
+                *(volatile int *)&S.dead = 1;
+                atomicExch(err, 1u);
+                return false;
+            }
+        }
+    }
+}
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned int bytes, unsigned long long *b)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(b))
+                 : "memory");
+}
+// Shared-memory descriptor of an operand stored without swizzle, K contiguous in 16-byte chunks: the next
+// chunk of 8 columns is 128 bytes on, the next group of 8 rows 512.
+__device__ __forceinline__ unsigned long long operand_desc(unsigned int addr)
+{
+    return (unsigned long long)((addr >> 4) & 0x3fffu) | (unsigned long long)(128 >> 4) << 16 |
+           (unsigned long long)(512 >> 4) << 32 | 1ull << 46;
+}
+// D FP32, A and B bfloat16, both K-major, 128 x 256
+constexpr unsigned int PT_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | ((128u >> 4) << 24);
+__device__ __forceinline__ void mma_bf16(unsigned int d, unsigned long long a, unsigned long long b, unsigned int acc)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d), "l"(a), "l"(b), "r"(PT_IDESC), "r"(acc)
+        : "memory");
+}
+__device__ __forceinline__ void mma_commit(unsigned long long *b)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(b))
+                 : "memory");
+}
+#define TM_LD32(v, addr)                                                                                       \
+    asm volatile(                                                                                                 \
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,"  \
+        "%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"                                        \
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]),             \
+          "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]),       \
+          "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]), "=f"(v[17]),   \
+          "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]),   \
+          "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]),   \
+          "=f"(v[30]), "=f"(v[31])                                                                        \
+        : "r"(addr))
+// the loaded registers hold their values from here on
+#define TM_WAIT32(v)                                                                                              \
+    asm volatile("tcgen05.wait::ld.sync.aligned;"                                                                 \
+                 : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]),   \
+                   "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]),         \
+                   "+f"(v[15]), "+f"(v[16]), "+f"(v[17]), "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]),       \
+                   "+f"(v[22]), "+f"(v[23]), "+f"(v[24]), "+f"(v[25]), "+f"(v[26]), "+f"(v[27]), "+f"(v[28]),       \
+                   "+f"(v[29])                                                                                    \
+                 :                                                                                                \
+                 : "memory");                                                                                     \
+    asm volatile("" : "+f"(v[30]), "+f"(v[31]))
+
+// system of particle p (of the group's, in ascending order)
+__device__ __forceinline__ int pt_system(const PtSys *sys, int nsys, int64_t p)
+{
+    int lo = 0, hi = nsys;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (sys[mid].part0 <= p)
+            lo = mid;
+        else
+            hi = mid;
+    }
+    return lo;
+}
+
+// segment holding index w of an ascending field
+template <class F>
+__device__ __forceinline__ int pt_find(const PtSeg *seg, int nseg, int64_t w, F field)
+{
+    int lo = 0, hi = nseg;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (field(seg[mid]) <= w)
+            lo = mid;
+        else
+            hi = mid;
+    }
+    return lo;
+}
+
+// Positions relative to the system's first particle as FP32 hi + lo parts.
+__global__ void k_pt_split(Pos pos, const PtSys *__restrict__ sys, int nsys, int64_t p0, int64_t n, float4 *qhi,
+                           float4 *qlo)
+{
+    const int64_t p = p0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= p0 + n) return;
+    const int64_t o = sys[pt_system(sys, nsys, p)].part0;
+    float hx, hy, hz, lx, ly, lz;
+    split<float>(pos.x[p] - pos.x[o], 0.0, hx, lx);
+    split<float>(pos.y[p] - pos.y[o], 0.0, hy, ly);
+    split<float>(pos.z[p] - pos.z[o], 0.0, hz, lz);
+    qhi[p] = make_float4(hx, hy, hz, 0.f);
+    qlo[p] = make_float4(lx, ly, lz, 0.f);
+}
+
+// The three bfloat16 parts of v, as 16-bit patterns: v = h + m + l to 2^-27 of |v|.
+__device__ __forceinline__ void split3(double v, unsigned short &h, unsigned short &m, unsigned short &l)
+{
+    const __nv_bfloat16 bh = __float2bfloat16_rn((float)v);
+    const float r1 = (float)(v - (double)__bfloat162float(bh));
+    const __nv_bfloat16 bm = __float2bfloat16_rn(r1);
+    const __nv_bfloat16 bl = __float2bfloat16_rn(r1 - __bfloat162float(bm));
+    h = __bfloat16_as_ushort(bh);
+    m = __bfloat16_as_ushort(bm);
+    l = __bfloat16_as_ushort(bl);
+}
+
+// One block: a row block (42 particles) against 32 particles k (three slabs).  A thread holds one particle
+// i and 8 particles k: 24 columns of its three rows, three 16-byte chunks per row and split.  The stores
+// are 16-byte pieces that L2 merges; the panel is 0.4% of the product's time at n = 8192.
+constexpr int PT_PANEL_THREADS = 192;
+__global__ void __launch_bounds__(PT_PANEL_THREADS) k_pt_panel(Pos pos, const PtSeg *__restrict__ seg, int nseg,
+                                                              unsigned char *__restrict__ panel)
+{
+    const PtSeg s = seg[pt_find(seg, nseg, (int64_t)blockIdx.x, [](const PtSeg &q) { return (int64_t)q.gen0; })];
+    const int groups = s.nslab / 3;
+    const int task = (int)blockIdx.x - s.gen0;
+    const int rb = task / groups, kg = task - rb * groups;
+    const int il = threadIdx.x % 48, oct = threadIdx.x / 48;
+    if (il > PT_PART) return;
+    const int i = rb * PT_PART + il;
+    const bool row_ok = il < PT_PART && i < s.n;
+    double xi = 0.0, yi = 0.0, zi = 0.0;
+    if (row_ok) {
+        xi = pos.x[s.part0 + i];
+        yi = pos.y[s.part0 + i];
+        zi = pos.z[s.part0 + i];
+    }
+    // packed bfloat16 pairs of the 24 columns: [split][row a][12 words]
+    unsigned int w[3][3][12];
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int c = 0; c < 12; ++c) w[q][a][c] = 0u;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const int k = s.k0 + kg * 32 + oct * 8 + e;
+        double t[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // xx xy xz yy yz zz
+        if (row_ok && k < s.n && k != i) {
+            const double x = pos.x[s.part0 + k] - xi, y = pos.y[s.part0 + k] - yi, z = pos.z[s.part0 + k] - zi;
+            const double ri = rsqrt(fma(x, x, fma(y, y, z * z)));
+            const double ri2 = ri * ri, i3 = ri * ri2, s5 = 3.0 * i3 * ri2;
+            t[0] = fma(s5 * x, x, -i3);
+            t[1] = s5 * x * y;
+            t[2] = s5 * x * z;
+            t[3] = fma(s5 * y, y, -i3);
+            t[4] = s5 * y * z;
+            t[5] = fma(s5 * z, z, -i3);
+        }
+        constexpr int at[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
+#pragma unroll
+        for (int c = 0; c < 6; ++c) {
+            unsigned short p[3];
+            split3(t[c], p[0], p[1], p[2]);
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int b = 0; b < 3; ++b)
+                    if (at[a][b] == c) {
+                        const int col = 3 * e + b;
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) w[q][a][col >> 1] |= (unsigned int)p[q] << ((col & 1) * 16);
+                    }
+        }
+    }
+    unsigned char *base = panel + s.mem + ((int64_t)rb * s.nslab + kg * 3) * PT_BLOCK_BYTES;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const int row = 3 * il + a;
+        if (row >= PT_ROWS) continue;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int chunk = oct * 3 + c;  // of the group's 12
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                unsigned char *dst = base + (chunk >> 2) * PT_BLOCK_BYTES + q * PT_SPLIT_BYTES + (row >> 3) * 512 +
+                                     (chunk & 3) * 128 + (row & 7) * 16;
+                *(uint4 *)dst = make_uint4(w[q][a][4 * c], w[q][a][4 * c + 1], w[q][a][4 * c + 2], w[q][a][4 * c + 3]);
+            }
+        }
+    }
+}
+
+// One item: a tile (row block a, column blocks 2 b and 2 b + 1) of G over one segment's k.
+struct PtItem {
+    PtSeg s;
+    int a, b;
+};
+__device__ __forceinline__ PtItem pt_item(const PtSeg *seg, int nseg, const unsigned int *tiles, int64_t w)
+{
+    PtItem it;
+    it.s = seg[pt_find(seg, nseg, w, [](const PtSeg &q) { return q.item0; })];
+    const unsigned int t = tiles[it.s.tab + (w - it.s.item0)];
+    it.a = (int)(t >> 16);
+    it.b = (int)(t & 0xffffu);
+    return it;
+}
+
+__global__ void __launch_bounds__(PT_WARPS * 32, 1)
+    k_pt_gemm(const PtSeg *__restrict__ seg, int nseg, int64_t items, const unsigned int *__restrict__ tiles,
+              const unsigned char *__restrict__ panel, const float4 *__restrict__ qhi, const float4 *__restrict__ qlo,
+              double *__restrict__ slots, double nu, unsigned int *err)
+{
+    extern __shared__ __align__(1024) unsigned char smraw[];
+    PtShared &S = *(PtShared *)smraw;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < PT_STAGES; ++k) {
+            bar_init(&S.full[k], 1);
+            bar_init(&S.empty[k], 1);
+        }
+        for (int k = 0; k < 2; ++k) {
+            bar_init(&S.acc_full[k], 1);
+            bar_init(&S.acc_empty[k], 8);
+        }
+        bar_init(&S.drained, 1);
+        S.dead = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 9) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&S.tmem))
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const unsigned int tmem = S.tmem;
+
+    // registers: 168 x 384 at launch = 216 x 256 + 72 x 128
+    if (warp >= 8) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+        if (warp == 8 && lane == 0) {
+            unsigned int n = 0;  // slabs loaded
+            for (int64_t w = blockIdx.x; w < items; w += gridDim.x) {
+                const PtItem it = pt_item(seg, nseg, tiles, w);
+                const int64_t row = (int64_t)it.s.nslab * PT_BLOCK_BYTES;
+                const unsigned char *pa = panel + it.s.mem + it.a * row, *pb = panel + it.s.mem + 2 * it.b * row;
+                for (int k = 0; k < it.s.nslab; ++k, ++n) {
+                    const int st = n % PT_STAGES;
+                    if (!bar_wait(&S.empty[st], ((n / PT_STAGES) & 1) ^ 1, S, err)) break;
+                    unsigned char *dst = S.stage[st];
+                    bar_expect(&S.full[st], PT_STAGE_BYTES);
+                    bulk_load(dst, pa + (int64_t)k * PT_BLOCK_BYTES, PT_BLOCK_BYTES, &S.full[st]);
+                    // B: the splits of the two row blocks side by side, 256 rows each
+                    for (int q = 0; q < 3; ++q)
+                        for (int h = 0; h < 2; ++h)
+                            bulk_load(dst + PT_BLOCK_BYTES + (2 * q + h) * PT_SPLIT_BYTES,
+                                      pb + h * row + (int64_t)k * PT_BLOCK_BYTES + q * PT_SPLIT_BYTES, PT_SPLIT_BYTES,
+                                      &S.full[st]);
+                }
+                if (*(volatile int *)&S.dead) break;
+            }
+            // a block that gave up leaves no copy in flight behind it
+            if (*(volatile int *)&S.dead)
+                for (unsigned int k = n > PT_STAGES ? n - PT_STAGES : 0; k < n; ++k) {
+                    const unsigned long long t0 = now_ns();
+                    while (!bar_try(&S.full[k % PT_STAGES], (k / PT_STAGES) & 1) && now_ns() - t0 < 100000000ull) {
+                    }
+                }
+        }
+        if (warp == 9 && lane == 0) {
+            unsigned int n = 0;
+            bool ok = true;
+            for (int64_t w = blockIdx.x; ok && w < items; w += gridDim.x) {
+                const PtItem it = pt_item(seg, nseg, tiles, w);
+                for (int k = 0; k < it.s.nslab; ++k, ++n) {
+                    const int st = n % PT_STAGES, buf = n & 1;
+                    ok = bar_wait(&S.acc_empty[buf], ((n >> 1) & 1) ^ 1, S, err) &&
+                         bar_wait(&S.full[st], (n / PT_STAGES) & 1, S, err);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const unsigned int A = smem_u32(S.stage[st]), B = A + PT_BLOCK_BYTES, D = tmem + buf * 256;
+                    // the small products first (l h, h l, m m, m h, h m), h h last
+                    constexpr int qa[6] = {2, 0, 1, 1, 0, 0}, qb[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+                    for (int p = 0; p < 6; ++p)
+#pragma unroll
+                        for (int kk = 0; kk < 2; ++kk)
+                            mma_bf16(D, operand_desc(A + qa[p] * PT_SPLIT_BYTES + kk * 256),
+                                     operand_desc(B + qb[p] * 2 * PT_SPLIT_BYTES + kk * 256), p + kk > 0);
+                    mma_commit(&S.empty[st]);
+                    mma_commit(&S.acc_full[buf]);
+                }
+            }
+            if (!ok) {  // products in flight end before the accumulators are given back
+                mma_commit(&S.drained);
+                const unsigned long long t0 = now_ns();
+                while (!bar_try(&S.drained, 0) && now_ns() - t0 < 100000000ull) {
+                }
+            }
+        }
+        __syncwarp();
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+        const int quad = warp & 3, half = warp >> 2;
+        const int row = quad * 32 + lane, ip = row / 3, al = row - 3 * ip;
+        const float ex = al == 0 ? 1.f : 0.f, ey = al == 1 ? 1.f : 0.f, ez = al == 2 ? 1.f : 0.f;
+        const unsigned int taddr = tmem + ((unsigned int)(quad * 32) << 16) + half * 128;
+        unsigned int n = 0;
+        for (int64_t w = blockIdx.x; w < items; w += gridDim.x) {
+            const PtItem it = pt_item(seg, nseg, tiles, w);
+            float g[128];
+#pragma unroll
+            for (int c = 0; c < 128; ++c) g[c] = 0.f;
+            for (int k = 0; k < it.s.nslab; ++k, ++n) {
+                const int buf = n & 1;
+                if (!bar_wait(&S.acc_full[buf], (n >> 1) & 1, S, err)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    float t[32];
+                    TM_LD32(t, taddr + buf * 256 + c * 32);
+                    TM_WAIT32(t);
+#pragma unroll
+                    for (int q = 0; q < 32; ++q) g[c * 32 + q] += t[q];
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                if (lane == 0) bar_arrive(&S.acc_empty[buf]);
+            }
+            // contraction: this thread's row (i, al) of G against dT_ij/dr for the 42 particles j of its
+            // column block; with g the row of G_ij, y = g.r and the unit vector e of the row, its part of
+            // G_ij : dT/dr is 3 / r^5 (y e + r_al g + (g_al - 5 r_al y / r^2) r)
+            const int i = it.a * PT_PART + ip, j0 = (2 * it.b + half) * PT_PART;
+            const bool iv = row < 3 * PT_PART && i < it.s.n;
+            const float4 ih = qhi[it.s.part0 + (iv ? i : 0)], il = qlo[it.s.part0 + (iv ? i : 0)];
+            double fx = 0.0, fy = 0.0, fz = 0.0, en = 0.0;
+#pragma unroll
+            for (int j6 = 0; j6 < PT_PART; j6 += 6) {
+                float sx = 0.f, sy = 0.f, sz = 0.f, se = 0.f;
+#pragma unroll
+                for (int jj = j6; jj < j6 + 6; ++jj) {
+                    const int j = j0 + jj, jc = it.s.part0 + min(j, it.s.n - 1);
+                    const float4 jh = __ldg(qhi + jc), jl = __ldg(qlo + jc);
+                    // r and what its rounding left out (the difference of the hi parts of near particles is exact)
+                    const float ax = jh.x - ih.x, ay = jh.y - ih.y, az = jh.z - ih.z;
+                    const float bx = jl.x - il.x, by = jl.y - il.y, bz = jl.z - il.z;
+                    const float rx = ax + bx, ry = ay + by, rz = az + bz;
+                    const float cx = bx - (rx - ax), cy = by - (ry - ay), cz = bz - (rz - az);
+                    const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+                    const float rc = fmaf(rx, cx, fmaf(ry, cy, rz * cz));
+                    // r^-5 = t^5 (1 + 5/2 e) with t the approximate r^-1 and e = 1 - r^2 t^2 (t^2 as s + sl)
+                    float t = rsqrt_(r2);
+                    if (!(iv && i < j && j < it.s.n)) t = 0.f;
+                    const float s = t * t, sl = fmaf(t, t, -s);
+                    float e = fmaf(-2.f * rc, s, fmaf(-r2, sl, fmaf(-r2, s, 1.f)));
+                    float i5 = s * s * t;
+                    i5 = fmaf(2.5f * e, i5, i5);
+                    const float ri2 = fmaf(e, s, s);
+                    const float gx = g[3 * jj], gy = g[3 * jj + 1], gz = g[3 * jj + 2];
+                    const float y = fmaf(gx, rx, fmaf(gy, ry, gz * rz));
+                    const float ra = fmaf(ex, rx, fmaf(ey, ry, ez * rz)), ga = fmaf(ex, gx, fmaf(ey, gy, ez * gz));
+                    const float ray = ra * y;
+                    const float sc = fmaf(-5.f * ri2, ray, ga);
+                    const float vx = fmaf(ex, y, fmaf(ra, gx, sc * rx)) * i5;
+                    const float vy = fmaf(ey, y, fmaf(ra, gy, sc * ry)) * i5;
+                    const float vz = fmaf(ez, y, fmaf(ra, gz, sc * rz)) * i5;
+                    sx += vx;
+                    sy += vy;
+                    sz += vz;
+                    se += i5 * fmaf(3.f, ray, -(ga * r2));  // row al of G_ij : T_ij
+                    g[3 * jj] = vx;
+                    g[3 * jj + 1] = vy;
+                    g[3 * jj + 2] = vz;
+                }
+                fx += (double)sx;
+                fy += (double)sy;
+                fz += (double)sz;
+                en += (double)se;
+            }
+            g[126] = g[127] = 0.f;
+            // f_j: sums over the warp's 32 rows, 4 columns left per lane
+#pragma unroll
+            for (int o = 16, m = 64; o >= 1; o >>= 1, m >>= 1) {
+                const bool up = (lane & o) != 0;
+#pragma unroll
+                for (int q = 0; q < 64; ++q)
+                    if (q < m) {
+                        const float keep = up ? g[q + m] : g[q], send = up ? g[q] : g[q + m];
+                        g[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                    }
+            }
+            const int col = ((lane >> 4) & 1) * 64 + ((lane >> 3) & 1) * 32 + ((lane >> 2) & 1) * 16 +
+                            ((lane >> 1) & 1) * 8 + (lane & 1) * 4;
+            *(float4 *)&S.fj[warp][col] = make_float4(g[0], g[1], g[2], g[3]);
+            S.fi[half][row][0] = fx;
+            S.fi[half][row][1] = fy;
+            S.fi[half][row][2] = fz;
+            en = warp_sum(en);
+            if (lane == 0) S.e[warp] = en;
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            double *slot = slots + (it.s.slot0 + (int64_t)it.b * (it.b + 1) + it.a) * PT_SLOT;
+            const int t = threadIdx.x;
+            if ((t & 127) < 126) {
+                double v = 0.0;
+                for (int q = 0; q < 4; ++q) v += (double)S.fj[(t >> 7) * 4 + q][t & 127];
+                slot[126 + (t >> 7) * 126 + (t & 127)] = -nu * v;
+            }
+            if (t < 126) {
+                const int p = t / 3, c = t - 3 * p;
+                double v = 0.0;
+                for (int h = 0; h < 2; ++h)
+                    for (int q = 0; q < 3; ++q) v += S.fi[h][3 * p + q][c];
+                slot[t] = nu * v;
+            }
+            if (t == 255) {
+                double v = 0.0;
+                for (int q = 0; q < 8; ++q) v += S.e[q];
+                slot[378] = -nu * v / 9.0;
+            }
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 9)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+}
+
+// Forces from the tiles' results: particle i of row block a sums the tiles (a, b) of its row and the tiles
+// (a', a / 2) of its column, over the system's segments.  A warp per particle; the lanes' sums and their
+// tree have a fixed order.  A system whose panels did not fit one launch is added up over launches.  A
+// launch that gave up gives NaN.
+__global__ void k_pt_reduce(int64_t p0, int64_t n, const PtSys *__restrict__ sys, int nsys, const double *__restrict__ slots, Out out,
+                            const unsigned int *__restrict__ err)
+{
+    const int64_t p = p0 + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    const int lane = threadIdx.x & 31;
+    if (p >= p0 + n) return;
+    const PtSys s = sys[pt_system(sys, nsys, p)];
+    const int i = (int)(p - s.part0), a = i / PT_PART, il = i - a * PT_PART;
+    const int b0 = a >> 1, rows = s.nb2 - b0, cols = 2 * b0 + 2, per = s.nb2 * (s.nb2 + 1);
+    double f[3] = {0.0, 0.0, 0.0};
+    for (int q = lane; q < s.nseg * (rows + cols); q += 32) {
+        const int sg = q / (rows + cols), r = q - sg * (rows + cols);
+        const int b = r < rows ? b0 + r : b0, ta = r < rows ? a : r - rows;
+        const double *src = slots + (s.slot0 + (int64_t)sg * per + (int64_t)b * (b + 1) + ta) * PT_SLOT +
+                            (r < rows ? 3 * il : 126 * (1 + (a & 1)) + 3 * il);
+        f[0] += src[0];
+        f[1] += src[1];
+        f[2] += src[2];
+    }
+    const bool bad = *err != 0u;
+    for (int c = 0; c < 3; ++c) f[c] = warp_sum(f[c]);
+    if (lane == 0) {
+        const double nan = __longlong_as_double(0x7ff8000000000000ll);
+        out.fx[p] = bad ? nan : (s.add ? out.fx[p] : 0.0) + f[0];
+        out.fy[p] = bad ? nan : (s.add ? out.fy[p] : 0.0) + f[1];
+        out.fz[p] = bad ? nan : (s.add ? out.fz[p] : 0.0) + f[2];
+    }
+}
+
+// Energy of each system: its tiles' energies, a block per system, in a fixed order.  Adds to energy[s]
+// (the caller zeroes it).
+__global__ void __launch_bounds__(512) k_pt_energy(const PtSys *__restrict__ sys, const double *__restrict__ slots,
+                                                   double *energy)
+{
+    __shared__ double part[16];
+    const PtSys s = sys[blockIdx.x];
+    const int64_t total = (int64_t)s.nseg * s.nb2 * (s.nb2 + 1);
+    double e = 0.0;
+    for (int64_t q = threadIdx.x; q < total; q += 512) e += slots[(s.slot0 + q) * PT_SLOT + 378];
+    e = warp_sum(e);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = e;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 16; ++k) e += part[k];
+        energy[s.index] += e;
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// Work lists (host)
+
+// Tile order of nb2 column blocks: strips of 8 column blocks, walked row by row, so that the tiles in
+// flight (one per SM) share row and column blocks in L2 (18 + 16 blocks of 1.1 MB at 512 k).
+static void pt_tiles(int nb2, std::vector<unsigned int> &out)
+{
+    for (int b0 = 0; b0 < nb2; b0 += 8) {
+        const int b1 = std::min(nb2, b0 + 8);
+        for (int a = 0; a < 2 * b1; ++a)
+            for (int b = std::max(b0, a >> 1); b < b1; ++b) out.push_back((unsigned int)a << 16 | (unsigned int)b);
+    }
+}
+
+// Particles k of one item: the range length with the least estimated time of all items, at 2,100 cycles a
+// slab (the product alone is 1,536; the rest is the operands' way through L2) and 10,000 an item (set-up,
+// contraction).  256 at most, for the accuracy of the FP32 sums over a range: with 512 (n = 8192: 73 ms
+// against 81) the forces' error was 5% above the pairwise sweep's at n = 2048 .. 6500.
+static int pt_range(const int64_t *sys_off, int nsys, int sms)
+{
+    int best = 256;
+    double least = 0.0;
+    for (int kp : {256, 192, 128, 96, 64, 32}) {
+        int64_t items = 0;
+        double slabs = 0.0;
+        for (int s = 0; s < nsys; ++s) {
+            const int64_t n = sys_off[s + 1] - sys_off[s], nb2 = (n + 2 * PT_PART - 1) / (2 * PT_PART);
+            items += nb2 * (nb2 + 1) * ((n + kp - 1) / kp);
+            slabs += (double)(nb2 * (nb2 + 1)) * (double)((n + 31) / 32 * 3);
+        }
+        const double t = (double)((items + sms - 1) / sms) * (slabs / (double)(items ? items : 1) * 2100.0 + 10000.0);
+        if (kp == 256 || t < 0.98 * least) {
+            least = t;
+            best = kp;
+        }
+    }
+    return best;
+}
+
+// Panels, tiles and results of all systems, in groups whose panel and results stay within `budget` bytes
+// (a group has at least one range); a system may go over several groups.
+void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, PtPlan &plan)
+{
+    plan = PtPlan{};
+    const int kp = pt_range(sys_off, nsys, sms);
+    PtGroup g{};
+    for (int s = 0; s < nsys; ++s) {
+        const int64_t n = sys_off[s + 1] - sys_off[s];
+        if (n < 1) continue;
+        const int nb2 = (int)((n + 2 * PT_PART - 1) / (2 * PT_PART));
+        const int64_t tiles = (int64_t)nb2 * (nb2 + 1);
+        const int tab = (int)plan.tiles.size();
+        pt_tiles(nb2, plan.tiles);
+        PtSys sy{sys_off[s], g.slots, (int)n, nb2, 0, s, 0, 0};
+        auto end_system = [&]() {
+            if (!sy.nseg) return;
+            plan.sys.push_back(sy);
+            ++g.nsys;
+        };
+        for (int64_t k0 = 0; k0 < n; k0 += kp) {
+            const int nslab = ((int)std::min<int64_t>(kp, n - k0) + 31) / 32 * 3;
+            const size_t mem = (size_t)nb2 * 2 * nslab * PT_BLOCK_BYTES;
+            if (g.nsegs && g.mem + mem + (size_t)(g.slots + tiles) * PT_SLOT * sizeof(double) > budget) {
+                end_system();
+                plan.groups.push_back(g);
+                g = PtGroup{};
+                g.seg0 = (int)plan.segs.size();
+                g.sys0 = (int)plan.sys.size();
+                sy.slot0 = 0;
+                sy.add = k0 > 0;
+                sy.nseg = 0;
+            }
+            plan.segs.push_back(PtSeg{(int64_t)g.mem, g.items, g.slots, (int)sys_off[s], (int)n, (int)k0, nslab, tab,
+                                      g.gen});
+            g.mem += mem;
+            g.items += tiles;
+            g.slots += tiles;
+            g.gen += 2 * nb2 * (nslab / 3);
+            ++g.nsegs;
+            ++sy.nseg;
+        }
+        end_system();
+    }
+    if (g.nsegs) plan.groups.push_back(g);
+    for (const PtGroup &q : plan.groups) {
+        plan.mem = std::max(plan.mem, q.mem);
+        plan.slots = std::max(plan.slots, (size_t)q.slots);
+    }
+}
+
+size_t pt_slot_bytes() { return PT_SLOT * sizeof(double); }
+
+cudaError_t pt_init()
+{
+    return cudaFuncSetAttribute(k_pt_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PtShared));
+}
+
+cudaError_t launch_pairs(Pos pos, Out out, const PtPlan &plan, const PtDev &d, double *energy,
+                         double nu, int sms, cudaStream_t st, int *launches)
+{
+    static_assert(sizeof(PtShared) <= 232448, "shared memory of one block");
+    for (const PtGroup &g : plan.groups) {
+        const PtSeg *seg = d.segs + g.seg0;
+        const PtSys *sys = d.sys + g.sys0;
+        const PtSys &first = plan.sys[g.sys0], &last = plan.sys[g.sys0 + g.nsys - 1];
+        const int64_t np = last.part0 + last.n - first.part0;
+        k_pt_split<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(pos, sys, g.nsys, first.part0, np, d.qhi, d.qlo);
+        k_pt_panel<<<(unsigned)g.gen, PT_PANEL_THREADS, 0, st>>>(pos, seg, g.nsegs, d.panel);
+        k_pt_gemm<<<(unsigned)std::min<int64_t>(g.items, sms), PT_WARPS * 32, sizeof(PtShared), st>>>(
+            seg, g.nsegs, g.items, d.tiles, d.panel, d.qhi, d.qlo, d.slots, nu, d.err);
+        k_pt_reduce<<<(unsigned)((np + 7) / 8), 256, 0, st>>>(first.part0, np, sys, g.nsys, d.slots, out, d.err);
+        *launches += 4;
+        if (energy) {
+            k_pt_energy<<<(unsigned)g.nsys, 512, 0, st>>>(sys, d.slots, energy);
+            *launches += 1;
+        }
+    }
+    return cudaGetLastError();
+}
+
+}  // namespace tbmd
