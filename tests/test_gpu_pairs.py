@@ -2,8 +2,8 @@
 edges of the 42-particle row blocks, of the 84-particle column blocks and of the ranges of k, against the
 FP64 oracle.
 
-Tolerance: an entry of G = T T is cut off twice and rounded at most 36 times (2 * 2^-23 + 36 * 2^-24 of its
-partial sums, 2.4e-6), and its contraction with dT/dr rounds fewer than 30 times (1.8e-6)."""
+Tolerance: an entry of G = T T is cut off twice and rounded at most 48 times (2 * 2^-23 + 48 * 2^-24 of its
+partial sums, 3.1e-6), and its contraction with dT/dr rounds fewer than 18 times (1.1e-6)."""
 import numpy as np
 import pytest
 

@@ -95,11 +95,11 @@ struct tbmd_ctx {
     DevBuf partial;
     int sweep_grid = 0;
     // no-cutoff forces of the mixed form as a product of pair tensors: the systems the plan was made
-    // for (their particle offsets), its tables on the device, panel, tile results, split positions
+    // for (their particle offsets), its tables on the device, panel, tile results
     std::vector<int64_t> pt_off;
     PtPlan pt;
     PtDev pt_dev{};
-    DevBuf pt_tab, pt_panel, pt_slots, pt_pos;
+    DevBuf pt_tab, pt_panel, pt_slots;
     int sms = 0;
 
     // P3BCA
@@ -302,7 +302,7 @@ static SweepWork single_sweep(tbmd_ctx *ctx)
 
 // Whether the no-cutoff forces of a system (or the largest of a batch) go through the pair-tensor product
 // (tbmd_pairs.cu) instead of a sweep: the mixed form's forces.  At n = 128 both take about 50 us on the
-// device (46 against 54), from there on the product is faster (n = 1000: 0.22 against 0.94 ms, 8192: 81
+// device (46 against 54), from there on the product is faster (n = 1000: 0.21 against 0.94 ms, 8192: 71
 // against 240 ms for AUTA and 541 for NATA); above 65,536 its panel and tile results would pass 4 GB.
 constexpr int64_t kPairsMin = 128, kPairsMax = 65536;
 static bool use_pairs(const tbmd_ctx *ctx, int64_t n, bool dual)
@@ -329,15 +329,13 @@ static tbmd_status ensure_pairs(tbmd_ctx *ctx, const int64_t *off, int nsys)
     CK(ctx->pt_tab.ensure(b_seg + b_sys + b_til));
     CK(ctx->pt_panel.ensure(p.mem));
     CK(ctx->pt_slots.ensure(p.slots * pt_slot_bytes()));
-    CK(ctx->pt_pos.ensure(sizeof(float4) * 2 * (size_t)off[nsys]));
     char *t = ctx->pt_tab.as<char>();
     CK(cudaMemcpyAsync(t, p.segs.data(), b_seg, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(t + b_seg, p.sys.data(), b_sys, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(t + b_seg + b_sys, p.tiles.data(), b_til, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->pt_dev = PtDev{(const PtSeg *)t, (const PtSys *)(t + b_seg), (const unsigned int *)(t + b_seg + b_sys),
-                        ctx->pt_panel.as<unsigned char>(), ctx->pt_slots.as<double>(), ctx->pt_pos.as<float4>(),
-                        ctx->pt_pos.as<float4>() + off[nsys], pairs_err(ctx)};
+                        ctx->pt_panel.as<unsigned char>(), ctx->pt_slots.as<double>(), pairs_err(ctx)};
     ctx->pt_off.assign(off, off + nsys + 1);
     return TBMD_OK;
 }
@@ -766,7 +764,7 @@ void tbmd_destroy(tbmd_ctx *ctx)
                       &ctx->cell_n, &ctx->cell_c, &ctx->nbr_buf, &ctx->dirs, &ctx->hvp, &ctx->gset_single,
                       &ctx->sweep_sys, &ctx->bpos, &ctx->bout, &ctx->bsys, &ctx->bprefix, &ctx->ncell_tab,
                       &ctx->staging, &ctx->long_buf, &ctx->gen_buf, &ctx->bext, &ctx->pt_tab, &ctx->pt_panel,
-                      &ctx->pt_slots, &ctx->pt_pos})
+                      &ctx->pt_slots})
         b->release();
     if (ctx->hpin) cudaFreeHost(ctx->hpin);
     if (ctx->copy_stream) {

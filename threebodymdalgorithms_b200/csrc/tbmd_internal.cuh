@@ -368,7 +368,6 @@ struct PtDev {
     const unsigned int *tiles;
     unsigned char *panel;
     double *slots;
-    float4 *qhi, *qlo;  // split positions
     unsigned int *err;  // set by a launch that gave up waiting
 };
 void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, PtPlan &plan);

@@ -7,25 +7,28 @@
 // which is the same sum over i < j < k as the pairwise sweeps (the blocks T_ii = 0 leave out repeated
 // indices).  G is a dense product of 27 n^3 FLOP over i < j; the rest is O(n^2).
 //
-//   k_pt_split   positions relative to the system's first particle as FP32 hi + lo parts
 //   k_pt_panel   T for a range of k, formed in FP64 and split exactly into three bfloat16 (h + m + l holds
 //                26 bits), written in the layout the matrix unit reads from shared memory
-//   k_pt_gemm    tiles of G (42 x 84 particles) by tcgen05.mma, contracted with dT/dr in the same kernel
+//   k_pt_gemm    tiles of G (84 x 84 particles over two SMs) by tcgen05.mma, contracted with dT/dr in the
+//                same kernel
 //   k_pt_reduce  each particle's force from its tiles, in a fixed order (deterministic)
 //
-// Bound: the tensor cores at the power cap for large n (n = 8192: 9.4e13 FLOP of bf16 in 81 ms, 1.16 PFLOP/s
-// of 1.36 sustained by cuBLAS; AUTA's FP32 sweep took 240 ms, NATA's 541), the operands' way from L2 for
-// medium n (a slab of 72 KB in 2,100 cycles, 1,536 of them product; n = 4096: 9.5 ms against 31.5 and 79).
-// A tile of 128 x 256 is the largest whose FP32 sums fit the registers (128 a thread in eight warps) beside
-// two accumulators of 256 TMEM columns, one filling while the other is added up.
+// Bound: the tensor cores, at the power cap for large n.  n = 8192: 9.4e13 FLOP of bf16 in 71 ms, 1.32
+// PFLOP/s of the 1.36 that cuBLAS sustains (AUTA's FP32 sweep took 240 ms, NATA's 541); n = 4096: 8.9 ms
+// (31.5 and 79).  A pair of SMs works on one tile of 256 x 256 (cta_group::2), which halves what each loads
+// of B: 48 KB a slab.  A block's 128 x 256 part is the largest whose FP32 sums fit the registers (128 a
+// thread in eight warps) beside two accumulators of 256 TMEM columns, one filling while the other is added
+// up (350 cycles of the 1,536 that a slab's product takes).  One block alone with the same tile of 128 x 256
+// and the FP32 geometry of each row's pairs in every thread took 82 ms: 17,000 cycles of contraction an item.
 //
 // Accuracy.  Six products of the splits are kept (hh, hm, mh, mm, hl, lh; the rest is below 2^-26), each
 // exact in FP32.  The tensor core adds into an FP32 accumulator that it truncates, so an accumulator only
 // lives for 32 columns of T: the ten small products go first, the two hh steps last, and the tile is then
-// added to FP32 registers with rounding.  After 256 particles at most the registers are contracted and the
+// added to FP32 registers with rounding.  After 512 particles at most the registers are contracted and the
 // forces go on in FP64.  Relative L2 error of the forces against FP64, thermal lattices of 512 .. 8192
-// particles: 2.0e-7 .. 2.6e-7 (the FP32 sweeps: 2.3e-7 .. 2.6e-7).  No step subtracts nearly equal numbers: a pair's force needs no difference of
-// large terms even where two of the three particles nearly coincide.
+// particles: 1.5e-7 .. 2.3e-7 (the FP32 sweeps: 2.3e-7 .. 2.6e-7).  No step subtracts nearly equal
+// numbers: a pair's force needs no difference of large terms even where two of the three particles nearly
+// coincide.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -34,22 +37,28 @@
 
 namespace tbmd {
 
-constexpr int PT_PART = 42;                 // particles of a row block: 126 of 128 matrix rows
+// A row block holds 42 particles in 126 of its 128 rows, two particles side by side in six rows (x x' y y'
+// z z'), so that the columns of a tile come in pairs that packed FP32 operations take at once.
+constexpr int PT_PART = 42;
 constexpr int PT_ROWS = 128;
 constexpr int PT_SLAB_K = 32;               // matrix columns of one slab (one pipeline stage)
 constexpr int PT_SPLIT_BYTES = PT_ROWS * PT_SLAB_K * 2;  // one split of a row block's slab: 8 KB
 constexpr int PT_BLOCK_BYTES = 3 * PT_SPLIT_BYTES;       // all three: 24 KB, contiguous in the panel
-constexpr int PT_STAGE_BYTES = 3 * PT_BLOCK_BYTES;       // one row block (A) and two (B)
+constexpr int PT_STAGE_BYTES = 2 * PT_BLOCK_BYTES;       // one row block of A and one of B
 constexpr int PT_STAGES = 3;
-constexpr int PT_WARPS = 12;                // 8 accumulate and contract, 1 loads, 1 issues the products, 2 idle
+constexpr int PT_GEO = 2 * (PT_PART / 2) * PT_PART;      // pair geometry of a block's tile: [pair of j][i]
+// 8 warps accumulate and contract, 1 loads, 1 issues the products, 2 fetch positions
+constexpr int PT_WARPS = 12;
 constexpr int PT_SLOT = 3 * PT_PART * 3 + 2;  // doubles of a tile's results: f_i, f_j (two blocks), energy, pad
 
 struct PtShared {
     unsigned char stage[PT_STAGES][PT_STAGE_BYTES];
+    float4 geo[2][PT_GEO];  // (n_x n_x' n_y n_y') and (n_z n_z' r^-4 r'^-4) of particle i and two j
+    double xj[3][2 * PT_PART], xi[3][PT_PART];  // positions of the tile's particles
     double fi[2][PT_ROWS][3];
     float fj[8][PT_ROWS];
     double e[8];
-    unsigned long long full[PT_STAGES], empty[PT_STAGES], acc_full[2], acc_empty[2], drained;
+    unsigned long long full[PT_STAGES], empty[PT_STAGES], acc_full[2], acc_empty[2], geo_full, geo_empty, drained;
     unsigned int tmem;
     int dead;
 };
@@ -67,6 +76,22 @@ __device__ __forceinline__ void bar_expect(unsigned long long *b, unsigned int b
 {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
 }
+// arrive on the same barrier of block `rank` of the cluster.  Nothing is handed over in memory (a release at
+// cluster scope would wait for the thread's global stores, 1,000 cycles a slab): what the arrivals order is
+// TMEM reads (tcgen05.fence) and bulk copies that have signalled their own barrier.
+__device__ __forceinline__ void bar_arrive_at(unsigned long long *b, unsigned int rank)
+{
+    asm volatile(
+        "{\n\t.reg .b32 a;\n\t"
+        "mapa.shared::cluster.u32 a, %0, %1;\n\t"
+        "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [a];\n\t}" ::"r"(smem_u32(b)),
+        "r"(rank)
+        : "memory");
+}
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __device__ __forceinline__ bool bar_try(unsigned long long *b, unsigned int parity)
 {
     unsigned int ok;
@@ -79,23 +104,17 @@ __device__ __forceinline__ bool bar_try(unsigned long long *b, unsigned int pari
         : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ unsigned long long now_ns()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-// Every wait ends: after two seconds it marks the block dead and the launch failed (*err); from then on
+// Every wait ends: after four billion cycles (two seconds or more) it marks the block dead and the launch failed (*err); from then on
 // waits return at once, no copy or product is issued, and the loops run out.
 __device__ __forceinline__ bool bar_wait(unsigned long long *b, unsigned int parity, PtShared &S, unsigned int *err)
 {
     if (bar_try(b, parity)) return true;
-    const unsigned long long t0 = now_ns();
+    const long long t0 = clock64();
     for (unsigned int n = 1;; ++n) {
         if (bar_try(b, parity)) return true;
         if ((n & 63u) == 0u) {
             if (*(volatile int *)&S.dead) return false;
-            if (now_ns() - t0 > 2000000000ull) {
+            if (clock64() - t0 > 4000000000ll) {
                 *(volatile int *)&S.dead = 1;
                 atomicExch(err, 1u);
                 return false;
@@ -117,44 +136,108 @@ __device__ __forceinline__ unsigned long long operand_desc(unsigned int addr)
     return (unsigned long long)((addr >> 4) & 0x3fffu) | (unsigned long long)(128 >> 4) << 16 |
            (unsigned long long)(512 >> 4) << 32 | 1ull << 46;
 }
-// D FP32, A and B bfloat16, both K-major, 128 x 256
-constexpr unsigned int PT_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | ((128u >> 4) << 24);
+// D FP32, A and B bfloat16, both K-major, 256 x 256 over the two blocks of a cluster: each holds 128 rows of
+// A, 128 of B, and 128 rows x 256 columns of D in its TMEM
+constexpr unsigned int PT_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | ((256u >> 4) << 24);
 __device__ __forceinline__ void mma_bf16(unsigned int d, unsigned long long a, unsigned long long b, unsigned int acc)
 {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d), "l"(a), "l"(b), "r"(PT_IDESC), "r"(acc)
         : "memory");
 }
+// the barrier at this address in both blocks gets an arrival when the products issued so far are done
 __device__ __forceinline__ void mma_commit(unsigned long long *b)
 {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(b))
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+                     smem_u32(b)),
+                 "h"((unsigned short)3)
                  : "memory");
 }
-#define TM_LD32(v, addr)                                                                                       \
-    asm volatile(                                                                                                 \
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,"  \
-        "%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"                                        \
-        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]),             \
-          "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]),       \
-          "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]), "=f"(v[17]),   \
-          "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]),   \
-          "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]),   \
-          "=f"(v[30]), "=f"(v[31])                                                                        \
+// 64 columns of this warp's 32 TMEM lanes
+#define TM_LD64(v, addr)                                                                                       \
+    asm volatile(                                                                                              \
+        "tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%1" \
+        "7,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%4" \
+        "2,%43,%44,%45,%46,%47,%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%64];"       \
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]),                              \
+          "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]),                            \
+          "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]), "=f"(v[17]),                        \
+          "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]),                        \
+          "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]),                        \
+          "=f"(v[30]), "=f"(v[31]), "=f"(v[32]), "=f"(v[33]), "=f"(v[34]), "=f"(v[35]),                        \
+          "=f"(v[36]), "=f"(v[37]), "=f"(v[38]), "=f"(v[39]), "=f"(v[40]), "=f"(v[41]),                        \
+          "=f"(v[42]), "=f"(v[43]), "=f"(v[44]), "=f"(v[45]), "=f"(v[46]), "=f"(v[47]),                        \
+          "=f"(v[48]), "=f"(v[49]), "=f"(v[50]), "=f"(v[51]), "=f"(v[52]), "=f"(v[53]),                        \
+          "=f"(v[54]), "=f"(v[55]), "=f"(v[56]), "=f"(v[57]), "=f"(v[58]), "=f"(v[59]),                        \
+          "=f"(v[60]), "=f"(v[61]), "=f"(v[62]), "=f"(v[63])                                                   \
         : "r"(addr))
 // the loaded registers hold their values from here on
-#define TM_WAIT32(v)                                                                                              \
-    asm volatile("tcgen05.wait::ld.sync.aligned;"                                                                 \
-                 : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]),   \
-                   "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]),         \
-                   "+f"(v[15]), "+f"(v[16]), "+f"(v[17]), "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]),       \
-                   "+f"(v[22]), "+f"(v[23]), "+f"(v[24]), "+f"(v[25]), "+f"(v[26]), "+f"(v[27]), "+f"(v[28]),       \
-                   "+f"(v[29])                                                                                    \
-                 :                                                                                                \
-                 : "memory");                                                                                     \
-    asm volatile("" : "+f"(v[30]), "+f"(v[31]))
+#define TM_WAIT64(v)                                                                             \
+    asm volatile("tcgen05.wait::ld.sync.aligned;"                                                \
+                 : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]),       \
+                   "+f"(v[6]), "+f"(v[7]), "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]),     \
+                   "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15]), "+f"(v[16]), "+f"(v[17]), \
+                   "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]), "+f"(v[22]), "+f"(v[23]), \
+                   "+f"(v[24]), "+f"(v[25]), "+f"(v[26]), "+f"(v[27])                            \
+                 :                                                                               \
+                 : "memory");                                                                    \
+    asm volatile(""                                                                              \
+                 : "+f"(v[28]), "+f"(v[29]), "+f"(v[30]), "+f"(v[31]), "+f"(v[32]), "+f"(v[33]), \
+                   "+f"(v[34]), "+f"(v[35]), "+f"(v[36]), "+f"(v[37]), "+f"(v[38]), "+f"(v[39]), \
+                   "+f"(v[40]), "+f"(v[41]), "+f"(v[42]), "+f"(v[43]), "+f"(v[44]), "+f"(v[45]), \
+                   "+f"(v[46]), "+f"(v[47]), "+f"(v[48]), "+f"(v[49]), "+f"(v[50]), "+f"(v[51]), \
+                   "+f"(v[52]), "+f"(v[53]), "+f"(v[54]), "+f"(v[55])                            \
+                 :                                                                               \
+                 : "memory");                                                                    \
+    asm volatile(""                                                                              \
+                 : "+f"(v[56]), "+f"(v[57]), "+f"(v[58]), "+f"(v[59]), "+f"(v[60]), "+f"(v[61]), \
+                   "+f"(v[62]), "+f"(v[63])                                                      \
+                 :                                                                               \
+                 : "memory")
+
+// two FP32 values in one register pair, and the packed operations on them
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pack2(float a, float b)
+{
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f2 v, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b)
+{
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 sub2(f2 a, f2 b)
+{
+    f2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b)
+{
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c)
+{
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f2 dot2(f2 ax, f2 ay, f2 az, f2 bx, f2 by, f2 bz)
+{
+    return fma2(ax, bx, fma2(ay, by, mul2(az, bz)));
+}
 
 // system of particle p (of the group's, in ascending order)
 __device__ __forceinline__ int pt_system(const PtSys *sys, int nsys, int64_t p)
@@ -185,20 +268,7 @@ __device__ __forceinline__ int pt_find(const PtSeg *seg, int nseg, int64_t w, F 
     return lo;
 }
 
-// Positions relative to the system's first particle as FP32 hi + lo parts.
-__global__ void k_pt_split(Pos pos, const PtSys *__restrict__ sys, int nsys, int64_t p0, int64_t n, float4 *qhi,
-                           float4 *qlo)
-{
-    const int64_t p = p0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= p0 + n) return;
-    const int64_t o = sys[pt_system(sys, nsys, p)].part0;
-    float hx, hy, hz, lx, ly, lz;
-    split<float>(pos.x[p] - pos.x[o], 0.0, hx, lx);
-    split<float>(pos.y[p] - pos.y[o], 0.0, hy, ly);
-    split<float>(pos.z[p] - pos.z[o], 0.0, hz, lz);
-    qhi[p] = make_float4(hx, hy, hz, 0.f);
-    qlo[p] = make_float4(lx, ly, lz, 0.f);
-}
+__device__ __forceinline__ int pt_row(int il, int c) { return 6 * (il >> 1) + 2 * c + (il & 1); }
 
 // The three bfloat16 parts of v, as 16-bit patterns: v = h + m + l to 2^-27 of |v|.
 __device__ __forceinline__ void split3(double v, unsigned short &h, unsigned short &m, unsigned short &l)
@@ -224,7 +294,7 @@ __global__ void __launch_bounds__(PT_PANEL_THREADS) k_pt_panel(Pos pos, const Pt
     const int task = (int)blockIdx.x - s.gen0;
     const int rb = task / groups, kg = task - rb * groups;
     const int il = threadIdx.x % 48, oct = threadIdx.x / 48;
-    if (il > PT_PART) return;
+    if (il > PT_PART + 1) return;  // 42 and 43 are the two rows left over
     const int i = rb * PT_PART + il;
     const bool row_ok = il < PT_PART && i < s.n;
     double xi = 0.0, yi = 0.0, zi = 0.0;
@@ -275,7 +345,7 @@ __global__ void __launch_bounds__(PT_PANEL_THREADS) k_pt_panel(Pos pos, const Pt
     unsigned char *base = panel + s.mem + ((int64_t)rb * s.nslab + kg * 3) * PT_BLOCK_BYTES;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const int row = 3 * il + a;
+        const int row = pt_row(il, a);
         if (row >= PT_ROWS) continue;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -290,7 +360,8 @@ __global__ void __launch_bounds__(PT_PANEL_THREADS) k_pt_panel(Pos pos, const Pt
     }
 }
 
-// One item: a tile (row block a, column blocks 2 b and 2 b + 1) of G over one segment's k.
+// One item of a cluster: row blocks 2 a and 2 a + 1 (one per block) and column blocks 2 b and 2 b + 1 of G
+// over one segment's k.
 struct PtItem {
     PtSeg s;
     int a, b;
@@ -305,34 +376,38 @@ __device__ __forceinline__ PtItem pt_item(const PtSeg *seg, int nseg, const unsi
     return it;
 }
 
-__global__ void __launch_bounds__(PT_WARPS * 32, 1)
-    k_pt_gemm(const PtSeg *__restrict__ seg, int nseg, int64_t items, const unsigned int *__restrict__ tiles,
-              const unsigned char *__restrict__ panel, const float4 *__restrict__ qhi, const float4 *__restrict__ qlo,
-              double *__restrict__ slots, double nu, unsigned int *err)
+template <bool ENERGY>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
+    k_pt_gemm(Pos pos, const PtSeg *__restrict__ seg, int nseg, int64_t items, const unsigned int *__restrict__ tiles,
+              const unsigned char *__restrict__ panel, double *__restrict__ slots, double nu, unsigned int *err)
 {
     extern __shared__ __align__(1024) unsigned char smraw[];
     PtShared &S = *(PtShared *)smraw;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = blockIdx.x & 1, cluster = blockIdx.x >> 1, clusters = gridDim.x >> 1;
     if (threadIdx.x == 0) {
         for (int k = 0; k < PT_STAGES; ++k) {
-            bar_init(&S.full[k], 1);
+            bar_init(&S.full[k], rank == 0 ? 2 : 1);  // block 0 also waits for block 1's loads
             bar_init(&S.empty[k], 1);
         }
         for (int k = 0; k < 2; ++k) {
             bar_init(&S.acc_full[k], 1);
-            bar_init(&S.acc_empty[k], 8);
+            bar_init(&S.acc_empty[k], 16);
         }
+        bar_init(&S.geo_full, 2);
+        bar_init(&S.geo_empty, 8);
         bar_init(&S.drained, 1);
         S.dead = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 9) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&S.tmem))
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&S.tmem))
                      : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    cluster_sync();  // both blocks' barriers are ready
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const unsigned int tmem = S.tmem;
 
@@ -341,37 +416,45 @@ __global__ void __launch_bounds__(PT_WARPS * 32, 1)
         asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
         if (warp == 8 && lane == 0) {
             unsigned int n = 0;  // slabs loaded
-            for (int64_t w = blockIdx.x; w < items; w += gridDim.x) {
+            for (int64_t w = cluster; w < items; w += clusters) {
                 const PtItem it = pt_item(seg, nseg, tiles, w);
                 const int64_t row = (int64_t)it.s.nslab * PT_BLOCK_BYTES;
-                const unsigned char *pa = panel + it.s.mem + it.a * row, *pb = panel + it.s.mem + 2 * it.b * row;
+                const unsigned char *pa = panel + it.s.mem + (2 * it.a + rank) * row,
+                                    *pb = panel + it.s.mem + (2 * it.b + rank) * row;
                 for (int k = 0; k < it.s.nslab; ++k, ++n) {
                     const int st = n % PT_STAGES;
                     if (!bar_wait(&S.empty[st], ((n / PT_STAGES) & 1) ^ 1, S, err)) break;
                     unsigned char *dst = S.stage[st];
                     bar_expect(&S.full[st], PT_STAGE_BYTES);
                     bulk_load(dst, pa + (int64_t)k * PT_BLOCK_BYTES, PT_BLOCK_BYTES, &S.full[st]);
-                    // B: the splits of the two row blocks side by side, 256 rows each
-                    for (int q = 0; q < 3; ++q)
-                        for (int h = 0; h < 2; ++h)
-                            bulk_load(dst + PT_BLOCK_BYTES + (2 * q + h) * PT_SPLIT_BYTES,
-                                      pb + h * row + (int64_t)k * PT_BLOCK_BYTES + q * PT_SPLIT_BYTES, PT_SPLIT_BYTES,
-                                      &S.full[st]);
+                    bulk_load(dst + PT_BLOCK_BYTES, pb + (int64_t)k * PT_BLOCK_BYTES, PT_BLOCK_BYTES, &S.full[st]);
                 }
                 if (*(volatile int *)&S.dead) break;
             }
             // a block that gave up leaves no copy in flight behind it
             if (*(volatile int *)&S.dead)
                 for (unsigned int k = n > PT_STAGES ? n - PT_STAGES : 0; k < n; ++k) {
-                    const unsigned long long t0 = now_ns();
-                    while (!bar_try(&S.full[k % PT_STAGES], (k / PT_STAGES) & 1) && now_ns() - t0 < 100000000ull) {
+                    const long long t0 = clock64();
+                    while (!bar_try(&S.full[k % PT_STAGES], (k / PT_STAGES) & 1) && clock64() - t0 < 200000000ll) {
                     }
                 }
         }
-        if (warp == 9 && lane == 0) {
+        if (warp == 9 && lane == 0 && rank == 1) {
+            // tell block 0, which issues the products of both, that this block's slab is there
+            unsigned int n = 0;
+            for (int64_t w = cluster; w < items; w += clusters) {
+                const PtItem it = pt_item(seg, nseg, tiles, w);
+                for (int k = 0; k < it.s.nslab; ++k, ++n) {
+                    if (!bar_wait(&S.full[n % PT_STAGES], (n / PT_STAGES) & 1, S, err)) break;
+                    bar_arrive_at(&S.full[n % PT_STAGES], 0);
+                }
+                if (*(volatile int *)&S.dead) break;
+            }
+        }
+        if (warp == 9 && lane == 0 && rank == 0) {
             unsigned int n = 0;
             bool ok = true;
-            for (int64_t w = blockIdx.x; ok && w < items; w += gridDim.x) {
+            for (int64_t w = cluster; ok && w < items; w += clusters) {
                 const PtItem it = pt_item(seg, nseg, tiles, w);
                 for (int k = 0; k < it.s.nslab; ++k, ++n) {
                     const int st = n % PT_STAGES, buf = n & 1;
@@ -387,96 +470,141 @@ __global__ void __launch_bounds__(PT_WARPS * 32, 1)
 #pragma unroll
                         for (int kk = 0; kk < 2; ++kk)
                             mma_bf16(D, operand_desc(A + qa[p] * PT_SPLIT_BYTES + kk * 256),
-                                     operand_desc(B + qb[p] * 2 * PT_SPLIT_BYTES + kk * 256), p + kk > 0);
+                                     operand_desc(B + qb[p] * PT_SPLIT_BYTES + kk * 256), p + kk > 0);
                     mma_commit(&S.empty[st]);
                     mma_commit(&S.acc_full[buf]);
                 }
             }
             if (!ok) {  // products in flight end before the accumulators are given back
                 mma_commit(&S.drained);
-                const unsigned long long t0 = now_ns();
-                while (!bar_try(&S.drained, 0) && now_ns() - t0 < 100000000ull) {
+                const long long t0 = clock64();
+                while (!bar_try(&S.drained, 0) && clock64() - t0 < 200000000ll) {
                 }
+            }
+        }
+        if (warp >= 10) {
+            // the positions of the tile's particles, fetched while its product runs
+            unsigned int m = 0;
+            for (int64_t w = cluster; w < items; w += clusters, ++m) {
+                const PtItem it = pt_item(seg, nseg, tiles, w);
+                const int i0 = (2 * it.a + rank) * PT_PART, j0 = 2 * it.b * PT_PART;
+                bar_wait(&S.geo_empty, (m & 1) ^ 1, S, err);
+                for (int q = (warp - 10) * 32 + lane; q < 3 * PT_PART; q += 64) {
+                    const bool is_j = q < 2 * PT_PART;
+                    const int64_t p = it.s.part0 + min(is_j ? j0 + q : i0 + q - 2 * PT_PART, it.s.n - 1);
+                    double *d = is_j ? &S.xj[0][q] : &S.xi[0][q - 2 * PT_PART];
+                    const int step = is_j ? 2 * PT_PART : PT_PART;
+                    d[0] = pos.x[p];
+                    d[step] = pos.y[p];
+                    d[2 * step] = pos.z[p];
+                }
+                __syncwarp();
+                if (lane == 0) bar_arrive(&S.geo_full);
             }
         }
         __syncwarp();
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
         const int quad = warp & 3, half = warp >> 2;
-        const int row = quad * 32 + lane, ip = row / 3, al = row - 3 * ip;
-        const float ex = al == 0 ? 1.f : 0.f, ey = al == 1 ? 1.f : 0.f, ez = al == 2 ? 1.f : 0.f;
+        const int row = quad * 32 + lane, ip = 2 * (row / 6) + (row & 1), al = row % 6 >> 1;
+        const f2 ex = pack2(al == 0, al == 0), ey = pack2(al == 1, al == 1), ez = pack2(al == 2, al == 2);  // unit vector
+        const f2 m5 = pack2(-5.f, -5.f), c3 = pack2(3.f, 3.f), m1 = pack2(-1.f, -1.f);
         const unsigned int taddr = tmem + ((unsigned int)(quad * 32) << 16) + half * 128;
-        unsigned int n = 0;
-        for (int64_t w = blockIdx.x; w < items; w += gridDim.x) {
+        unsigned int n = 0, m = 0;
+        for (int64_t w = cluster; w < items; w += clusters, ++m) {
             const PtItem it = pt_item(seg, nseg, tiles, w);
-            float g[128];
+            f2 g2[64];  // columns 2 c and 2 c + 1
 #pragma unroll
-            for (int c = 0; c < 128; ++c) g[c] = 0.f;
+            for (int c = 0; c < 64; ++c) g2[c] = 0ull;
             for (int k = 0; k < it.s.nslab; ++k, ++n) {
                 const int buf = n & 1;
                 if (!bar_wait(&S.acc_full[buf], (n >> 1) & 1, S, err)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    float t[32];
-                    TM_LD32(t, taddr + buf * 256 + c * 32);
-                    TM_WAIT32(t);
+                for (int c = 0; c < 2; ++c) {
+                    float t[64];
+                    TM_LD64(t, taddr + buf * 256 + c * 64);
+                    TM_WAIT64(t);
+                    if (c == 1) {  // the accumulator is in registers: free for the next but one slab
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        if (lane == 0) bar_arrive_at(&S.acc_empty[buf], 0);
+                    }
 #pragma unroll
-                    for (int q = 0; q < 32; ++q) g[c * 32 + q] += t[q];
+                    for (int q = 0; q < 32; ++q) g2[c * 32 + q] = add2(g2[c * 32 + q], pack2(t[2 * q], t[2 * q + 1]));
                 }
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                if (lane == 0) bar_arrive(&S.acc_empty[buf]);
             }
+            // Geometry of the tile's pairs: n = r / |r| and r^-4, rounded once from FP64 (in FP32 their rounding
+            // would count four times in the force).  1 / r is the FP32 approximation t with one step on its
+            // FP64 residual, t (1 + (1 - r^2 t^2) / 2): 2^-44.  Done here, in the pause of the product, since
+            // the operands' reads leave shared memory no room for it while the product runs.
+            const int i0 = (2 * it.a + rank) * PT_PART, j0 = 2 * it.b * PT_PART;
+            bar_wait(&S.geo_full, m & 1, S, err);
+            for (int q = threadIdx.x; q < PT_GEO; q += 256) {
+                const int jp = q / PT_PART, il = q - jp * PT_PART, i = i0 + il;
+                const double xi = S.xi[0][il], yi = S.xi[1][il], zi = S.xi[2][il];
+                float v[2][4];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int j = j0 + 2 * jp + u;
+                    const double x = S.xj[0][2 * jp + u] - xi, y = S.xj[1][2 * jp + u] - yi, z = S.xj[2][2 * jp + u] - zi;
+                    const double r2 = fma(x, x, fma(y, y, z * z)), t = (double)rsqrt_((float)r2);
+                    const double ri = fma(0.5 * fma(-r2, t * t, 1.0), t, t), ri2 = ri * ri;
+                    const bool ok = i < j && j < it.s.n;
+                    v[u][0] = ok ? (float)(x * ri) : 0.f;
+                    v[u][1] = ok ? (float)(y * ri) : 0.f;
+                    v[u][2] = ok ? (float)(z * ri) : 0.f;
+                    v[u][3] = ok ? (float)(ri2 * ri2) : 0.f;
+                }
+                S.geo[0][q] = make_float4(v[0][0], v[1][0], v[0][1], v[1][1]);
+                S.geo[1][q] = make_float4(v[0][2], v[1][2], v[0][3], v[1][3]);
+            }
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            if (lane == 0) bar_arrive(&S.geo_empty);
             // contraction: this thread's row (i, al) of G against dT_ij/dr for the 42 particles j of its
-            // column block; with g the row of G_ij, y = g.r and the unit vector e of the row, its part of
-            // G_ij : dT/dr is 3 / r^5 (y e + r_al g + (g_al - 5 r_al y / r^2) r)
-            const int i = it.a * PT_PART + ip, j0 = (2 * it.b + half) * PT_PART;
-            const bool iv = row < 3 * PT_PART && i < it.s.n;
-            const float4 ih = qhi[it.s.part0 + (iv ? i : 0)], il = qlo[it.s.part0 + (iv ? i : 0)];
+            // column block, two at a time; with g the row of G_ij, n = r / |r|, y = g.n and the unit vector e
+            // of the row, its part of G_ij : dT/dr is 3 / r^4 (y e + n_al g + (g_al - 5 n_al y) n)
+            const int go = half * (PT_PART / 2) * PT_PART + (row < 3 * PT_PART ? ip : 0);
+            const float rv = row < 3 * PT_PART ? 1.f : 0.f;
             double fx = 0.0, fy = 0.0, fz = 0.0, en = 0.0;
 #pragma unroll
-            for (int j6 = 0; j6 < PT_PART; j6 += 6) {
-                float sx = 0.f, sy = 0.f, sz = 0.f, se = 0.f;
+            for (int p3 = 0; p3 < PT_PART / 2; p3 += 3) {
+                f2 sx = 0ull, sy = 0ull, sz = 0ull, se = 0ull;
 #pragma unroll
-                for (int jj = j6; jj < j6 + 6; ++jj) {
-                    const int j = j0 + jj, jc = it.s.part0 + min(j, it.s.n - 1);
-                    const float4 jh = __ldg(qhi + jc), jl = __ldg(qlo + jc);
-                    // r and what its rounding left out (the difference of the hi parts of near particles is exact)
-                    const float ax = jh.x - ih.x, ay = jh.y - ih.y, az = jh.z - ih.z;
-                    const float bx = jl.x - il.x, by = jl.y - il.y, bz = jl.z - il.z;
-                    const float rx = ax + bx, ry = ay + by, rz = az + bz;
-                    const float cx = bx - (rx - ax), cy = by - (ry - ay), cz = bz - (rz - az);
-                    const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-                    const float rc = fmaf(rx, cx, fmaf(ry, cy, rz * cz));
-                    // r^-5 = t^5 (1 + 5/2 e) with t the approximate r^-1 and e = 1 - r^2 t^2 (t^2 as s + sl)
-                    float t = rsqrt_(r2);
-                    if (!(iv && i < j && j < it.s.n)) t = 0.f;
-                    const float s = t * t, sl = fmaf(t, t, -s);
-                    float e = fmaf(-2.f * rc, s, fmaf(-r2, sl, fmaf(-r2, s, 1.f)));
-                    float i5 = s * s * t;
-                    i5 = fmaf(2.5f * e, i5, i5);
-                    const float ri2 = fmaf(e, s, s);
-                    const float gx = g[3 * jj], gy = g[3 * jj + 1], gz = g[3 * jj + 2];
-                    const float y = fmaf(gx, rx, fmaf(gy, ry, gz * rz));
-                    const float ra = fmaf(ex, rx, fmaf(ey, ry, ez * rz)), ga = fmaf(ex, gx, fmaf(ey, gy, ez * gz));
-                    const float ray = ra * y;
-                    const float sc = fmaf(-5.f * ri2, ray, ga);
-                    const float vx = fmaf(ex, y, fmaf(ra, gx, sc * rx)) * i5;
-                    const float vy = fmaf(ey, y, fmaf(ra, gy, sc * ry)) * i5;
-                    const float vz = fmaf(ez, y, fmaf(ra, gz, sc * rz)) * i5;
-                    sx += vx;
-                    sy += vy;
-                    sz += vz;
-                    se += i5 * fmaf(3.f, ray, -(ga * r2));  // row al of G_ij : T_ij
-                    g[3 * jj] = vx;
-                    g[3 * jj + 1] = vy;
-                    g[3 * jj + 2] = vz;
+                for (int p = p3; p < p3 + 3; ++p) {
+                    const float4 A = S.geo[0][go + p * PT_PART], B = S.geo[1][go + p * PT_PART];
+                    const f2 nx = pack2(A.x, A.y), ny = pack2(A.z, A.w), nz = pack2(B.x, B.y);
+                    const f2 i4 = pack2(B.z * rv, B.w * rv);
+                    const f2 gx = g2[3 * p], gy = g2[3 * p + 1], gz = g2[3 * p + 2];
+                    const f2 y = dot2(gx, gy, gz, nx, ny, nz);
+                    const f2 na = al == 0 ? nx : al == 1 ? ny : nz, ga = al == 0 ? gx : al == 1 ? gy : gz;
+                    const f2 nay = mul2(na, y), sc = fma2(m5, nay, ga);
+                    const f2 vx = mul2(fma2(ex, y, fma2(na, gx, mul2(sc, nx))), i4);
+                    const f2 vy = mul2(fma2(ey, y, fma2(na, gy, mul2(sc, ny))), i4);
+                    const f2 vz = mul2(fma2(ez, y, fma2(na, gz, mul2(sc, nz))), i4);
+                    sx = add2(sx, vx);
+                    sy = add2(sy, vy);
+                    sz = add2(sz, vz);
+                    if (ENERGY) {  // row al of G_ij : T_ij, with r^-3 = r^-4 r
+                        const float q0 = rsqrt_(fmaxf(B.z, 1e-36f)), q1 = rsqrt_(fmaxf(B.w, 1e-36f));  // r^2
+                        se = fma2(mul2(i4, pack2(q0 * rsqrt_(q0), q1 * rsqrt_(q1))), fma2(c3, nay, mul2(m1, ga)), se);
+                    }
+                    g2[3 * p] = vx;
+                    g2[3 * p + 1] = vy;
+                    g2[3 * p + 2] = vz;
                 }
-                fx += (double)sx;
-                fy += (double)sy;
-                fz += (double)sz;
-                en += (double)se;
+                float u0, u1;
+                unpack2(sx, u0, u1);
+                fx += (double)(u0 + u1);
+                unpack2(sy, u0, u1);
+                fy += (double)(u0 + u1);
+                unpack2(sz, u0, u1);
+                fz += (double)(u0 + u1);
+                unpack2(se, u0, u1);
+                if (ENERGY) en += (double)(u0 + u1);
             }
+            float g[128];
+#pragma unroll
+            for (int c = 0; c < 63; ++c) unpack2(g2[c], g[2 * c], g[2 * c + 1]);
             g[126] = g[127] = 0.f;
             // f_j: sums over the warp's 32 rows, 4 columns left per lane
 #pragma unroll
@@ -495,24 +623,27 @@ __global__ void __launch_bounds__(PT_WARPS * 32, 1)
             S.fi[half][row][0] = fx;
             S.fi[half][row][1] = fy;
             S.fi[half][row][2] = fz;
-            en = warp_sum(en);
-            if (lane == 0) S.e[warp] = en;
+            if (ENERGY) {
+                en = warp_sum(en);
+                if (lane == 0) S.e[warp] = en;
+            }
             asm volatile("bar.sync 1, 256;" ::: "memory");
-            double *slot = slots + (it.s.slot0 + (int64_t)it.b * (it.b + 1) + it.a) * PT_SLOT;
+            double *slot = slots + (it.s.slot0 + (int64_t)it.b * (it.b + 1) + 2 * it.a + rank) * PT_SLOT;
             const int t = threadIdx.x;
             if ((t & 127) < 126) {
                 double v = 0.0;
                 for (int q = 0; q < 4; ++q) v += (double)S.fj[(t >> 7) * 4 + q][t & 127];
-                slot[126 + (t >> 7) * 126 + (t & 127)] = -nu * v;
+                const int c = t & 127;
+                slot[126 + (t >> 7) * 126 + 3 * (2 * (c / 6) + (c & 1)) + (c % 6 >> 1)] = -nu * v;
             }
             if (t < 126) {
                 const int p = t / 3, c = t - 3 * p;
                 double v = 0.0;
                 for (int h = 0; h < 2; ++h)
-                    for (int q = 0; q < 3; ++q) v += S.fi[h][3 * p + q][c];
+                    for (int q = 0; q < 3; ++q) v += S.fi[h][pt_row(p, q)][c];
                 slot[t] = nu * v;
             }
-            if (t == 255) {
+            if (ENERGY && t == 255) {
                 double v = 0.0;
                 for (int q = 0; q < 8; ++q) v += S.e[q];
                 slot[378] = -nu * v / 9.0;
@@ -522,8 +653,9 @@ __global__ void __launch_bounds__(PT_WARPS * 32, 1)
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    cluster_sync();  // no arrival or product of the other block is left
     if (warp == 9)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem));
 }
 
 // Forces from the tiles' results: particle i of row block a sums the tiles (a, b) of its row and the tiles
@@ -581,35 +713,35 @@ __global__ void __launch_bounds__(512) k_pt_energy(const PtSys *__restrict__ sys
 // ---------------------------------------------------------------------------------------------
 // Work lists (host)
 
-// Tile order of nb2 column blocks: strips of 8 column blocks, walked row by row, so that the tiles in
-// flight (one per SM) share row and column blocks in L2 (18 + 16 blocks of 1.1 MB at 512 k).
+// Tile order of nb2 blocks of 84 particles: strips of 8 column blocks, walked row by row, so that the tiles
+// in flight (one per two SMs) share row and column blocks in L2 (17 blocks, 20 MB at 256 k).
 static void pt_tiles(int nb2, std::vector<unsigned int> &out)
 {
     for (int b0 = 0; b0 < nb2; b0 += 8) {
         const int b1 = std::min(nb2, b0 + 8);
-        for (int a = 0; a < 2 * b1; ++a)
-            for (int b = std::max(b0, a >> 1); b < b1; ++b) out.push_back((unsigned int)a << 16 | (unsigned int)b);
+        for (int a = 0; a < b1; ++a)
+            for (int b = std::max(b0, a); b < b1; ++b) out.push_back((unsigned int)a << 16 | (unsigned int)b);
     }
 }
 
-// Particles k of one item: the range length with the least estimated time of all items, at 2,100 cycles a
-// slab (the product alone is 1,536; the rest is the operands' way through L2) and 10,000 an item (set-up,
-// contraction).  256 at most, for the accuracy of the FP32 sums over a range: with 512 (n = 8192: 73 ms
-// against 81) the forces' error was 5% above the pairwise sweep's at n = 2048 .. 6500.
+// Particles k of one item: the range length with the least estimated time of all items, at 1,536 cycles a
+// slab (what its product takes) and 14,000 an item, while the product pauses (geometry 5,800, contraction
+// 4,800, the rest sums over rows and set-up).  512 at most, for the accuracy of the FP32 sums over a range.
 static int pt_range(const int64_t *sys_off, int nsys, int sms)
 {
-    int best = 256;
+    int best = 512;
     double least = 0.0;
-    for (int kp : {256, 192, 128, 96, 64, 32}) {
+    for (int kp : {512, 384, 256, 192, 128, 96, 64, 32}) {
         int64_t items = 0;
         double slabs = 0.0;
         for (int s = 0; s < nsys; ++s) {
             const int64_t n = sys_off[s + 1] - sys_off[s], nb2 = (n + 2 * PT_PART - 1) / (2 * PT_PART);
-            items += nb2 * (nb2 + 1) * ((n + kp - 1) / kp);
-            slabs += (double)(nb2 * (nb2 + 1)) * (double)((n + 31) / 32 * 3);
+            items += nb2 * (nb2 + 1) / 2 * ((n + kp - 1) / kp);
+            slabs += (double)(nb2 * (nb2 + 1) / 2) * (double)((n + 31) / 32 * 3);
         }
-        const double t = (double)((items + sms - 1) / sms) * (slabs / (double)(items ? items : 1) * 2100.0 + 10000.0);
-        if (kp == 256 || t < 0.98 * least) {
+        const int pairs = sms / 2;
+        const double t = (double)((items + pairs - 1) / pairs) * (slabs / (double)(items ? items : 1) * 1536.0 + 14000.0);
+        if (kp == 512 || t < 0.98 * least) {
             least = t;
             best = kp;
         }
@@ -653,7 +785,7 @@ void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, PtPlan &p
             plan.segs.push_back(PtSeg{(int64_t)g.mem, g.items, g.slots, (int)sys_off[s], (int)n, (int)k0, nslab, tab,
                                       g.gen});
             g.mem += mem;
-            g.items += tiles;
+            g.items += tiles / 2;
             g.slots += tiles;
             g.gen += 2 * nb2 * (nslab / 3);
             ++g.nsegs;
@@ -672,7 +804,11 @@ size_t pt_slot_bytes() { return PT_SLOT * sizeof(double); }
 
 cudaError_t pt_init()
 {
-    return cudaFuncSetAttribute(k_pt_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PtShared));
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_pt_gemm<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PtShared));
+    return e != cudaSuccess ? e
+                            : cudaFuncSetAttribute(k_pt_gemm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)sizeof(PtShared));
 }
 
 cudaError_t launch_pairs(Pos pos, Out out, const PtPlan &plan, const PtDev &d, double *energy,
@@ -684,12 +820,12 @@ cudaError_t launch_pairs(Pos pos, Out out, const PtPlan &plan, const PtDev &d, d
         const PtSys *sys = d.sys + g.sys0;
         const PtSys &first = plan.sys[g.sys0], &last = plan.sys[g.sys0 + g.nsys - 1];
         const int64_t np = last.part0 + last.n - first.part0;
-        k_pt_split<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(pos, sys, g.nsys, first.part0, np, d.qhi, d.qlo);
         k_pt_panel<<<(unsigned)g.gen, PT_PANEL_THREADS, 0, st>>>(pos, seg, g.nsegs, d.panel);
-        k_pt_gemm<<<(unsigned)std::min<int64_t>(g.items, sms), PT_WARPS * 32, sizeof(PtShared), st>>>(
-            seg, g.nsegs, g.items, d.tiles, d.panel, d.qhi, d.qlo, d.slots, nu, d.err);
+        const unsigned blocks = 2 * (unsigned)std::min<int64_t>(g.items, sms / 2);
+        auto gemm = energy ? k_pt_gemm<true> : k_pt_gemm<false>;
+        gemm<<<blocks, PT_WARPS * 32, sizeof(PtShared), st>>>(pos, seg, g.nsegs, g.items, d.tiles, d.panel, d.slots, nu, d.err);
         k_pt_reduce<<<(unsigned)((np + 7) / 8), 256, 0, st>>>(first.part0, np, sys, g.nsys, d.slots, out, d.err);
-        *launches += 4;
+        *launches += 3;
         if (energy) {
             k_pt_energy<<<(unsigned)g.nsys, 512, 0, st>>>(sys, d.slots, energy);
             *launches += 1;
