@@ -109,8 +109,8 @@ struct tbmd_ctx {
     GridSet gset{};       // device tables of the systems being evaluated
     DevBuf gset_single;   // Grid[1] + cell_off[2] + sys_off[2] of the single-system case
     alignas(8) unsigned char gset_host[256] = {};  // host copy of what gset_single holds
-    DevBuf ncell_tab;     // neighbour-cell table of the cells being evaluated (27 per cell)
-    Grid ncell_grid{};    // grid the single-system table was built for
+    DevBuf ncell_tab;     // neighbour-cell table of the cells being evaluated (27 runs per cell)
+    int ncell_dims[3] = {0, 0, 0};  // cells per axis the single-system table was built for
     bool ncell_single = false;
     std::vector<int32_t> ncell_batch_key;  // per-system dims the batched table was built for
     int max_stage = 256;  // neighbour staging capacity
@@ -435,6 +435,8 @@ static tbmd_status ensure_cell_bufs(tbmd_ctx *ctx, int64_t n, int64_t nc, bool d
     ctx->cb.long_count = (unsigned int *)(ctx->scalars.as<char>() + 40);
     ctx->cb.long_max = (unsigned int *)(ctx->scalars.as<char>() + 44);
     ctx->cb.cap = ctx->cap;
+    if (!ctx->sms) CK(cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device));
+    ctx->cb.sms = ctx->sms;
     const int key[5] = {mixed(ctx) ? 1 : 0, dual ? 1 : 0, energy ? 1 : 0, ctx->cap, ctx->p3_warps};
     if (std::memcmp(key, ctx->plan_key, sizeof key) != 0) {
         CK(plan_p3bca(mixed(ctx), dual, energy, ctx->cap, ctx->p3_warps, &ctx->plan));
@@ -472,14 +474,12 @@ static tbmd_status ensure_cells(tbmd_ctx *ctx, int64_t n, bool dual, bool energy
     ctx->gset = GridSet{(const Grid *)base, (const int64_t *)(base + offsetof(decltype(tab), cell_off)),
                         (const int64_t *)(base + offsetof(decltype(tab), sys_off)), 1};
     ctx->max_stage = neighbor_stage_cap(ctx->grid, n);
-    if (!ctx->ncell_single || std::memcmp(&ctx->ncell_grid, &ctx->grid, sizeof(Grid)) != 0) {
-        std::vector<int32_t> tab27((size_t)ctx->grid.ncells * 27);
-        neighbor_cell_table(ctx->grid, 0, tab27.data());
-        CK(ctx->ncell_tab.ensure(sizeof(int32_t) * tab27.size()));
-        CK(cudaMemcpyAsync(ctx->ncell_tab.p, tab27.data(), sizeof(int32_t) * tab27.size(), cudaMemcpyHostToDevice,
-                           ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        ctx->ncell_grid = ctx->grid;
+    if (!ctx->ncell_single || std::memcmp(ctx->ncell_dims, ctx->grid.dims, sizeof ctx->ncell_dims) != 0) {
+        CK(ctx->ncell_tab.ensure(sizeof(int2) * 27 * (size_t)ctx->grid.ncells));
+        CK(launch_neighbor_table(ctx->grid, ctx->gset, ctx->ncell_tab.as<int2>(), ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));  // the lists may be built on another stream
+        ctx->launches += 1;
+        std::memcpy(ctx->ncell_dims, ctx->grid.dims, sizeof ctx->ncell_dims);
         ctx->ncell_single = true;
     }
     return ensure_cell_bufs(ctx, n, ctx->grid.ncells, dual, energy);
@@ -524,7 +524,7 @@ static tbmd_status enqueue_forces(tbmd_ctx *ctx, int64_t n, Pos pos, Out out, bo
         phase_mark(ctx, st, PH_CELLS, *nl);
         CK(launch_cell_build(n, pos, ctx->grid, ctx->gset, cb, dual, st, nl));
         phase_mark(ctx, st, PH_NEIGHBORS, *nl);
-        CK(launch_neighbors(n, ctx->grid, ctx->gset, ctx->ncell_tab.as<int32_t>(), ctx->max_stage, cb, st));
+        CK(launch_neighbors(n, ctx->grid, ctx->gset, ctx->ncell_tab.as<int2>(), ctx->max_stage, cb, st));
         *nl += 1;
         CK(cudaMemsetAsync(cb.fs[0], 0, sizeof(double) * 3 * n, st));  // fs[0..2] are adjacent
         if (dual) CK(cudaMemsetAsync(cb.hs[0], 0, sizeof(double) * 3 * n, st));
@@ -593,7 +593,7 @@ static tbmd_status enqueue_step(tbmd_ctx *ctx, cudaStream_t st, int *nl)
         CK(launch_step_cells(n, s, ctx->cfg.dt, ctx->grid, cb, st, nl));
         if (ctx->pos_event) CK(cudaEventRecordWithFlags(ctx->pos_event, st, cudaEventRecordExternal));
         phase_mark(ctx, st, PH_NEIGHBORS, *nl);
-        CK(launch_neighbors(n, ctx->grid, ctx->gset, ctx->ncell_tab.as<int32_t>(), ctx->max_stage, cb, st));
+        CK(launch_neighbors(n, ctx->grid, ctx->gset, ctx->ncell_tab.as<int2>(), ctx->max_stage, cb, st));
         *nl += 1;
         CK(cudaMemsetAsync(cb.fs[0], 0, sizeof(double) * 3 * n, st));  // fs[0..2] are adjacent
         phase_mark(ctx, st, PH_TRIPLETS, *nl);
@@ -1648,15 +1648,7 @@ static tbmd_status batch_eval(tbmd_ctx *ctx, int32_t nsys, const int64_t *offset
         std::vector<int32_t> tkey(3 * (size_t)nsys);
         for (int s = 0; s < nsys; ++s)
             for (int d = 0; d < 3; ++d) tkey[3 * s + d] = grids[s].dims[d];
-        if (ctx->ncell_single || tkey != ctx->ncell_batch_key) {
-            std::vector<int32_t> tab27((size_t)cell_off[nsys] * 27);
-            for (int s = 0; s < nsys; ++s) neighbor_cell_table(grids[s], cell_off[s], tab27.data());
-            CK(ctx->ncell_tab.ensure(sizeof(int32_t) * tab27.size()));
-            CK(cudaMemcpyAsync(ctx->ncell_tab.p, tab27.data(), sizeof(int32_t) * tab27.size(), cudaMemcpyHostToDevice,
-                               sm));
-            CK(cudaStreamSynchronize(sm));  // tab27 lives on this stack frame
-            ctx->ncell_batch_key = tkey;
-        }
+        const bool new_table = ctx->ncell_single || tkey != ctx->ncell_batch_key;
         ctx->ncell_single = false;  // the single-system table is rebuilt on the next single evaluation
         const size_t gbytes = sizeof(Grid) * nsys, obytes = sizeof(int64_t) * (nsys + 1);
         CK(ctx->bsys.ensure(gbytes + 2 * obytes + 64));
@@ -1667,6 +1659,13 @@ static tbmd_status batch_eval(tbmd_ctx *ctx, int32_t nsys, const int64_t *offset
         const int saved_cap = ctx->cap;
         Grid all = grids[0];
         all.ncells = cell_off[nsys];
+        if (new_table) {
+            CK(ctx->ncell_tab.ensure(sizeof(int2) * 27 * (size_t)cell_off[nsys]));
+            const GridSet gs{(const Grid *)tb, (const int64_t *)(tb + gbytes), (const int64_t *)(tb + gbytes + obytes), nsys};
+            CK(launch_neighbor_table(all, gs, ctx->ncell_tab.as<int2>(), sm));
+            nl += 1;
+            ctx->ncell_batch_key = tkey;
+        }
         ctx->cap = cap;
         tbmd_status r = TBMD_CAPACITY_RETRY;
         for (int attempt = 0; attempt < 4; ++attempt) {
@@ -1680,7 +1679,7 @@ static tbmd_status batch_eval(tbmd_ctx *ctx, int32_t nsys, const int64_t *offset
             CK(cudaMemsetAsync(E, 0, sizeof(double) * 2 * nsys, sm));
             CellBufs &cb = ctx->cb;
             CK(launch_cell_build(N, pos, ctx->grid, ctx->gset, cb, dual, sm, &nl));
-            CK(launch_neighbors(N, ctx->grid, ctx->gset, ctx->ncell_tab.as<int32_t>(), ctx->max_stage, cb, sm));
+            CK(launch_neighbors(N, ctx->grid, ctx->gset, ctx->ncell_tab.as<int2>(), ctx->max_stage, cb, sm));
             CK(cudaMemsetAsync(cb.fs[0], 0, sizeof(double) * 3 * N, sm));  // fs[0..2] are adjacent
             if (dual) CK(cudaMemsetAsync(cb.hs[0], 0, sizeof(double) * 3 * N, sm));
             CK(launch_p3bca(mx, dual, true, N, ctx->grid, ctx->gset, cb, nu, E, CNT, ctx->plan, sm));

@@ -400,6 +400,7 @@ struct CellBufs {
     int32_t *max_count;    // [1] largest list length seen (overflow detection)
     unsigned int *work_counter;  // [2] dynamic item counters of the triplet kernel (particles, chunk pairs)
     int cap;
+    int sms;  // of the device
     // lists longer than P3_CHUNK: (s << 32 | I << 16 | J) chunk-pair items, queued by the neighbour kernel
     unsigned long long *long_items;  // [long_cap]
     int long_cap;
@@ -418,11 +419,11 @@ cudaError_t launch_step_cells(int64_t n, double *const st13[13], double dt, cons
 cudaError_t launch_unsort_update(int64_t n, const CellBufs &cb, double *const st13[13], double dt, const double g3[3],
                                  unsigned long long *cur, unsigned long long *per_step, unsigned int *step,
                                  cudaStream_t st);
-cudaError_t launch_neighbors(int64_t n, const Grid &g, const GridSet &set, const int32_t *nbr_cells, int max_stage,
+cudaError_t launch_neighbors(int64_t n, const Grid &g, const GridSet &set, const int2 *nbr_runs, int max_stage,
                              CellBufs &cb, cudaStream_t st);
 int neighbor_stage_cap(const Grid &g, int64_t n);
-// host: neighbour-cell table rows (27 ints per cell, ids >= the cell's own, ascending, -1 padded)
-void neighbor_cell_table(const Grid &g, int64_t cell0, int32_t *out);
+// neighbour-cell table: 27 runs of cells per cell; depends only on the systems' cells per axis
+cudaError_t launch_neighbor_table(const Grid &g, const GridSet &set, int2 *out, cudaStream_t st);
 // Launch shape of the P3BCA triplet kernel for a list capacity; computed outside graph capture.
 struct P3Plan {
     int warps = 0;

@@ -810,13 +810,14 @@ cudaError_t launch_unsort_update(int64_t n, const CellBufs &cb, double *const st
 //
 // Block per cell c.  Particles are counting-sorted by cell id, so the candidates t > s of a
 // particle s in c are: the particles of c after s, and all particles of the neighbour cells with
-// id > c.  nbr_cells (built on the host with the grid) lists, per cell, its neighbour cells with
-// id >= c in increasing id order (-1 padded to 27).  The block scans their sizes and stages their
-// particles (FP32 hi/lo positions relative to the box corner, with the sorted index in the hi
-// record's spare w) in shared memory in that order - cell by cell, so every copy is coalesced - and
+// id > c.  nbr_runs (k_neighbor_table) lists, per cell, its neighbour cells with id >= c in increasing
+// id order as runs of consecutive cells, whose particles are consecutive too.  The block scans the runs'
+// sizes and stages their particles (FP32 hi/lo positions relative to the box corner, with the sorted
+// index in the hi record's spare w) in shared memory in that order, so every copy is coalesced, and
 // the candidates of the i-th particle of c are the suffix after i.  Warps take the particles of c in
 // turn and sweep their suffix 32 candidates at a time, writing survivors compacted by ballot.  A
-// cell whose candidates exceed the staging capacity reads them from global memory instead.  Lists
+// cell whose candidates exceed the staging capacity stages them in turns, its lists' lengths kept in
+// nbr_count between two turns.  With few cells, `split` blocks share a cell's particles.  Lists
 // longer than cap are truncated; the largest length is recorded so the host can enlarge cap and
 // recompute.
 //
@@ -836,8 +837,9 @@ constexpr int NB_THREADS = 128;
 constexpr unsigned int P3_NO_WORK = 0x80000000u;
 constexpr size_t NB_STAGE_BYTES = 2 * sizeof(float4);  // per staged candidate (hi with the index in w, lo)
 
+template <bool SPLIT>
 __global__ void __launch_bounds__(NB_THREADS, 10) k_neighbors(int64_t n, const __grid_constant__ Grid g, GridSet set,
-                                                          const int32_t *__restrict__ nbr_cells,
+                                                          const int2 *__restrict__ nbr_runs,
                                                           const float4 *__restrict__ qhi,
                                                           const float4 *__restrict__ qlo,
                                                           const double *__restrict__ xs,
@@ -846,7 +848,7 @@ __global__ void __launch_bounds__(NB_THREADS, 10) k_neighbors(int64_t n, const _
                                                           const int32_t *__restrict__ cell_start,
                                                           const int32_t *__restrict__ cell_out, int32_t *nbr,
                                                           int32_t *nbr_count, int32_t *max_count, int cap,
-                                                          int max_stage, unsigned long long *long_items,
+                                                          int max_stage, int lsplit, unsigned long long *long_items,
                                                           unsigned int long_cap, unsigned int *long_count,
                                                           unsigned int *long_max, unsigned int *work_counter)
 {
@@ -865,22 +867,30 @@ __global__ void __launch_bounds__(NB_THREADS, 10) k_neighbors(int64_t n, const _
     __shared__ int cstart[32], cpre[33], raw_cell;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int NW = NB_THREADS / 32;
+    const int room = max_stage - 32;  // candidates staged at a time
     int warp_max = 0;  // longest list this warp produced (one atomic per warp at the end)
-    for (int64_t c = blockIdx.x; c < g.ncells; c += gridDim.x) {
+    const int split = SPLIT ? 1 << lsplit : 1;  // a constant where cells are not shared: 2% of the kernel at 19 particles a cell
+    for (int64_t b = blockIdx.x; b < (SPLIT ? g.ncells << lsplit : g.ncells); b += gridDim.x) {
+        const int64_t c = SPLIT ? b >> lsplit : b;
+        const int part = SPLIT ? (int)b & (split - 1) : 0;
         const int b0 = cell_start[c], e0 = cell_start[c + 1];
-        if (b0 == e0) continue;
+        if (b0 + part * NW >= e0) continue;
         const int sys = system_of(set.cell_off, set.nsys, c);
         const Grid &G = set.nsys > 1 ? set.grids[sys] : g;
         const float Lx = (float)G.L[0], Ly = (float)G.L[1], Lz = (float)G.L[2];
         const float sq_lo = (float)G.sqcut - G.band, sq_hi = (float)G.sqcut + G.band;
         if (warp == 0) {
-            int nc = lane < 27 ? nbr_cells[c * 27 + lane] : -1;
-            if (nc >= 0) nc = (int)TBMD_IX(nc, g.ncells, BS_NBR_CELL);
-            const int cs = nc >= 0 ? cell_start[nc] : 0;
-            const int len = nc >= 0 ? cell_start[nc + 1] - cs : 0;
+            // this lane's run of neighbour cells and its particles, which are consecutive
+            int2 run = lane < 27 ? nbr_runs[c * 27 + lane] : make_int2(0, 0);
+            if (run.x < 0) run = make_int2(0, 0);
+            if (run.y > run.x) run.x = (int)TBMD_IX(run.x, g.ncells, BS_NBR_CELL);
+            const int cs = cell_start[run.x], len = cell_start[run.y] - cs;
             // raw test: an interior cell (at least 4 cells per axis, not on the boundary, so no
             // candidate cell wraps) whose candidate cells hold only particles inside the box
-            const bool any_out = __any_sync(0xffffffffu, nc >= 0 && cell_out[nc] != 0);
+            const int end = max(run.y - 1, run.x);
+            int outside = cell_out[run.x] | cell_out[min(run.x + 1, end)] | cell_out[min(run.x + 2, end)];
+            for (int k = run.x + 3; k < run.y; ++k) outside |= cell_out[k];
+            const bool any_out = __any_sync(0xffffffffu, run.y > run.x && outside != 0);
             if (lane == 0) {
                 const int64_t lc = c - (set.nsys > 1 ? set.cell_off[sys] : 0);
                 const int cx = (int)(lc % G.dims[0]), cy = (int)((lc / G.dims[0]) % G.dims[1]),
@@ -901,10 +911,7 @@ __global__ void __launch_bounds__(NB_THREADS, 10) k_neighbors(int64_t n, const _
         }
         __syncthreads();
         const int T = cpre[32];
-        // staged: the candidates and, after them, 32 far-away sentinels, so that a warp's scan
-        // needs no bounds test (a lane past T reads a sentinel, which fails the cutoff)
-        const bool staged = T + 32 <= max_stage;
-        // candidate q lies in table entry k: the largest k with cpre[k] <= q (empty entries have
+        // candidate q lies in run k: the largest k with cpre[k] <= q (empty runs have
         // cpre[k] == cpre[k + 1] and are skipped by taking the largest)
         auto entry_of = [&](int q) {
             int k = 0;
@@ -915,11 +922,16 @@ __global__ void __launch_bounds__(NB_THREADS, 10) k_neighbors(int64_t n, const _
         };
         // read before the barrier below: warp 0 rewrites raw_cell for its next cell once past it
         const bool raw = raw_cell != 0;
-        if (staged) {
-            for (int q = threadIdx.x; q < T + 32; q += NB_THREADS) {
-                if (q < T) {
-                    const int k = entry_of(q);
-                    const int t = (int)TBMD_IX(cstart[k] + (q - cpre[k]), n, BS_CANDIDATE);
+#pragma unroll 1
+        for (int base = 0; base < T; base += room) {
+            // staged: candidates base .. base + m - 1 and, after them, 32 far-away sentinels, so that a
+            // warp's scan needs no bounds test (a lane past the end reads a sentinel, which fails the cutoff)
+            const int m = min(room, T - base);
+            const bool last = base + m == T;
+            for (int q = threadIdx.x; q < m + 32; q += NB_THREADS) {
+                if (q < m) {
+                    const int k = entry_of(base + q);
+                    const int t = (int)TBMD_IX(cstart[k] + (base + q - cpre[k]), n, BS_CANDIDATE);
                     (void)TBMD_IX(q, max_stage, BS_STAGE);
                     float4 h = qhi[t];
                     h.w = __int_as_float(t);  // the sorted index rides in the unused w
@@ -930,169 +942,179 @@ __global__ void __launch_bounds__(NB_THREADS, 10) k_neighbors(int64_t n, const _
                     slo[q] = make_float4(0.f, 0.f, 0.f, 0.f);
                 }
             }
-        }
-        __syncthreads();
-        // particle sl scans the candidates after it, so earlier particles have longer scans: the warps
-        // take them in a snake order (0 1 2 3 3 2 1 0 0 1 ...) so that their totals even out before the
-        // barrier at the end of the cell
-        for (int it = 0; it * NW < e0 - b0; ++it) {
-            const int sl = it * NW + ((it & 1) ? NW - 1 - warp : warp);
-            if (sl >= e0 - b0) continue;
-            const int s = b0 + sl;  // cell c comes first in the candidate order: q = sl
-            const float4 oh = staged ? shi[sl] : qhi[s], ol = staged ? slo[sl] : qlo[s];
-            int cnt = 0;
-            int32_t *dst = nbr + (int64_t)s * cap;
-            // one candidate per lane and iteration; the pass mask compacts the list in order
-            auto emit = [&](bool pass, int t) {
-                const unsigned m = __ballot_sync(0xffffffffu, pass);
-                const int off = cnt + __popc(m & ((1u << lane) - 1u));
-                if (pass && off < cap) dst[off] = t;
-                cnt += __popc(m);
-            };
-            auto exact = [&](int t) {
-                return sqdist_periodic(xs[s], ys[s], zs[s], xs[t], ys[t], zs[t], G) <= G.sqcut;
-            };
-            if (staged && raw) {
-                // every coordinate lies in the box: the hi parts alone are within 2^-24 L, and the
-                // periodic form is the raw distance (each axis under 2 cells <= L / 2).  Two
-                // iterations per trip let the next candidate's loads and test overlap this one's
-                // compaction (1% faster than one).
-#pragma unroll 2
-                for (int q0 = sl + 1; q0 < T; q0 += 32) {
-                    const int q = q0 + lane;
-                    const float4 h = shi[q];
-                    const int t = __float_as_int(h.w);
-                    const float dx = h.x - oh.x, dy = h.y - oh.y, dz = h.z - oh.z;
-                    const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                    bool pass = d2 <= sq_lo;
-                    if (!pass && d2 <= sq_hi) pass = exact(t);
-                    emit(pass, t);
+            __syncthreads();
+            // particle sl scans the candidates after it, so earlier particles have longer scans: the warps
+            // take them in a snake order (0 1 2 3 3 2 1 0 0 1 ...) so that their totals even out before the
+            // barrier at the end of the cell
+            for (int it = part; it * NW < e0 - b0; it += split) {
+                const int sl = it * NW + ((it & 1) ? NW - 1 - warp : warp);
+                if (sl >= e0 - b0) continue;
+                const int s = b0 + sl;  // cell c comes first in the candidate order: q = sl
+                float4 oh, ol;
+                int cnt = 0;
+                if (base == 0 && sl < m) {
+                    oh = shi[sl];
+                    ol = slo[sl];
+                } else {
+                    oh = qhi[s];
+                    ol = qlo[s];
+                    if (base > 0) cnt = nbr_count[s];
                 }
-            } else if (staged) {
+                int32_t *dst = nbr + (int64_t)s * cap;
+                // one candidate per lane and iteration; the pass mask compacts the list in order
+                auto emit = [&](bool pass, int t) {
+                    const unsigned mk = __ballot_sync(0xffffffffu, pass);
+                    const int off = cnt + __popc(mk & ((1u << lane) - 1u));
+                    if (pass && off < cap) dst[off] = t;
+                    cnt += __popc(mk);
+                };
+                auto exact = [&](int t) {
+                    return sqdist_periodic(xs[s], ys[s], zs[s], xs[t], ys[t], zs[t], G) <= G.sqcut;
+                };
+                const int first = max(sl + 1 - base, 0);
+                if (raw) {
+                    // every coordinate lies in the box: the hi parts alone are within 2^-24 L, and the
+                    // periodic form is the raw distance (each axis under 2 cells <= L / 2).  Two
+                    // iterations per trip let the next candidate's loads and test overlap this one's
+                    // compaction (1% faster than one).
 #pragma unroll 2
-                for (int q0 = sl + 1; q0 < T; q0 += 32) {
-                    const int q = q0 + lane;
-                    const float4 h = shi[q], l = slo[q];
-                    const int t = __float_as_int(h.w);
-                    const float dx = (h.x - oh.x) + (l.x - ol.x), dy = (h.y - oh.y) + (l.y - ol.y),
-                                dz = (h.z - oh.z) + (l.z - ol.z);
-                    const float ax = fabsf(dx), ay = fabsf(dy), az = fabsf(dz);
-                    const float mx = fminf(ax, Lx - ax), my = fminf(ay, Ly - ay), mz = fminf(az, Lz - az);
-                    const float d2 = fmaf(mx, mx, fmaf(my, my, mz * mz));
-                    bool pass = d2 <= sq_lo;
-                    if (!pass && d2 <= sq_hi) pass = exact(t);
-                    emit(pass, t);
-                }
-            } else {
-                // more candidates than the staging holds: read them from global memory
-                for (int q0 = sl + 1; q0 < T; q0 += 32) {
-                    const int q = q0 + lane;
-                    bool pass = false;
-                    int t = 0;
-                    if (q < T) {
-                        const int k = entry_of(q);
-                        t = (int)TBMD_IX(cstart[k] + (q - cpre[k]), n, BS_CANDIDATE);
-                        const float4 h = qhi[t];
-                        float d2;
-                        if (raw) {
-                            const float dx = h.x - oh.x, dy = h.y - oh.y, dz = h.z - oh.z;
-                            d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                        } else {
-                            const float4 l = qlo[t];
-                            const float dx = (h.x - oh.x) + (l.x - ol.x), dy = (h.y - oh.y) + (l.y - ol.y),
-                                        dz = (h.z - oh.z) + (l.z - ol.z);
-                            const float ax = fabsf(dx), ay = fabsf(dy), az = fabsf(dz);
-                            const float mx = fminf(ax, Lx - ax), my = fminf(ay, Ly - ay),
-                                        mz = fminf(az, Lz - az);
-                            d2 = fmaf(mx, mx, fmaf(my, my, mz * mz));
-                        }
-                        pass = d2 <= sq_lo;
+                    for (int q0 = first; q0 < m; q0 += 32) {
+                        const float4 h = shi[q0 + lane];
+                        const int t = __float_as_int(h.w);
+                        const float dx = h.x - oh.x, dy = h.y - oh.y, dz = h.z - oh.z;
+                        const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                        bool pass = d2 <= sq_lo;
                         if (!pass && d2 <= sq_hi) pass = exact(t);
+                        emit(pass, t);
                     }
-                    emit(pass, t);
+                } else {
+#pragma unroll 2
+                    for (int q0 = first; q0 < m; q0 += 32) {
+                        const float4 h = shi[q0 + lane], l = slo[q0 + lane];
+                        const int t = __float_as_int(h.w);
+                        const float dx = (h.x - oh.x) + (l.x - ol.x), dy = (h.y - oh.y) + (l.y - ol.y),
+                                    dz = (h.z - oh.z) + (l.z - ol.z);
+                        const float ax = fabsf(dx), ay = fabsf(dy), az = fabsf(dz);
+                        const float mx = fminf(ax, Lx - ax), my = fminf(ay, Ly - ay), mz = fminf(az, Lz - az);
+                        const float d2 = fmaf(mx, mx, fmaf(my, my, mz * mz));
+                        bool pass = d2 <= sq_lo;
+                        if (!pass && d2 <= sq_hi) pass = exact(t);
+                        emit(pass, t);
+                    }
+                }
+                if (lane == 0) nbr_count[s] = cnt;
+                if (!last) continue;
+                warp_max = cnt > warp_max ? cnt : warp_max;
+                // a list longer than one chunk: queue its chunk pairs (I <= J) for the triplet kernel
+                const int M = cnt < cap ? cnt : cap;
+                if (M > P3_CHUNK) {
+                    const unsigned int nch = (unsigned int)((M + P3_CHUNK - 1) / P3_CHUNK);
+                    const unsigned int nitems = nch * (nch + 1) / 2;
+                    unsigned int at = 0;
+                    if (lane == 0) {
+                        at = atomicAdd(long_count, nitems);
+                        atomicMax(long_max, at + nitems);
+                    }
+                    at = __shfl_sync(0xffffffffu, at, 0);
+                    for (unsigned int k = lane; k < nitems; k += 32) {
+                        unsigned int I = 0, r = k;
+                        while (r >= nch - I) {
+                            r -= nch - I;
+                            ++I;
+                        }
+                        if (at + k < long_cap)
+                            long_items[at + k] = ((unsigned long long)(unsigned int)s << 32) | (I << 16) | (I + r);
+                    }
                 }
             }
-            if (lane == 0) nbr_count[s] = cnt;
-            warp_max = cnt > warp_max ? cnt : warp_max;
-            // a list longer than one chunk: queue its chunk pairs (I <= J) for the triplet kernel
-            const int M = cnt < cap ? cnt : cap;
-            if (M > P3_CHUNK) {
-                const unsigned int nch = (unsigned int)((M + P3_CHUNK - 1) / P3_CHUNK);
-                const unsigned int nitems = nch * (nch + 1) / 2;
-                unsigned int base = 0;
-                if (lane == 0) {
-                    base = atomicAdd(long_count, nitems);
-                    atomicMax(long_max, base + nitems);
-                }
-                base = __shfl_sync(0xffffffffu, base, 0);
-                for (unsigned int k = lane; k < nitems; k += 32) {
-                    unsigned int I = 0, r = k;
-                    while (r >= nch - I) {
-                        r -= nch - I;
-                        ++I;
-                    }
-                    if (base + k < long_cap)
-                        long_items[base + k] = ((unsigned long long)(unsigned int)s << 32) | (I << 16) | (I + r);
-                }
-            }
+            __syncthreads();
         }
-        __syncthreads();
     }
     if (lane == 0 && warp_max > 0) atomicMax(max_count, warp_max);
 }
 
-// Staging capacity: 1.6 times the expected candidate count (14 of the 27 cells have id >= c on
-// average), at least 256, at most 4096 (144 KiB).
+// Staging capacity (32 sentinels included): all candidates of a cell whose neighbours all have higher ids,
+// as those of the low faces have in a periodic box (27 cells, or 9, 3 or 1 on one-cell axes), plus 3.5
+// standard deviations; at most 1,024, so that seven blocks fit an SM.  Cells with more candidates stage
+// them in turns.
 int neighbor_stage_cap(const Grid &g, int64_t n)
 {
     const double mean = (double)n / (double)g.ncells;
     const int cells = (g.dims[0] == 1 ? 1 : 3) * (g.dims[1] == 1 ? 1 : 3) * (g.dims[2] == 1 ? 1 : 3);
-    int want = (int)(1.6 * mean * (cells / 2 + 1)) + 128;
-    want = (want + 31) / 32 * 32;
-    return want < 256 ? 256 : (want > 4096 ? 4096 : want);
+    const double all = mean * cells;
+    const double want = all + 3.5 * sqrt(all) + 32.0;
+    const int cap = want < 1024.0 ? ((int)want + 31) / 32 * 32 : 1024;
+    return cap < 256 ? 256 : cap;
 }
 
-// Per cell of grid g (cells numbered from cell0), its neighbour cells with id >= its own id in
-// increasing order, -1 padded to 27 entries.
-void neighbor_cell_table(const Grid &g, int64_t cell0, int32_t *out)
+// Blocks per cell: the particles of a cell over up to 8 blocks while there are fewer than four blocks an SM.
+// The logarithm of that number.
+static int neighbor_split(int64_t n, int64_t ncells, int sms)
 {
-    const int ox = g.dims[0] == 1 ? 0 : 1, oy = g.dims[1] == 1 ? 0 : 1, oz = g.dims[2] == 1 ? 0 : 1;
-    for (int64_t lc = 0; lc < g.ncells; ++lc) {
-        const int cx = (int)(lc % g.dims[0]), cy = (int)((lc / g.dims[0]) % g.dims[1]),
-                  cz = (int)(lc / ((int64_t)g.dims[0] * g.dims[1]));
-        int32_t ids[27];
-        int K = 0;
-        for (int dz = -oz; dz <= oz; ++dz)
-            for (int dy = -oy; dy <= oy; ++dy)
-                for (int dx = -ox; dx <= ox; ++dx) {
-                    const int nx = (cx + dx + g.dims[0]) % g.dims[0];
-                    const int ny = (cy + dy + g.dims[1]) % g.dims[1];
-                    const int nz = (cz + dz + g.dims[2]) % g.dims[2];
-                    const int64_t nc = (int64_t)(nz * g.dims[1] + ny) * g.dims[0] + nx;
-                    if (nc < lc) continue;
-                    int q = K++;
-                    while (q > 0 && ids[q - 1] > nc + cell0) {
-                        ids[q] = ids[q - 1];
-                        --q;
-                    }
-                    ids[q] = (int32_t)(nc + cell0);
-                }
-        int32_t *row = out + (cell0 + lc) * 27;
-        for (int k = 0; k < 27; ++k) row[k] = k < K ? ids[k] : -1;
-    }
+    int l = 0;
+    while (l < 3 && (ncells << l) < 4ll * sms && n > (4 * ncells << l)) ++l;
+    return l;
 }
 
-cudaError_t launch_neighbors(int64_t n, const Grid &g, const GridSet &set, const int32_t *nbr_cells, int max_stage,
+// Per cell, its neighbour cells with id >= its own in increasing order, as runs of consecutive ids
+// [first, end) padded with (-1, -1) to 27: an interior cell has five (its own row and the next one, and
+// three rows of the layer above).
+__global__ void k_neighbor_table(const __grid_constant__ Grid g, GridSet set, int2 *__restrict__ out)
+{
+    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= g.ncells) return;
+    const int sys = system_of(set.cell_off, set.nsys, c);
+    const Grid &G = set.nsys > 1 ? set.grids[sys] : g;
+    const int64_t cell0 = set.nsys > 1 ? set.cell_off[sys] : 0, lc = c - cell0;
+    const int ox = G.dims[0] == 1 ? 0 : 1, oy = G.dims[1] == 1 ? 0 : 1, oz = G.dims[2] == 1 ? 0 : 1;
+    const int cx = (int)(lc % G.dims[0]), cy = (int)((lc / G.dims[0]) % G.dims[1]),
+              cz = (int)(lc / ((int64_t)G.dims[0] * G.dims[1]));
+    int ids[27];
+    int K = 0;
+    for (int dz = -oz; dz <= oz; ++dz)
+        for (int dy = -oy; dy <= oy; ++dy)
+            for (int dx = -ox; dx <= ox; ++dx) {
+                const int nx = (cx + dx + G.dims[0]) % G.dims[0];
+                const int ny = (cy + dy + G.dims[1]) % G.dims[1];
+                const int nz = (cz + dz + G.dims[2]) % G.dims[2];
+                const int64_t nc = (int64_t)(nz * G.dims[1] + ny) * G.dims[0] + nx;
+                if (nc < lc) continue;
+                int q = K++;
+                while (q > 0 && ids[q - 1] > nc) {
+                    ids[q] = ids[q - 1];
+                    --q;
+                }
+                ids[q] = (int)nc;
+            }
+    int r = 0;
+    for (int k = 0; k < K;) {
+        int e = k + 1;
+        while (e < K && ids[e] == ids[e - 1] + 1) ++e;
+        out[c * 27 + r++] = make_int2((int)cell0 + ids[k], (int)cell0 + ids[e - 1] + 1);
+        k = e;
+    }
+    for (; r < 27; ++r) out[c * 27 + r] = make_int2(-1, -1);
+}
+
+cudaError_t launch_neighbor_table(const Grid &g, const GridSet &set, int2 *out, cudaStream_t st)
+{
+    k_neighbor_table<<<(unsigned)((g.ncells + 127) / 128), 128, 0, st>>>(g, set, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_neighbors(int64_t n, const Grid &g, const GridSet &set, const int2 *nbr_runs, int max_stage,
                              CellBufs &cb, cudaStream_t st)
 {
     const size_t smem = (size_t)max_stage * NB_STAGE_BYTES;
-    int64_t blocks = g.ncells < 65535 * 16 ? g.ncells : 65535 * 16;
+    const int lsplit = neighbor_split(n, g.ncells, cb.sms);
+    int64_t blocks = g.ncells << lsplit < 65535 * 16 ? g.ncells << lsplit : 65535 * 16;
     cudaError_t e = cudaMemsetAsync(cb.long_count, 0, sizeof(unsigned int), st);
     if (e != cudaSuccess) return e;
-    k_neighbors<<<(unsigned)blocks, NB_THREADS, smem, st>>>(n, g, set, nbr_cells, cb.qhi, cb.qlo, cb.xs, cb.ys, cb.zs,
+    auto kern = lsplit ? k_neighbors<true> : k_neighbors<false>;
+    kern<<<(unsigned)blocks, NB_THREADS, smem, st>>>(n, g, set, nbr_runs, cb.qhi, cb.qlo, cb.xs, cb.ys, cb.zs,
                                                             cb.cell_start, cb.cell_out, cb.nbr, cb.nbr_count,
                                                             cb.max_count, cb.cap,
-                                                            max_stage, cb.long_items, (unsigned int)cb.long_cap,
+                                                            max_stage, lsplit, cb.long_items, (unsigned int)cb.long_cap,
                                                             cb.long_count, cb.long_max, cb.work_counter);
     return cudaGetLastError();
 }
@@ -1875,9 +1897,12 @@ static cudaError_t plan_p3bca_t(bool energy, int cap, int warps, P3Plan *plan)
 
 cudaError_t plan_p3bca(bool mixed, bool dual, bool energy, int cap, int warps, P3Plan *plan)
 {
-    // the neighbour kernel's largest staging size (4096 candidates), set once outside any capture
-    cudaError_t e0 = cudaFuncSetAttribute(k_neighbors, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)(4096 * NB_STAGE_BYTES));
+    // the neighbour kernel's largest staging size (1,024 candidates), set once outside any capture
+    cudaError_t e0 = cudaFuncSetAttribute(k_neighbors<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)(1024 * NB_STAGE_BYTES));
+    if (e0 == cudaSuccess)
+        e0 = cudaFuncSetAttribute(k_neighbors<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(1024 * NB_STAGE_BYTES));
     if (e0 != cudaSuccess) return e0;
     if (dual) {
         if (mixed) return plan_p3bca_t<Dual<float>>(energy, cap, warps, plan);
