@@ -49,6 +49,20 @@ struct DevBuf {
     T *as() const { return (T *)p; }
 };
 
+// Everything that a step's launches take by value: a graph holds them as they were at its capture.
+// Zeroed before it is filled, since it is compared bytewise.
+struct GraphKey {
+    Grid grid;
+    GridSet gset;
+    CellBufs cb;
+    P3Plan plan;
+    SweepWork sweep;
+    PtDev pairs;
+    const void *table, *state, *step_counts, *partial;
+    int64_t n;
+    int max_stage, sweep_grid;
+};
+
 }  // namespace
 
 struct tbmd_ctx {
@@ -148,7 +162,8 @@ struct tbmd_ctx {
     int cur_phase = -1;
     int cur_phase_launch0 = 0;
 
-    // graph of one step
+    // graph of one step, and what the step's launches were given when it was captured
+    GraphKey graph_key{}, last_key{};
     cudaGraphExec_t gexec = nullptr;
     bool graph_valid = false;
     int graph_launches_per_step = 0;
@@ -581,6 +596,16 @@ static tbmd_status enqueue_forces(tbmd_ctx *ctx, int64_t n, Pos pos, Out out, bo
 static Pos state_pos(tbmd_ctx *c) { return Pos{c->s[0], c->s[1], c->s[2], nullptr, nullptr, nullptr}; }
 static Out state_out(tbmd_ctx *c) { return Out{c->s[10], c->s[11], c->s[12], nullptr, nullptr, nullptr}; }
 
+// The event that the positions of a step are final: an external event node while a graph is captured.
+static cudaError_t record_positions(tbmd_ctx *ctx, cudaStream_t st)
+{
+    cudaStreamCaptureStatus cap;
+    const cudaError_t e = cudaStreamIsCapturing(st, &cap);
+    if (e != cudaSuccess) return e;
+    return cudaEventRecordWithFlags(ctx->pos_event, st,
+                                    cap == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault);
+}
+
 // One Simulation::Start iteration: predictor, forces, update, per-step count.
 static tbmd_status enqueue_step(tbmd_ctx *ctx, cudaStream_t st, int *nl)
 {
@@ -591,7 +616,7 @@ static tbmd_status enqueue_step(tbmd_ctx *ctx, cudaStream_t st, int *nl)
         CellBufs &cb = ctx->cb;
         phase_mark(ctx, st, PH_CELLS, *nl);  // the predictor runs inside the cell build
         CK(launch_step_cells(n, s, ctx->cfg.dt, ctx->grid, cb, st, nl));
-        if (ctx->pos_event) CK(cudaEventRecordWithFlags(ctx->pos_event, st, cudaEventRecordExternal));
+        if (ctx->pos_event) CK(record_positions(ctx, st));
         phase_mark(ctx, st, PH_NEIGHBORS, *nl);
         CK(launch_neighbors(n, ctx->grid, ctx->gset, ctx->ncell_tab.as<int2>(), ctx->max_stage, cb, st));
         *nl += 1;
@@ -610,7 +635,7 @@ static tbmd_status enqueue_step(tbmd_ctx *ctx, cudaStream_t st, int *nl)
     phase_mark(ctx, st, PH_PREDICTOR, *nl);
     CK(launch_predictor(n, s[0], s[1], s[2], s[3], s[4], s[5], s[6], ctx->cfg.dt, st));
     *nl += 1;
-    if (ctx->pos_event) CK(cudaEventRecordWithFlags(ctx->pos_event, st, cudaEventRecordExternal));
+    if (ctx->pos_event) CK(record_positions(ctx, st));
     // forces of the step's count go to count_cur; the no-cutoff count C(n,3) is added by k_add_u64
     tbmd_status r = enqueue_forces(ctx, n, state_pos(ctx), state_out(ctx), false, nullptr, count_ptr(ctx), st, nl);
     if (r != TBMD_OK) return r;
@@ -620,6 +645,28 @@ static tbmd_status enqueue_step(tbmd_ctx *ctx, cudaStream_t st, int *nl)
     *nl += 2;
     phase_mark(ctx, st, PH_END, *nl);
     return TBMD_OK;
+}
+
+static void fill_graph_key(tbmd_ctx *ctx, GraphKey &k)
+{
+    std::memset((void *)&k, 0, sizeof k);
+    k.n = ctx->n;
+    k.state = ctx->state.p;
+    k.step_counts = ctx->step_counts.p;
+    if (is_p3bca_cut(ctx)) {
+        k.grid = ctx->grid;
+        k.gset = ctx->gset;
+        k.cb = ctx->cb;
+        k.plan = ctx->plan;
+        k.table = ctx->ncell_tab.p;
+        k.max_stage = ctx->max_stage;
+    } else if (use_pairs(ctx, ctx->n, false)) {
+        k.pairs = ctx->pt_dev;
+    } else {
+        k.sweep = single_sweep(ctx);
+        k.partial = ctx->partial.p;
+        k.sweep_grid = ctx->sweep_grid;
+    }
 }
 
 static tbmd_status build_graph(tbmd_ctx *ctx)
@@ -1087,21 +1134,27 @@ static tbmd_status run_steps(tbmd_ctx *ctx, int32_t iterations, uint64_t *counts
     unsigned long long *hcounts = (unsigned long long *)((char *)ctx->hstep + 32);  // 8-byte aligned
     tbmd_status st = TBMD_OK;
     for (int attempt = 0; attempt < 4; ++attempt) {
-        void *before[5] = {ctx->state.p, ctx->nbr_buf.p, ctx->cell_n.p, ctx->prefix.p, ctx->long_buf.p};
         st = prepare(ctx, n, false, false);
         if (st != TBMD_OK) return st;
-        void *after[5] = {ctx->state.p, ctx->nbr_buf.p, ctx->cell_n.p, ctx->prefix.p, ctx->long_buf.p};
-        if (std::memcmp(before, after, sizeof before)) invalidate_graph(ctx);
+        // a graph of other arguments (another domain, moved buffers) is not replayed
+        GraphKey key;
+        fill_graph_key(ctx, key);
+        if (std::memcmp(&key, &ctx->graph_key, sizeof key) != 0) invalidate_graph(ctx);
+        // few steps with arguments not seen in the last call (a new particle set) are launched one by one: a
+        // capture costs more than it saves
+        const bool capture = ctx->graph_valid || iterations >= 8 || std::memcmp(&key, &ctx->last_key, sizeof key) == 0;
+        ctx->last_key = key;
         CK(cudaMemsetAsync(ctx->scalars.as<char>() + 8, 0, 56, ctx->stream));
         if (cut) {
             CK(ctx->snapshot.ensure(sizeof(double) * 9 * (size_t)n));
             CK(cudaMemcpyAsync(ctx->snapshot.p, ctx->s[0], sizeof(double) * 9 * n, cudaMemcpyDeviceToDevice,
                                ctx->stream));
         }
-        if (ctx->cfg.use_graph && !ctx->profiling) {
+        if (ctx->cfg.use_graph && !ctx->profiling && capture) {
             if (!ctx->graph_valid) {
                 st = build_graph(ctx);
                 if (st != TBMD_OK) return st;
+                ctx->graph_key = key;
             }
             for (int it = 0; it < iterations; ++it) CK(cudaGraphLaunch(ctx->gexec, ctx->stream));
             ctx->launches += (uint64_t)ctx->graph_launches_per_step * iterations;
