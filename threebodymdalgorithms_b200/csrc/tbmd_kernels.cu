@@ -1515,11 +1515,19 @@ struct P3MaxReg<Dual<double>, E> {
     static constexpr int value = E ? 168 : 128;
 };
 
-template <class S, bool ENERGY>
+// PARTS: the pair steps of a long list are dealt out to up to 1 << lparts work items (part p takes the steps
+// p, p + parts, ... of every block pair), each staging and flushing the slots for itself.  For systems whose
+// time is that of the longest list: 1,000 particles at density 1, cutoff 2, 30 -> 18 us (FP64) and 20.5 -> 18
+// us (mixed).  The empty parts of short lists cost a counter increment each, so the line is drawn at 2/5 of
+// the resident warps (1,180 and 1,660 particles); 2,900 particles lose by it (27 -> 30 and 20 -> 31 us).
+template <class S, bool ENERGY, bool PARTS>
 __global__ void __maxnreg__((P3MaxReg<S, ENERGY>::value))
     k_p3bca(int64_t n, const __grid_constant__ Grid g, GridSet set, CellBufs cb, double nu_d, double *energy_out,
-            unsigned long long *count_out)
+            unsigned long long *count_out, int lparts)
 {
+    int parts = 1, part = 0;  // of the current item
+    // how many parts an item of M slots is worth: about one per four pair steps, at most 1 << lparts
+    auto parts_of = [&](int M) { return min(1 << lparts, 1 << max(0, 23 - __clz(M * M))); };
     using Acc = typename Traits<S>::Acc;
     using L = SlotLayout<S>;
     constexpr int SL = 2 * P3_CHUNK;  // staged slots per warp: one or two chunks of a half list
@@ -1659,8 +1667,12 @@ __global__ void __maxnreg__((P3MaxReg<S, ENERGY>::value))
                     // pairs inside block A: circular diagonals; y = (lane + d) mod mA advances by one per
                     // diagonal (lanes past the block cycle through valid slots and are masked)
                     int y = own ? lane : 0;
-                    for (int d = 1; 2 * d <= mA; ++d) {
-                        y = y + 1 == mA ? 0 : y + 1;
+                    if (PARTS) y = (y + 1 + part + (mA << 3) - parts) % mA;
+                    for (int d = 1 + (PARTS ? part : 0); 2 * d <= mA; d += parts) {
+                        if (PARTS)
+                            y = (y + parts) % mA;
+                        else
+                            y = y + 1 == mA ? 0 : y + 1;
                         const bool act = own && (2 * d < mA || lane < d);
                         const int b = A0 + y;
                         const PGrad<S> gb = pair(act, b);
@@ -1674,7 +1686,7 @@ __global__ void __maxnreg__((P3MaxReg<S, ENERGY>::value))
                     // a full block: 32 steps of distinct partners; a short block: mB steps in lane
                     // groups
                     if (mB == 32) {
-                        for (int t = 0; t < 32; ++t) {
+                        for (int t = PARTS ? part : 0; t < 32; t += parts) {
                             const int y = (lane + t) & 31;
                             const bool act = own && y < mB;
                             const int b = B0 + (y < mB ? y : 0);
@@ -1689,8 +1701,8 @@ __global__ void __maxnreg__((P3MaxReg<S, ENERGY>::value))
                         // copy l (partner l mod mB), and the copies of a partner sum down the lanes
                         // l, l + mB, l + 2 mB, ... into lane l < mB.
                         const int g = lane / mB, j = lane - g * mB;
-                        int y = j;
-                        for (int t = 0; t < mB; ++t) {
+                        int y = PARTS ? (j + part) % mB : j;
+                        for (int t = PARTS ? part : 0; t < mB; t += parts) {
                             const int b = B0 + y;
                             const PGrad<S> gb = pair(own, b);
                             if (own) {
@@ -1700,7 +1712,10 @@ __global__ void __maxnreg__((P3MaxReg<S, ENERGY>::value))
                                     pgrad_add_copy(W, (int)TBMD_IX((g - 1) * mB + y, P3_COPIES, BS_SLOT), gb);
                             }
                             __syncwarp();
-                            y = y + 1 == mB ? 0 : y + 1;
+                            if (PARTS)
+                                y = (y + parts) % mB;
+                            else
+                                y = y + 1 == mB ? 0 : y + 1;
                         }
                         Grad<S> c = W.copy(lane);
                         W.set_copy(lane, grad_zero<S>());
@@ -1757,7 +1772,8 @@ __global__ void __maxnreg__((P3MaxReg<S, ENERGY>::value))
         // forces kernel gains 0.8% at C3 and C4 from it, and the mixed forces kernel loses 3.5%, so it
         // keeps the two loops below.
         for (int kind = 0; kind < 2; ++kind) {
-            const unsigned int lim = kind == 0 ? (unsigned int)n : min(*cb.long_count, (unsigned int)cb.long_cap);
+            const unsigned int lim =
+                (kind == 0 ? (unsigned int)n : min(*cb.long_count, (unsigned int)cb.long_cap)) << (PARTS ? lparts : 0);
             unsigned int w = 0;
             if (lane == 0) w = atomicAdd(cb.work_counter + kind, 1u);
             w = __shfl_sync(0xffffffffu, w, 0);
@@ -1765,6 +1781,10 @@ __global__ void __maxnreg__((P3MaxReg<S, ENERGY>::value))
                 unsigned int wn = 0;
                 if (lane == 0) wn = atomicAdd(cb.work_counter + kind, 1u);
                 int s, offI = 0, mI, offJ = 0, mJ = 0;
+                if (PARTS) {
+                    part = (int)w & ((1 << lparts) - 1);
+                    w >>= lparts;
+                }
                 if (kind == 0) {
                     s = (int)w;
                     mI = min(cb.nbr_count[s], cap);
@@ -1781,7 +1801,8 @@ __global__ void __maxnreg__((P3MaxReg<S, ENERGY>::value))
                         mJ = min(P3_CHUNK, M - offJ);
                     }
                 }
-                if (mI + mJ > 1) item(s, offI, mI, offJ, mJ);
+                if (PARTS) parts = parts_of(mI + mJ);
+                if (mI + mJ > 1 && (!PARTS || part < parts)) item(s, offI, mI, offJ, mJ);
                 w = __shfl_sync(0xffffffffu, wn, 0);
             }
         }
@@ -1790,28 +1811,38 @@ __global__ void __maxnreg__((P3MaxReg<S, ENERGY>::value))
         unsigned int w = 0;
         if (lane == 0) w = atomicAdd(cb.work_counter, 1u);
         w = __shfl_sync(0xffffffffu, w, 0);
-        while ((int64_t)w < n) {
+        while ((int64_t)w < (PARTS ? n << lparts : n)) {
             unsigned int wn = 0;
             if (lane == 0) wn = atomicAdd(cb.work_counter, 1u);
+            if (PARTS) {
+                part = (int)w & ((1 << lparts) - 1);
+                w >>= lparts;
+            }
             const int s = (int)w;
             const int M = min(cb.nbr_count[s], cap);
-            if (M <= P3_CHUNK && M > 1) item(s, 0, M, 0, 0);
+            if (PARTS) parts = parts_of(M);
+            if (M <= P3_CHUNK && M > 1 && (!PARTS || part < parts)) item(s, 0, M, 0, 0);
             w = __shfl_sync(0xffffffffu, wn, 0);
         }
         // longer lists: the chunk-pair items the neighbour kernel queued
-        const unsigned int nlong = min(*cb.long_count, (unsigned int)cb.long_cap);
+        const unsigned int nlong = min(*cb.long_count, (unsigned int)cb.long_cap) << (PARTS ? lparts : 0);
         if (lane == 0) w = atomicAdd(cb.work_counter + 1, 1u);
         w = __shfl_sync(0xffffffffu, w, 0);
         while (w < nlong) {
             unsigned int wn = 0;
             if (lane == 0) wn = atomicAdd(cb.work_counter + 1, 1u);
+            if (PARTS) {
+                part = (int)w & ((1 << lparts) - 1);
+                w >>= lparts;
+            }
             const unsigned long long it = cb.long_items[w];
             const int s = (int)TBMD_IX((int64_t)(it >> 32), n, BS_LONG_ITEM), I = (int)((it >> 16) & 0xffffu),
                       J = (int)(it & 0xffffu);
             const int M = min(cb.nbr_count[s], cap);
             const int mI = min(P3_CHUNK, M - I * P3_CHUNK);
             const int mJ = J != I ? min(P3_CHUNK, M - J * P3_CHUNK) : 0;
-            item(s, I * P3_CHUNK, mI, J * P3_CHUNK, mJ);
+            if (PARTS) parts = parts_of(mI + mJ);
+            if (!PARTS || part < parts) item(s, I * P3_CHUNK, mI, J * P3_CHUNK, mJ);
             w = __shfl_sync(0xffffffffu, wn, 0);
         }
     }
@@ -1883,8 +1914,10 @@ static cudaError_t plan_p3bca_t(bool energy, int cap, int warps, P3Plan *plan)
     while (warps > 1 && per_warp * warps > smem_cap) --warps;
     if (per_warp * warps > smem_cap) return cudaErrorInvalidValue;
     const size_t smem = per_warp * warps;
-    auto kern = energy ? k_p3bca<S, true> : k_p3bca<S, false>;
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+    auto kern = energy ? k_p3bca<S, true, false> : k_p3bca<S, false, false>;
+    auto kern_parts = energy ? k_p3bca<S, true, true> : k_p3bca<S, false, true>;
+    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess ||
+        (e = cudaFuncSetAttribute(kern_parts, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
         return e;
     int per_sm = 0;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, smem)) != cudaSuccess) return e;
@@ -1917,8 +1950,13 @@ static cudaError_t launch_p3bca_t(bool energy, int64_t n, const Grid &g, const G
                                   double *eo, unsigned long long *co, const P3Plan &plan, cudaStream_t st)
 {
     // the work counters were armed by the neighbour kernel of the same step
-    auto kern = energy ? k_p3bca<S, true> : k_p3bca<S, false>;
-    kern<<<plan.grid, plan.warps * 32, plan.smem, st>>>(n, g, set, cb, nu, eo, co);
+    const int lparts = 5 * n <= 2 * (int64_t)plan.grid * plan.warps ? 3 : 0;
+    if (lparts)
+        (energy ? k_p3bca<S, true, true> : k_p3bca<S, false, true>)<<<plan.grid, plan.warps * 32, plan.smem, st>>>(
+            n, g, set, cb, nu, eo, co, lparts);
+    else
+        (energy ? k_p3bca<S, true, false> : k_p3bca<S, false, false>)<<<plan.grid, plan.warps * 32, plan.smem, st>>>(
+            n, g, set, cb, nu, eo, co, 0);
     return cudaGetLastError();
 }
 
