@@ -1,8 +1,8 @@
-"""The mixed no-cutoff forces as a product of pair tensors, at the sizes where its tiling can go wrong: the
-edges of the 42-particle row blocks, of the 84-particle column blocks and of the ranges of k, against the
-FP64 oracle.
+"""The no-cutoff forces as a product of pair tensors, at the sizes where its tiling can go wrong: the edges of
+the row blocks (42 particles mixed, 32 FP64), of the column blocks (84, 64) and of the ranges of k, against
+the FP64 oracle.
 
-Tolerance: an entry of G = T T is cut off twice and rounded at most 48 times (2 * 2^-23 + 48 * 2^-24 of its
+Tolerance, FP64: 1e-12, as for every FP64 evaluation.  Mixed: an entry of G = T T is cut off twice and rounded at most 48 times (2 * 2^-23 + 48 * 2^-24 of its
 partial sums, 3.1e-6), and its contraction with dT/dr rounds fewer than 18 times (1.1e-6)."""
 import numpy as np
 import pytest
@@ -12,7 +12,8 @@ from threebodymdalgorithms_b200 import Context
 
 pytestmark = pytest.mark.gpu
 
-TOL = 4.2e-6
+TOL = {"mixed": 4.2e-6, "fp64": 1e-12}
+PRECISIONS = ["mixed", "fp64"]
 
 
 def lattice(n, seed, scale=1.0):
@@ -28,27 +29,29 @@ def rel(a, b):
     return float(np.linalg.norm(a - b) / np.linalg.norm(b))
 
 
+@pytest.mark.parametrize("precision", PRECISIONS)
 @pytest.mark.parametrize("algo", ["auta", "nata"])
-@pytest.mark.parametrize("n", [128, 129, 167, 168, 169, 252, 253, 383, 385, 420, 513, 769])
-def test_pair_tensor_forces(algo, n):
+@pytest.mark.parametrize("n", [128, 129, 167, 168, 169, 192, 193, 252, 253, 256, 383, 385, 420, 513, 769])
+def test_pair_tensor_forces(algo, n, precision):
     x, y, z = lattice(n, n)
-    ctx = Context(algo, "mixed", nu=1.3)
+    ctx = Context(algo, precision, nu=1.3)
     ctx.set_particles(x, y, z)
     fx, fy, fz, e, c = ctx.forces()
     again = ctx.forces()
     ctx.close()
     rx, ry, rz, rc = O.forces(x, y, z, 1.3, -1.0, nthreads=0)
     assert c == rc
-    assert rel(np.stack([fx, fy, fz]), np.stack([rx, ry, rz])) <= TOL
-    assert abs(e - O.energy(x, y, z, 1.3, -1.0)) <= TOL * O.energy_abs(x, y, z, 1.3, -1.0)
+    assert rel(np.stack([fx, fy, fz]), np.stack([rx, ry, rz])) <= TOL[precision]
+    assert abs(e - O.energy(x, y, z, 1.3, -1.0)) <= TOL[precision] * O.energy_abs(x, y, z, 1.3, -1.0)
     assert all(np.array_equal(a, b) for a, b in zip((fx, fy, fz, e), again))  # fixed order of summation
 
 
-def test_pair_tensor_batch_of_uneven_systems():
+@pytest.mark.parametrize("precision", PRECISIONS)
+def test_pair_tensor_batch_of_uneven_systems(precision):
     sizes = [1, 84, 2, 0, 300, 43, 3, 42, 85, 126, 500]
     offsets = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
     pos = np.concatenate([lattice(n, 7 + n) for n in sizes if n], 1)
-    ctx = Context("auta", "mixed")
+    ctx = Context("auta", precision)
     fx, fy, fz, e, counts = ctx.batch_forces(offsets, *pos)
     ctx.close()
     for s, n in enumerate(sizes):
@@ -60,16 +63,48 @@ def test_pair_tensor_batch_of_uneven_systems():
         x, y, z = (np.ascontiguousarray(p[sl]) for p in pos)
         rx, ry, rz, rc = O.forces(x, y, z, 1.0, -1.0, nthreads=0)
         assert counts[s] == rc
-        assert rel(f, np.stack([rx, ry, rz])) <= TOL, n
-        assert abs(e[s] - O.energy(x, y, z, 1.0, -1.0)) <= TOL * O.energy_abs(x, y, z, 1.0, -1.0), n
+        assert rel(f, np.stack([rx, ry, rz])) <= TOL[precision], n
+        assert abs(e[s] - O.energy(x, y, z, 1.0, -1.0)) <= TOL[precision] * O.energy_abs(x, y, z, 1.0, -1.0), n
 
 
+@pytest.mark.parametrize("precision", PRECISIONS)
 @pytest.mark.parametrize("scale", [0.05, 30.0])
-def test_pair_tensor_range_of_lengths(scale):
+def test_pair_tensor_range_of_lengths(scale, precision):
     """Pair tensors from 1 / 30^3 / 9^3 to 1 / 0.03^3: the same forces up to the scale's power."""
     x, y, z = lattice(300, 3, scale)
-    ctx = Context("nata", "mixed")
+    ctx = Context("nata", precision)
     ctx.set_particles(x, y, z)
     f = np.stack(ctx.forces()[:3])
     ctx.close()
-    assert rel(f, np.stack(O.forces(x, y, z, 1.0, -1.0, nthreads=0)[:3])) <= TOL
+    assert rel(f, np.stack(O.forces(x, y, z, 1.0, -1.0, nthreads=0)[:3])) <= TOL[precision]
+
+
+@pytest.mark.parametrize("algo,precision,tol", [("auta", "fp64", 1e-12), ("nata", "mixed", 1e-5)])
+def test_fits_that_do_not_wait(algo, precision, tol):
+    """Forward and backward of several sizes, issued without waiting on two streams: each call's work lists,
+    tables and workspaces are those of its own size while earlier ones still run."""
+    import torch
+
+    from threebodymdalgorithms_b200.autograd import AxilrodTeller
+
+    sizes = [100, 489, 100, 300, 127, 700]
+    at = AxilrodTeller(algo, precision)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    got, want = [], []
+    for q, n in enumerate(sizes):
+        x = torch.tensor(lattice(n, n).T.copy(), device="cuda", requires_grad=True)
+        nu = torch.tensor(1.1, dtype=torch.float64, device="cuda", requires_grad=True)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(streams[q % 2]):
+            f, e = at(x, nu)
+            got.append((f, e, *torch.autograd.grad([f.square().sum() + e], [x, nu])))
+    torch.cuda.synchronize()
+    for n in sizes:
+        x = torch.tensor(lattice(n, n).T.copy(), device="cuda", requires_grad=True)
+        nu = torch.tensor(1.1, dtype=torch.float64, device="cuda", requires_grad=True)
+        f, e = AxilrodTeller(algo, "fp64")(x, nu)
+        want.append((f, e, *torch.autograd.grad([f.square().sum() + e], [x, nu])))
+        torch.cuda.synchronize()
+    for n, g, w in zip(sizes, got, want):
+        for a, b in zip(g, w):
+            assert float((a - b).detach().norm()) <= tol * max(float(b.detach().norm()), 1e-300), n

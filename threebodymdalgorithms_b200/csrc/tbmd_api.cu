@@ -99,15 +99,23 @@ struct tbmd_ctx {
 
     // no-cutoff sweeps
     int R_auta = 4, R_nata = 2, R_fp64 = 2;
-    DevBuf sweep_sys;  // single system: sys_items[2], sys_off[2], sys_prefix[1], sys_nblocks[1]
-    DevBuf prefix;
-    int prefix_JB = 0, prefix_alg = -1;
-    int64_t prefix_kseg = 0;  // k range per AUTA item of the current work list (0: the whole sweep)
-    int64_t prefix_n = -1;
-    int nblocks = 0;
-    int64_t total_items = 0;
+    // single-system work lists of the sweeps: [0] forces, [1] adjoint, which a fit evaluates in turn
+    struct SweepList {
+        DevBuf sys;  // sys_items[2], sys_off[2], sys_prefix[1], sys_nblocks[1]
+        DevBuf prefix;
+        int JB = 0, alg = -1;
+        int64_t kseg = 0;  // k range per AUTA item (0: the whole sweep)
+        int64_t n = -1;
+        int nblocks = 0;
+        int64_t total_items = 0;
+    } sweep[2];
     DevBuf partial;
     int sweep_grid = 0;
+    // No-cutoff evaluations return without waiting, on the caller's stream: the event after the last one,
+    // and its stream.  The next one on another stream waits for it on the device (they share the work lists'
+    // counter and the workspaces), and tables are rewritten after it on the host.
+    cudaEvent_t ws_event = nullptr;
+    cudaStream_t ws_stream = nullptr;
     // no-cutoff forces of the mixed form as a product of pair tensors: the systems the plan was made
     // for (their particle offsets), its tables on the device, panel, tile results
     std::vector<int64_t> pt_off;
@@ -258,6 +266,28 @@ static void phase_resolve(tbmd_ctx *ctx)
     ctx->cur_phase = -1;
 }
 
+static bool capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &c) == cudaSuccess && c != cudaStreamCaptureStatusNone;
+}
+static cudaError_t ws_acquire(tbmd_ctx *ctx, cudaStream_t st)
+{
+    if (!ctx->ws_event || ctx->ws_stream == st || capturing(st)) return cudaSuccess;
+    return cudaStreamWaitEvent(st, ctx->ws_event, 0);
+}
+static cudaError_t ws_release(tbmd_ctx *ctx, cudaStream_t st)
+{
+    if (capturing(st)) return cudaSuccess;
+    if (!ctx->ws_event) {
+        const cudaError_t e = cudaEventCreateWithFlags(&ctx->ws_event, cudaEventDisableTiming);
+        if (e != cudaSuccess) return e;
+    }
+    ctx->ws_stream = st;
+    return cudaEventRecord(ctx->ws_event, st);
+}
+static cudaError_t ws_wait_host(tbmd_ctx *ctx) { return ctx->ws_event ? cudaEventSynchronize(ctx->ws_event) : cudaSuccess; }
+
 // Work list of the no-cutoff sweep for (algorithm, n, R).  A small AUTA system has fewer (block, i)
 // items than the GPU has resident warps, and their k sweeps differ in length by the whole system, so
 // the longest one sets the kernel time: its items are then split by k range (kseg particles each),
@@ -278,28 +308,30 @@ static tbmd_status ensure_sweep(tbmd_ctx *ctx, int alg, int64_t n, int R, bool d
             }
         }
     }
-    if (ctx->prefix_n != n || ctx->prefix_JB != JB || ctx->prefix_alg != alg || ctx->prefix_kseg != kseg) {
+    tbmd_ctx::SweepList &l = ctx->sweep[dual ? 1 : 0];
+    if (l.n != n || l.JB != JB || l.alg != alg || l.kseg != kseg) {
+        CK(ws_wait_host(ctx));  // a sweep on a caller's stream may still read the old list
         std::vector<int64_t> pre((size_t)(n / JB + 3), 0);
         int64_t total = sweep_items(alg, n, JB, pre.data(), kseg);
         int64_t nb = n >= 3 ? (n - 2 + JB) / JB : 0;
         if (total >= (int64_t)UINT32_MAX - 65536)
             return fail(ctx, TBMD_INVALID_ARG, "n = %lld gives too many sweep work items", (long long)n);
-        CK(ctx->prefix.ensure(sizeof(int64_t) * (nb + 1)));
-        CK(cudaMemcpyAsync(ctx->prefix.p, pre.data(), sizeof(int64_t) * (nb + 1), cudaMemcpyHostToDevice, ctx->stream));
+        CK(l.prefix.ensure(sizeof(int64_t) * (nb + 1)));
+        CK(cudaMemcpyAsync(l.prefix.p, pre.data(), sizeof(int64_t) * (nb + 1), cudaMemcpyHostToDevice, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
-        ctx->prefix_n = n;
-        ctx->prefix_JB = JB;
-        ctx->prefix_alg = alg;
-        ctx->prefix_kseg = kseg;
-        ctx->nblocks = (int)nb;
-        ctx->total_items = total;
+        l.n = n;
+        l.JB = JB;
+        l.alg = alg;
+        l.kseg = kseg;
+        l.nblocks = (int)nb;
+        l.total_items = total;
         // one system: sys_items = {0, total}, sys_off = {0, n}, sys_prefix = {0}, sys_nblocks = {nb}
         struct {
             int64_t items[2], off[2], pre[1];
             int32_t nbl[2];
         } tab = {{0, total}, {0, n}, {0}, {(int32_t)nb, 0}};
-        CK(ctx->sweep_sys.ensure(sizeof tab));
-        CK(cudaMemcpyAsync(ctx->sweep_sys.p, &tab, sizeof tab, cudaMemcpyHostToDevice, ctx->stream));
+        CK(l.sys.ensure(sizeof tab));
+        CK(cudaMemcpyAsync(l.sys.p, &tab, sizeof tab, cudaMemcpyHostToDevice, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         if (alg == TBMD_NATA) CK(ctx->partial.ensure(sizeof(double) * 3 * (size_t)n * (size_t)(nb > 0 ? nb : 1)));
     }
@@ -307,12 +339,13 @@ static tbmd_status ensure_sweep(tbmd_ctx *ctx, int alg, int64_t n, int R, bool d
 }
 
 // Work list of the single system of the context (tables filled by ensure_sweep).
-static SweepWork single_sweep(tbmd_ctx *ctx)
+static SweepWork single_sweep(tbmd_ctx *ctx, bool dual)
 {
-    const char *t = ctx->sweep_sys.as<char>();
-    return SweepWork{ctx->prefix.as<int64_t>(), ctx->nblocks, ctx->total_items, sweep_counter(ctx), 1,
+    const tbmd_ctx::SweepList &l = ctx->sweep[dual ? 1 : 0];
+    const char *t = l.sys.as<char>();
+    return SweepWork{l.prefix.as<int64_t>(), l.nblocks, l.total_items, sweep_counter(ctx), 1,
                      (const int64_t *)t, (const int64_t *)(t + 16), (const int64_t *)(t + 32),
-                     (const int32_t *)(t + 40), ctx->prefix_kseg};
+                     (const int32_t *)(t + 40), l.kseg};
 }
 
 // Whether the no-cutoff forces of a system (or the largest of a batch) go through the pair-tensor product
@@ -322,7 +355,7 @@ static SweepWork single_sweep(tbmd_ctx *ctx)
 constexpr int64_t kPairsMin = 128, kPairsMax = 65536;
 static bool use_pairs(const tbmd_ctx *ctx, int64_t n, bool dual)
 {
-    return mixed(ctx) && !dual && n >= kPairsMin && n <= kPairsMax;
+    return !dual && n >= kPairsMin && n <= kPairsMax;
 }
 
 // Plan, tables and workspaces of the pair-tensor product for systems at offsets off[0 .. nsys].  The
@@ -331,19 +364,18 @@ static tbmd_status ensure_pairs(tbmd_ctx *ctx, const int64_t *off, int nsys)
 {
     if (ctx->pt_off.size() == (size_t)nsys + 1 && std::memcmp(ctx->pt_off.data(), off, sizeof(int64_t) * (nsys + 1)) == 0)
         return TBMD_OK;
-    // the tables are rewritten: a launch on a caller's stream may still read the old ones
-    CK(cudaDeviceSynchronize());
+    CK(ws_wait_host(ctx));  // a launch on a caller's stream may still read the old tables
     ctx->pt_off.clear();
     invalidate_graph(ctx);
     if (!ctx->sms) CK(cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device));
     CK(pt_init());
-    pt_plan(off, nsys, ctx->sms, (size_t)1 << 30, ctx->pt);
+    pt_plan(off, nsys, ctx->sms, (size_t)1 << 30, !mixed(ctx), ctx->pt);
     const PtPlan &p = ctx->pt;
     const size_t b_seg = sizeof(PtSeg) * p.segs.size(), b_sys = sizeof(PtSys) * p.sys.size(),
                  b_til = sizeof(unsigned int) * p.tiles.size();
     CK(ctx->pt_tab.ensure(b_seg + b_sys + b_til));
     CK(ctx->pt_panel.ensure(p.mem));
-    CK(ctx->pt_slots.ensure(p.slots * pt_slot_bytes()));
+    CK(ctx->pt_slots.ensure(p.slots * p.slot_bytes));
     char *t = ctx->pt_tab.as<char>();
     CK(cudaMemcpyAsync(t, p.segs.data(), b_seg, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(t + b_seg, p.sys.data(), b_sys, cudaMemcpyHostToDevice, ctx->stream));
@@ -562,14 +594,14 @@ static tbmd_status enqueue_forces(tbmd_ctx *ctx, int64_t n, Pos pos, Out out, bo
         }
         return TBMD_OK;
     }
-    SweepWork w = single_sweep(ctx);
+    SweepWork w = single_sweep(ctx, dual);
     CK(cudaMemsetAsync(w.counter, 0, sizeof(unsigned int), st));
     if (ctx->cfg.algorithm == TBMD_NATA && !dual) {
-        CK(launch_nata(mx, false, ctx->prefix_JB / 32, energy != nullptr, n, pos, out, energy, nu, w,
+        CK(launch_nata(mx, false, ctx->sweep[0].JB / 32, energy != nullptr, n, pos, out, energy, nu, w,
                        ctx->partial.as<double>(), ctx->sweep_grid, st));
         *nl += 1;
         phase_mark(ctx, st, PH_UPDATE, *nl);
-        CK(launch_nata_reduce(false, n, ctx->nblocks, ctx->partial.as<double>(), out, st));
+        CK(launch_nata_reduce(false, n, ctx->sweep[0].nblocks, ctx->partial.as<double>(), out, st));
         *nl += 1;
     } else {
         CK(cudaMemsetAsync(out.fx, 0, sizeof(double) * n, st));
@@ -580,7 +612,7 @@ static tbmd_status enqueue_forces(tbmd_ctx *ctx, int64_t n, Pos pos, Out out, bo
             CK(cudaMemsetAsync(out.hy, 0, sizeof(double) * n, st));
             CK(cudaMemsetAsync(out.hz, 0, sizeof(double) * n, st));
         }
-        CK(launch_auta(mx, dual, ctx->prefix_JB / 32, energy != nullptr, n, pos, out, energy, nu, w, ctx->sweep_grid,
+        CK(launch_auta(mx, dual, ctx->sweep[dual ? 1 : 0].JB / 32, energy != nullptr, n, pos, out, energy, nu, w, ctx->sweep_grid,
                        st));
         *nl += 1;
         phase_mark(ctx, st, PH_UPDATE, *nl);
@@ -663,7 +695,7 @@ static void fill_graph_key(tbmd_ctx *ctx, GraphKey &k)
     } else if (use_pairs(ctx, ctx->n, false)) {
         k.pairs = ctx->pt_dev;
     } else {
-        k.sweep = single_sweep(ctx);
+        k.sweep = single_sweep(ctx, false);
         k.partial = ctx->partial.p;
         k.sweep_grid = ctx->sweep_grid;
     }
@@ -807,9 +839,9 @@ void tbmd_destroy(tbmd_ctx *ctx)
     invalidate_graph(ctx);
     for (auto &m : ctx->marks) cudaEventDestroy(m.second);
     for (cudaEvent_t e : ctx->event_pool) cudaEventDestroy(e);
-    for (DevBuf *b : {&ctx->state, &ctx->snapshot, &ctx->scalars, &ctx->step_counts, &ctx->prefix, &ctx->partial,
+    for (DevBuf *b : {&ctx->state, &ctx->snapshot, &ctx->scalars, &ctx->step_counts, &ctx->partial,
                       &ctx->cell_n, &ctx->cell_c, &ctx->nbr_buf, &ctx->dirs, &ctx->hvp, &ctx->gset_single,
-                      &ctx->sweep_sys, &ctx->bpos, &ctx->bout, &ctx->bsys, &ctx->bprefix, &ctx->ncell_tab,
+                      &ctx->sweep[0].sys, &ctx->sweep[0].prefix, &ctx->sweep[1].sys, &ctx->sweep[1].prefix, &ctx->bpos, &ctx->bout, &ctx->bsys, &ctx->bprefix, &ctx->ncell_tab,
                       &ctx->staging, &ctx->long_buf, &ctx->gen_buf, &ctx->bext, &ctx->pt_tab, &ctx->pt_panel,
                       &ctx->pt_slots})
         b->release();
@@ -820,6 +852,7 @@ void tbmd_destroy(tbmd_ctx *ctx)
     }
     if (ctx->hstep) cudaFreeHost(ctx->hstep);
     if (ctx->pos_event) cudaEventDestroy(ctx->pos_event);
+    if (ctx->ws_event) cudaEventDestroy(ctx->ws_event);
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -1136,6 +1169,7 @@ static tbmd_status run_steps(tbmd_ctx *ctx, int32_t iterations, uint64_t *counts
     for (int attempt = 0; attempt < 4; ++attempt) {
         st = prepare(ctx, n, false, false);
         if (st != TBMD_OK) return st;
+        CK(ws_acquire(ctx, ctx->stream));
         // a graph of other arguments (another domain, moved buffers) is not replayed
         GraphKey key;
         fill_graph_key(ctx, key);
@@ -1251,6 +1285,8 @@ static tbmd_status evaluate(tbmd_ctx *ctx, int64_t n, Pos pos, Out out, bool dua
     for (int attempt = 0; attempt < 4; ++attempt) {
         tbmd_status s = prepare(ctx, n, dual, energy != nullptr);
         if (s != TBMD_OK) return s;
+        const bool cut = is_p3bca_cut(ctx);
+        if (!cut) CK(ws_acquire(ctx, st));
         CK(reset_cap_flags(ctx, st));
         if (energy) CK(cudaMemsetAsync(energy, 0, sizeof(double), st));
         if (count) CK(cudaMemsetAsync(count, 0, sizeof(unsigned long long), st));
@@ -1263,7 +1299,10 @@ static tbmd_status evaluate(tbmd_ctx *ctx, int64_t n, Pos pos, Out out, bool dua
             CK(cudaStreamSynchronize(st));
             phase_resolve(ctx);
         }
-        if (!is_p3bca_cut(ctx)) return TBMD_OK;
+        if (!cut) {
+            CK(ws_release(ctx, st));
+            return TBMD_OK;
+        }
         CapSeen seen{};
         CK(read_cap_flags(ctx, st, &seen));
         CK(cudaStreamSynchronize(st));
@@ -1618,6 +1657,7 @@ static tbmd_status batch_eval(tbmd_ctx *ctx, int32_t nsys, const int64_t *offset
     st = ensure_scalars(ctx);
     if (st != TBMD_OK) return st;
     CK(cudaStreamSynchronize(ctx->stream));
+    CK(ws_acquire(ctx, ctx->stream));
     invalidate_graph(ctx);
     const bool mx = mixed(ctx);
     const double nu = ctx->cfg.nu == 0.0 ? 1.0 : ctx->cfg.nu;  // nu = 0: evaluate the nu = 1 parts
@@ -1751,7 +1791,7 @@ static tbmd_status batch_eval(tbmd_ctx *ctx, int32_t nsys, const int64_t *offset
         CK(cudaMemcpyAsync(c.data(), CNT, sizeof(unsigned long long) * nsys, cudaMemcpyDeviceToHost, sm));
         CK(cudaStreamSynchronize(sm));
         for (int s = 0; s < nsys; ++s) res.counts[s] = c[s];
-    } else if (!dual && mx && N >= kPairsMin && nmax <= kPairsMax) {
+    } else if (!dual && N >= kPairsMin && nmax <= kPairsMax) {
         CK(reset_cap_flags(ctx, sm));
         st = ensure_pairs(ctx, offsets, nsys);
         if (st != TBMD_OK) return st;

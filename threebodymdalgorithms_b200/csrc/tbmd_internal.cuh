@@ -332,7 +332,7 @@ cudaError_t launch_nata(bool mixed, bool dual, int R, bool energy, int64_t n, Po
                         double nu, SweepWork work, double *partial, int grid, cudaStream_t st);
 cudaError_t launch_nata_reduce(bool dual, int64_t n, int nblocks, const double *partial, Out out, cudaStream_t st);
 
-// No-cutoff forces of the mixed form as a product of pair tensors (tbmd_pairs.cu).  A segment is one
+// No-cutoff forces as a product of pair tensors (tbmd_pairs.cu).  A segment is one
 // system's range of k; an item is one tile of one segment.  Offsets are within the group (one launch).
 struct PtSeg {
     int64_t mem;    // bytes into the panel
@@ -361,6 +361,8 @@ struct PtPlan {
     std::vector<unsigned int> tiles;
     std::vector<PtGroup> groups;
     size_t mem = 0, slots = 0;  // largest group's panel bytes and tile results
+    size_t slot_bytes = 0;      // of one tile result
+    bool fp64 = false;          // the FP64 form (panel steps of 8 k, row blocks of 32 particles)
 };
 struct PtDev {
     const PtSeg *segs;
@@ -370,8 +372,7 @@ struct PtDev {
     double *slots;
     unsigned int *err;  // set by a launch that gave up waiting
 };
-void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, PtPlan &plan);
-size_t pt_slot_bytes();
+void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, bool fp64, PtPlan &plan);
 cudaError_t pt_init();
 // forces overwritten; energy (one accumulator per system, may be NULL) added to
 cudaError_t launch_pairs(Pos pos, Out out, const PtPlan &plan, const PtDev &d, double *energy,

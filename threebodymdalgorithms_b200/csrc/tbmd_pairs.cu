@@ -49,7 +49,9 @@ constexpr int PT_STAGES = 3;
 constexpr int PT_GEO = 2 * (PT_PART / 2) * PT_PART;      // pair geometry of a block's tile: [pair of j][i]
 // 8 warps accumulate and contract, 1 loads, 1 issues the products, 2 fetch positions
 constexpr int PT_WARPS = 12;
-constexpr int PT_SLOT = 3 * PT_PART * 3 + 2;  // doubles of a tile's results: f_i, f_j (two blocks), energy, pad
+// doubles of a tile's results for row blocks of `part` particles: f_i, f_j (two blocks), energy, pad
+__host__ __device__ constexpr int pt_slot(int part) { return 9 * part + 2; }
+constexpr int PT_SLOT = pt_slot(PT_PART);
 
 struct PtShared {
     unsigned char stage[PT_STAGES][PT_STAGE_BYTES];
@@ -106,7 +108,8 @@ __device__ __forceinline__ bool bar_try(unsigned long long *b, unsigned int pari
 }
 // Every wait ends: after four billion cycles (two seconds or more) it marks the block dead and the launch failed (*err); from then on
 // waits return at once, no copy or product is issued, and the loops run out.
-__device__ __forceinline__ bool bar_wait(unsigned long long *b, unsigned int parity, PtShared &S, unsigned int *err)
+template <class Shared>
+__device__ __forceinline__ bool bar_wait(unsigned long long *b, unsigned int parity, Shared &S, unsigned int *err)
 {
     if (bar_try(b, parity)) return true;
     const long long t0 = clock64();
@@ -658,10 +661,229 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem));
 }
 
+// ---------------------------------------------------------------------------------------------
+// FP64 form.  Only the symmetric part of G_ij acts on the symmetric dT/dr, and sym(T_ik T_kj) is a symmetric
+// bilinear form of the two tensors: with A = T_ik, B = T_jk, traceless, its entries are sums of
+//   A_xx B_xx, A_yy B_yy, A_zz B_zz, A_xy B_xy, A_xz B_xz, A_yz B_yz                         (d_x d_y d_z, s_xy ..)
+// and, since ab' + a'b = (a + b)(a' + b') - aa' - bb', of six products of sums, (A_xy + A_zz)(B_xy + B_zz),
+// (A_xz + A_yz)(..), (A_xz + A_yy)(..), (A_xy + A_yz)(..), (A_yz + A_xx)(..), (A_xy + A_xz)(..):
+//   G_xx = d_x + s_xy + s_xz,  2 G_xy = -(p_0 - s_xy - d_z) + (p_1 - s_xz - s_yz),  and cyclic.
+// So twelve features F of every pair tensor give G by twelve products F F^T: 12 FMA per pair and k, 6 n^3 in
+// all, where the AUTA sweep takes about 10 n^3 FP64 operations and NATA's three times that.
+//
+//   k_p64_panel  the features of a range of k, in the order the matrix instruction's operands are read
+//   k_p64_gemm   tiles of 32 x 64 particles (a warp: 16 x 16 pairs x 12 sums) by the FP64 matrix instruction,
+//                contracted with dT/dr
+//
+// Bound: the FP64 rate, which the matrix instruction reaches with few warps (36.9 TFLOP/s with 8 on an SM) and
+// few shared-memory reads (half the wavefront slots): 192 registers of sums leave one block of 8 warps an SM.
+// Plain FMA on 2 x 4 pairs a thread, with three 16-byte reads for 8 FMA, reached 0.41 of the rate (n = 8192:
+// 477 ms).
+constexpr int P64_PART = 32, P64_K = 8, P64_F = 12, P64_STAGES = 3;
+constexpr int P64_BLOCK = P64_K * P64_F * P64_PART;  // doubles of one row block and 8 k: 24 KB
+constexpr int P64_SLOT = pt_slot(P64_PART);
+
+struct P64Shared {
+    // row block i, two blocks j: [four k][pair of features][8 particles][particle, k][feature], so that the 32
+    // lanes' operands, for two features, are 512 consecutive bytes
+    double stage[P64_STAGES][3][P64_BLOCK];
+    double fi[4][P64_PART][3], fj[2][2 * P64_PART][3], e[8];
+    unsigned long long full[P64_STAGES];
+    int dead;
+};
+
+__global__ void __launch_bounds__(P64_K * P64_PART) k_p64_panel(Pos pos, const PtSeg *__restrict__ seg, int nseg,
+                                                              double *__restrict__ panel)
+{
+    const PtSeg s = seg[pt_find(seg, nseg, (int64_t)blockIdx.x, [](const PtSeg &q) { return (int64_t)q.gen0; })];
+    const int task = (int)blockIdx.x - s.gen0, rb = task / s.nslab, kc = task - rb * s.nslab;
+    const int il = threadIdx.x & 31, kl = threadIdx.x >> 5;
+    const int i = rb * P64_PART + il, k = s.k0 + kc * P64_K + kl;
+    double xx = 0.0, xy = 0.0, xz = 0.0, yy = 0.0, yz = 0.0, zz = 0.0;
+    if (i < s.n && k < s.n && i != k) {
+        const double x = pos.x[s.part0 + k] - pos.x[s.part0 + i], y = pos.y[s.part0 + k] - pos.y[s.part0 + i],
+                     z = pos.z[s.part0 + k] - pos.z[s.part0 + i];
+        const double ri = rsqrt(fma(x, x, fma(y, y, z * z)));
+        const double ri2 = ri * ri, i3 = ri * ri2, s5 = 3.0 * i3 * ri2;
+        xx = fma(s5 * x, x, -i3);
+        xy = s5 * x * y;
+        xz = s5 * x * z;
+        yy = fma(s5 * y, y, -i3);
+        yz = s5 * y * z;
+        zz = fma(s5 * z, z, -i3);
+    }
+    double *dst = panel + s.mem / 8 + ((int64_t)rb * s.nslab + kc) * P64_BLOCK +
+                  ((kl >> 2) * (P64_F / 2) * 4 + (il >> 3)) * 64 + ((il & 7) * 4 + (kl & 3)) * 2;
+    const double f[P64_F] = {xx, yy, zz, xy, xz, yz, xy + zz, xz + yz, xz + yy, xy + yz, yz + xx, xy + xz};
+#pragma unroll
+    for (int m = 0; m < P64_F / 2; ++m) *(double2 *)(dst + m * 256) = make_double2(f[2 * m], f[2 * m + 1]);
+}
+
+// D += A B, A 8 x 4 (lane: row lane / 4, column lane % 4), B 4 x 8 (lane: row lane % 4, column lane / 4), D 8 x 8
+// (lane: row lane / 4, columns 2 (lane % 4) and + 1)
+__device__ __forceinline__ void mma_f64(double &d0, double &d1, double a, double b)
+{
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(d0), "+d"(d1)
+        : "d"(a), "d"(b));
+}
+
+template <bool ENERGY>
+__global__ void __launch_bounds__(256, 1)
+    k_p64_gemm(Pos pos, const PtSeg *__restrict__ seg, int nseg, int64_t items, const unsigned int *__restrict__ tiles,
+               const double *__restrict__ panel, double *__restrict__ slots, double nu, unsigned int *err)
+{
+    extern __shared__ __align__(1024) unsigned char smraw[];
+    P64Shared &S = *(P64Shared *)smraw;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int iw = warp & 1, jw = warp >> 1, li = lane >> 2, lj = lane & 3;
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < P64_STAGES; ++k) bar_init(&S.full[k], 1);
+        S.dead = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    // thread 0 loads, two steps of 8 k ahead of the products and across items
+    int64_t lw = blockIdx.x;  // item and step that is loaded next
+    int lk = 0;
+    unsigned int ln = 0;
+    PtItem lit{};
+    auto load = [&]() {
+        if (lw >= items || *(volatile int *)&S.dead) return;
+        if (lk == 0) lit = pt_item(seg, nseg, tiles, lw);
+        const int st = ln % P64_STAGES;
+        const double *src = panel + lit.s.mem / 8 + (int64_t)lk * P64_BLOCK;
+        const int64_t row = (int64_t)lit.s.nslab * P64_BLOCK;
+        bar_expect(&S.full[st], 3 * P64_BLOCK * 8);
+        bulk_load(S.stage[st][0], src + lit.a * row, P64_BLOCK * 8, &S.full[st]);
+        bulk_load(S.stage[st][1], src + 2 * lit.b * row, P64_BLOCK * 8, &S.full[st]);
+        bulk_load(S.stage[st][2], src + (2 * lit.b + 1) * row, P64_BLOCK * 8, &S.full[st]);
+        ++ln;
+        if (++lk == lit.s.nslab) {
+            lk = 0;
+            lw += gridDim.x;
+        }
+    };
+    if (threadIdx.x == 0)
+        for (int k = 0; k < P64_STAGES; ++k) load();
+    unsigned int n = 0;
+    for (int64_t w = blockIdx.x; w < items; w += gridDim.x) {
+        const PtItem it = pt_item(seg, nseg, tiles, w);
+        double acc[P64_F][2][4];
+#pragma unroll
+        for (int m = 0; m < P64_F; ++m)
+#pragma unroll
+            for (int q = 0; q < 8; ++q) acc[m][q >> 2][q & 3] = 0.0;
+        for (int kc = 0; kc < it.s.nslab; ++kc, ++n) {
+            const int st = n % P64_STAGES;
+            bar_wait(&S.full[st], (n / P64_STAGES) & 1, S, err);
+            const double2 *I = (const double2 *)S.stage[st][0] + iw * 64 + lane,
+                          *J = (const double2 *)S.stage[st][1 + (jw >> 1)] + (jw & 1) * 64 + lane;
+#pragma unroll 1
+            for (int k = 0; k < P64_K / 4; ++k) {
+#pragma unroll
+                for (int m = 0; m < P64_F / 2; ++m) {
+                    const int o = (k * (P64_F / 2) + m) * 128;
+                    const double2 a[2] = {I[o], I[o + 32]}, b[2] = {J[o], J[o + 32]};
+#pragma unroll
+                    for (int u = 0; u < 2; ++u)
+#pragma unroll
+                        for (int v = 0; v < 2; ++v) {
+                            mma_f64(acc[2 * m][u][2 * v], acc[2 * m][u][2 * v + 1], a[u].x, b[v].x);
+                            mma_f64(acc[2 * m + 1][u][2 * v], acc[2 * m + 1][u][2 * v + 1], a[u].y, b[v].y);
+                        }
+                }
+            }
+            __syncthreads();  // the stage has been read
+            if (threadIdx.x == 0) load();
+        }
+        // contraction of G with dT/dr: with n = r / |r|, q = n.G n
+        //   f_i += nu / r^4 (2 G n + (tr G - 5 q) n),  E -= nu / (9 r^3) (3 q - tr G)
+        const int64_t P = it.s.part0;
+        const int ia = it.a * P64_PART + iw * 16 + li, jb = 2 * it.b * P64_PART + jw * 16 + lj * 2;
+        double fi[2][3] = {}, fj[4][3] = {}, en = 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int u = q >> 2, v = q & 3, i = ia + u * 8, j = jb + (v >> 1) * 8 + (v & 1);
+            if (i < j && j < it.s.n) {
+                const double x = pos.x[P + j] - pos.x[P + i], y = pos.y[P + j] - pos.y[P + i],
+                             z = pos.z[P + j] - pos.z[P + i];
+                const double ri = rsqrt(fma(x, x, fma(y, y, z * z))), ri2 = ri * ri;
+                const double nx = x * ri, ny = y * ri, nz = z * ri;
+                const double dx = acc[0][u][v], dy = acc[1][u][v], dz = acc[2][u][v], sxy = acc[3][u][v], sxz = acc[4][u][v],
+                             syz = acc[5][u][v];
+                const double gxx = dx + sxy + sxz, gyy = dy + sxy + syz, gzz = dz + sxz + syz;
+                // twice the off-diagonal entries
+                const double gxy = (acc[7][u][v] - sxz - syz) - (acc[6][u][v] - sxy - dz);
+                const double gxz = (acc[9][u][v] - sxy - syz) - (acc[8][u][v] - sxz - dy);
+                const double gyz = (acc[11][u][v] - sxy - sxz) - (acc[10][u][v] - syz - dx);
+                const double hx = 2.0 * gxx * nx + gxy * ny + gxz * nz, hy = gxy * nx + 2.0 * gyy * ny + gyz * nz,
+                             hz = gxz * nx + gyz * ny + 2.0 * gzz * nz;
+                const double tr = gxx + gyy + gzz, qq = 0.5 * (hx * nx + hy * ny + hz * nz);
+                const double c = nu * ri2 * ri2, d = tr - 5.0 * qq;
+                const double vx = c * (hx + d * nx), vy = c * (hy + d * ny), vz = c * (hz + d * nz);
+                fi[u][0] += vx;
+                fi[u][1] += vy;
+                fi[u][2] += vz;
+                fj[v][0] -= vx;
+                fj[v][1] -= vy;
+                fj[v][2] -= vz;
+                if (ENERGY) en -= nu * ri * ri2 * (3.0 * qq - tr) / 9.0;
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                double v = fi[u][c];
+                for (int o = 1; o < 4; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lj == 0) S.fi[jw][iw * 16 + li + u * 8][c] = v;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                double v = fj[u][c];
+                for (int o = 4; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (li == 0) S.fj[iw][jw * 16 + lj * 2 + (u >> 1) * 8 + (u & 1)][c] = v;
+            }
+        }
+        if (ENERGY) {
+            en = warp_sum(en);
+            if (lane == 0) S.e[warp] = en;
+        }
+        __syncthreads();
+        double *slot = slots + (it.s.slot0 + (int64_t)it.b * (it.b + 1) + it.a) * P64_SLOT;
+        for (int t = threadIdx.x; t < 9 * P64_PART; t += 256) {
+            double v;
+            if (t < 3 * P64_PART) {
+                v = S.fi[0][t / 3][t % 3];
+                for (int q = 1; q < 4; ++q) v += S.fi[q][t / 3][t % 3];
+            } else {
+                const int c = t - 3 * P64_PART;
+                v = S.fj[0][c / 3][c % 3] + S.fj[1][c / 3][c % 3];
+            }
+            slot[t] = v;
+        }
+        if (ENERGY && threadIdx.x == 0) {
+            double v = S.e[0];
+            for (int q = 1; q < 8; ++q) v += S.e[q];
+            slot[9 * P64_PART] = v;
+        }
+        __syncthreads();
+    }
+    // a block that gave up leaves no copy in flight behind it
+    if (threadIdx.x == 0 && *(volatile int *)&S.dead)
+        for (unsigned int k = ln > P64_STAGES ? ln - P64_STAGES : 0; k < ln; ++k) {
+            const long long t0 = clock64();
+            while (!bar_try(&S.full[k % P64_STAGES], (k / P64_STAGES) & 1) && clock64() - t0 < 200000000ll) {
+            }
+        }
+}
+
 // Forces from the tiles' results: particle i of row block a sums the tiles (a, b) of its row and the tiles
 // (a', a / 2) of its column, over the system's segments.  A warp per particle; the lanes' sums and their
 // tree have a fixed order.  A system whose panels did not fit one launch is added up over launches.  A
 // launch that gave up gives NaN.
+template <int PART>
 __global__ void k_pt_reduce(int64_t p0, int64_t n, const PtSys *__restrict__ sys, int nsys, const double *__restrict__ slots, Out out,
                             const unsigned int *__restrict__ err)
 {
@@ -669,14 +891,14 @@ __global__ void k_pt_reduce(int64_t p0, int64_t n, const PtSys *__restrict__ sys
     const int lane = threadIdx.x & 31;
     if (p >= p0 + n) return;
     const PtSys s = sys[pt_system(sys, nsys, p)];
-    const int i = (int)(p - s.part0), a = i / PT_PART, il = i - a * PT_PART;
+    const int i = (int)(p - s.part0), a = i / PART, il = i - a * PART;
     const int b0 = a >> 1, rows = s.nb2 - b0, cols = 2 * b0 + 2, per = s.nb2 * (s.nb2 + 1);
     double f[3] = {0.0, 0.0, 0.0};
     for (int q = lane; q < s.nseg * (rows + cols); q += 32) {
         const int sg = q / (rows + cols), r = q - sg * (rows + cols);
         const int b = r < rows ? b0 + r : b0, ta = r < rows ? a : r - rows;
-        const double *src = slots + (s.slot0 + (int64_t)sg * per + (int64_t)b * (b + 1) + ta) * PT_SLOT +
-                            (r < rows ? 3 * il : 126 * (1 + (a & 1)) + 3 * il);
+        const double *src = slots + (s.slot0 + (int64_t)sg * per + (int64_t)b * (b + 1) + ta) * pt_slot(PART) +
+                            (r < rows ? 3 * il : 3 * PART * (1 + (a & 1)) + 3 * il);
         f[0] += src[0];
         f[1] += src[1];
         f[2] += src[2];
@@ -693,6 +915,7 @@ __global__ void k_pt_reduce(int64_t p0, int64_t n, const PtSys *__restrict__ sys
 
 // Energy of each system: its tiles' energies, a block per system, in a fixed order.  Adds to energy[s]
 // (the caller zeroes it).
+template <int PART>
 __global__ void __launch_bounds__(512) k_pt_energy(const PtSys *__restrict__ sys, const double *__restrict__ slots,
                                                    double *energy)
 {
@@ -700,7 +923,7 @@ __global__ void __launch_bounds__(512) k_pt_energy(const PtSys *__restrict__ sys
     const PtSys s = sys[blockIdx.x];
     const int64_t total = (int64_t)s.nseg * s.nb2 * (s.nb2 + 1);
     double e = 0.0;
-    for (int64_t q = threadIdx.x; q < total; q += 512) e += slots[(s.slot0 + q) * PT_SLOT + 378];
+    for (int64_t q = threadIdx.x; q < total; q += 512) e += slots[(s.slot0 + q) * pt_slot(PART) + 9 * PART];
     e = warp_sum(e);
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = e;
     __syncthreads();
@@ -713,34 +936,43 @@ __global__ void __launch_bounds__(512) k_pt_energy(const PtSys *__restrict__ sys
 // ---------------------------------------------------------------------------------------------
 // Work lists (host)
 
-// Tile order of nb2 blocks of 84 particles: strips of 8 column blocks, walked row by row, so that the tiles
-// in flight (one per two SMs) share row and column blocks in L2 (17 blocks, 20 MB at 256 k).
-static void pt_tiles(int nb2, std::vector<unsigned int> &out)
+// Tile order of nb2 column blocks: strips of 8 of them, walked row by row, so that the tiles in flight share
+// row and column blocks in L2 (mixed form, one tile per two SMs, rows as wide as columns: 17 blocks, 40 MB
+// at 512 k; FP64 form, one per SM, rows half as wide: 53 MB).
+static void pt_tiles(int nb2, bool fp64, std::vector<unsigned int> &out)
 {
+    const int per = fp64 ? 2 : 1;  // rows per column block
     for (int b0 = 0; b0 < nb2; b0 += 8) {
         const int b1 = std::min(nb2, b0 + 8);
-        for (int a = 0; a < b1; ++a)
-            for (int b = std::max(b0, a); b < b1; ++b) out.push_back((unsigned int)a << 16 | (unsigned int)b);
+        for (int a = 0; a < per * b1; ++a)
+            for (int b = std::max(b0, a / per); b < b1; ++b) out.push_back((unsigned int)a << 16 | (unsigned int)b);
     }
 }
 
-// Particles k of one item: the range length with the least estimated time of all items, at 1,536 cycles a
-// slab (what its product takes) and 14,000 an item, while the product pauses (geometry 5,800, contraction
-// 4,800, the rest sums over rows and set-up).  512 at most, for the accuracy of the FP32 sums over a range.
-static int pt_range(const int64_t *sys_off, int nsys, int sms)
+static int pt_width(bool fp64) { return 2 * (fp64 ? P64_PART : PT_PART); }
+static int64_t pt_items(int64_t nb2, bool fp64) { return fp64 ? nb2 * (nb2 + 1) : nb2 * (nb2 + 1) / 2; }
+// panel steps of a range of k: slabs of 32 columns (three per 32 particles), or 8 particles
+static int pt_steps(int64_t k, bool fp64) { return fp64 ? (int)((k + P64_K - 1) / P64_K) : (int)((k + 31) / 32 * 3); }
+
+// Particles k of one item: the range length with the least estimated time of all items.  Mixed: 1,536 cycles
+// a slab (what its product takes) and 14,000 an item, while the product pauses (geometry 5,800, contraction
+// 4,800, the rest sums over rows and set-up).  FP64: 3,072 cycles for 8 k, 6,000 an item.  512 at most, for the
+// accuracy of the mixed form's FP32 sums over a range, and for L2.
+static int pt_range(const int64_t *sys_off, int nsys, int sms, bool fp64)
 {
+    const int units = fp64 ? sms : sms / 2;  // items in flight
     int best = 512;
     double least = 0.0;
     for (int kp : {512, 384, 256, 192, 128, 96, 64, 32}) {
         int64_t items = 0;
-        double slabs = 0.0;
+        double steps = 0.0;
         for (int s = 0; s < nsys; ++s) {
-            const int64_t n = sys_off[s + 1] - sys_off[s], nb2 = (n + 2 * PT_PART - 1) / (2 * PT_PART);
-            items += nb2 * (nb2 + 1) / 2 * ((n + kp - 1) / kp);
-            slabs += (double)(nb2 * (nb2 + 1) / 2) * (double)((n + 31) / 32 * 3);
+            const int64_t n = sys_off[s + 1] - sys_off[s], nb2 = (n + pt_width(fp64) - 1) / pt_width(fp64);
+            items += pt_items(nb2, fp64) * ((n + kp - 1) / kp);
+            steps += (double)pt_items(nb2, fp64) * (double)pt_steps(n, fp64);
         }
-        const int pairs = sms / 2;
-        const double t = (double)((items + pairs - 1) / pairs) * (slabs / (double)(items ? items : 1) * 1536.0 + 14000.0);
+        const double t = (double)((items + units - 1) / units) *
+                         (steps / (double)(items ? items : 1) * (fp64 ? 3072.0 : 1536.0) + (fp64 ? 6000.0 : 14000.0));
         if (kp == 512 || t < 0.98 * least) {
             least = t;
             best = kp;
@@ -751,18 +983,21 @@ static int pt_range(const int64_t *sys_off, int nsys, int sms)
 
 // Panels, tiles and results of all systems, in groups whose panel and results stay within `budget` bytes
 // (a group has at least one range); a system may go over several groups.
-void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, PtPlan &plan)
+void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, bool fp64, PtPlan &plan)
 {
+    static_assert(P64_BLOCK * sizeof(double) == PT_BLOCK_BYTES, "both forms' panels are planned alike");
     plan = PtPlan{};
-    const int kp = pt_range(sys_off, nsys, sms);
+    plan.fp64 = fp64;
+    plan.slot_bytes = sizeof(double) * (size_t)(fp64 ? P64_SLOT : PT_SLOT);
+    const int kp = pt_range(sys_off, nsys, sms, fp64);
     PtGroup g{};
     for (int s = 0; s < nsys; ++s) {
         const int64_t n = sys_off[s + 1] - sys_off[s];
         if (n < 1) continue;
-        const int nb2 = (int)((n + 2 * PT_PART - 1) / (2 * PT_PART));
+        const int nb2 = (int)((n + pt_width(fp64) - 1) / pt_width(fp64));
         const int64_t tiles = (int64_t)nb2 * (nb2 + 1);
         const int tab = (int)plan.tiles.size();
-        pt_tiles(nb2, plan.tiles);
+        pt_tiles(nb2, fp64, plan.tiles);
         PtSys sy{sys_off[s], g.slots, (int)n, nb2, 0, s, 0, 0};
         auto end_system = [&]() {
             if (!sy.nseg) return;
@@ -770,9 +1005,9 @@ void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, PtPlan &p
             ++g.nsys;
         };
         for (int64_t k0 = 0; k0 < n; k0 += kp) {
-            const int nslab = ((int)std::min<int64_t>(kp, n - k0) + 31) / 32 * 3;
+            const int nslab = pt_steps(std::min<int64_t>(kp, n - k0), fp64);
             const size_t mem = (size_t)nb2 * 2 * nslab * PT_BLOCK_BYTES;
-            if (g.nsegs && g.mem + mem + (size_t)(g.slots + tiles) * PT_SLOT * sizeof(double) > budget) {
+            if (g.nsegs && g.mem + mem + (size_t)(g.slots + tiles) * plan.slot_bytes > budget) {
                 end_system();
                 plan.groups.push_back(g);
                 g = PtGroup{};
@@ -785,9 +1020,9 @@ void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, PtPlan &p
             plan.segs.push_back(PtSeg{(int64_t)g.mem, g.items, g.slots, (int)sys_off[s], (int)n, (int)k0, nslab, tab,
                                       g.gen});
             g.mem += mem;
-            g.items += tiles / 2;
+            g.items += pt_items(nb2, fp64);
             g.slots += tiles;
-            g.gen += 2 * nb2 * (nslab / 3);
+            g.gen += 2 * nb2 * (fp64 ? nslab : nslab / 3);
             ++g.nsegs;
             ++sy.nseg;
         }
@@ -800,36 +1035,44 @@ void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, PtPlan &p
     }
 }
 
-size_t pt_slot_bytes() { return PT_SLOT * sizeof(double); }
-
 cudaError_t pt_init()
 {
-    const cudaError_t e =
-        cudaFuncSetAttribute(k_pt_gemm<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PtShared));
-    return e != cudaSuccess ? e
-                            : cudaFuncSetAttribute(k_pt_gemm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)sizeof(PtShared));
+    cudaError_t e;
+    for (auto k : {k_pt_gemm<false>, k_pt_gemm<true>})
+        if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PtShared))) != cudaSuccess)
+            return e;
+    for (auto k : {k_p64_gemm<false>, k_p64_gemm<true>})
+        if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(P64Shared))) != cudaSuccess)
+            return e;
+    return cudaSuccess;
 }
 
 cudaError_t launch_pairs(Pos pos, Out out, const PtPlan &plan, const PtDev &d, double *energy,
                          double nu, int sms, cudaStream_t st, int *launches)
 {
-    static_assert(sizeof(PtShared) <= 232448, "shared memory of one block");
+    static_assert(sizeof(PtShared) <= 232448 && sizeof(P64Shared) <= 232448, "shared memory of one block");
     for (const PtGroup &g : plan.groups) {
         const PtSeg *seg = d.segs + g.seg0;
         const PtSys *sys = d.sys + g.sys0;
         const PtSys &first = plan.sys[g.sys0], &last = plan.sys[g.sys0 + g.nsys - 1];
         const int64_t np = last.part0 + last.n - first.part0;
-        k_pt_panel<<<(unsigned)g.gen, PT_PANEL_THREADS, 0, st>>>(pos, seg, g.nsegs, d.panel);
-        const unsigned blocks = 2 * (unsigned)std::min<int64_t>(g.items, sms / 2);
-        auto gemm = energy ? k_pt_gemm<true> : k_pt_gemm<false>;
-        gemm<<<blocks, PT_WARPS * 32, sizeof(PtShared), st>>>(pos, seg, g.nsegs, g.items, d.tiles, d.panel, d.slots, nu, d.err);
-        k_pt_reduce<<<(unsigned)((np + 7) / 8), 256, 0, st>>>(first.part0, np, sys, g.nsys, d.slots, out, d.err);
-        *launches += 3;
-        if (energy) {
-            k_pt_energy<<<(unsigned)g.nsys, 512, 0, st>>>(sys, d.slots, energy);
-            *launches += 1;
+        const unsigned reduce_blocks = (unsigned)((np + 7) / 8);
+        if (plan.fp64) {
+            k_p64_panel<<<(unsigned)g.gen, P64_K * P64_PART, 0, st>>>(pos, seg, g.nsegs, (double *)d.panel);
+            auto gemm = energy ? k_p64_gemm<true> : k_p64_gemm<false>;
+            gemm<<<(unsigned)std::min<int64_t>(g.items, sms), 256, sizeof(P64Shared), st>>>(
+                pos, seg, g.nsegs, g.items, d.tiles, (const double *)d.panel, d.slots, nu, d.err);
+            k_pt_reduce<P64_PART><<<reduce_blocks, 256, 0, st>>>(first.part0, np, sys, g.nsys, d.slots, out, d.err);
+            if (energy) k_pt_energy<P64_PART><<<(unsigned)g.nsys, 512, 0, st>>>(sys, d.slots, energy);
+        } else {
+            k_pt_panel<<<(unsigned)g.gen, PT_PANEL_THREADS, 0, st>>>(pos, seg, g.nsegs, d.panel);
+            auto gemm = energy ? k_pt_gemm<true> : k_pt_gemm<false>;
+            gemm<<<2 * (unsigned)std::min<int64_t>(g.items, sms / 2), PT_WARPS * 32, sizeof(PtShared), st>>>(
+                pos, seg, g.nsegs, g.items, d.tiles, d.panel, d.slots, nu, d.err);
+            k_pt_reduce<PT_PART><<<reduce_blocks, 256, 0, st>>>(first.part0, np, sys, g.nsys, d.slots, out, d.err);
+            if (energy) k_pt_energy<PT_PART><<<(unsigned)g.nsys, 512, 0, st>>>(sys, d.slots, energy);
         }
+        *launches += energy ? 4 : 3;
     }
     return cudaGetLastError();
 }
