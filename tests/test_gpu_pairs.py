@@ -46,6 +46,29 @@ def test_pair_tensor_forces(algo, n, precision):
     assert all(np.array_equal(a, b) for a, b in zip((fx, fy, fz, e), again))  # fixed order of summation
 
 
+@pytest.mark.parametrize("n", [299, 300, 336, 337, 385, 504, 513, 640])
+def test_pair_tensor_adjoint(n):
+    """The mixed adjoint (H g and the strength's gradient) against the FP64 one, within the 1e-5 that every
+    mixed adjoint is held to; the same in every run."""
+    x, y, z = lattice(n, n)
+    g = np.random.default_rng(n).standard_normal((3, n))
+    out = {}
+    for precision in ("fp64", "mixed", "mixed"):
+        ctx = Context("auta", precision, nu=0.8)
+        ctx.set_particles(x, y, z)
+        h = ctx.adjoint(*g, 0.3)
+        st = ctx.get_state()
+        ctx.close()
+        r = (np.stack(h[:3]), h[3], np.stack([st[k] for k in ("fx", "fy", "fz")]))
+        if precision in out and n >= 300:
+            assert all(np.array_equal(a, b) for a, b in zip(r, out[precision]))
+        out[precision] = r
+    (hm, num, fm), (h, nu, f) = out["mixed"], out["fp64"]
+    assert rel(hm, h) <= 1e-5
+    assert rel(fm, f) <= 1e-5
+    assert abs(num - nu) <= 1e-5 * (np.abs(g * f).sum() + abs(nu))
+
+
 @pytest.mark.parametrize("precision", PRECISIONS)
 def test_pair_tensor_batch_of_uneven_systems(precision):
     sizes = [1, 84, 2, 0, 300, 43, 3, 42, 85, 126, 500]

@@ -59,7 +59,7 @@ struct GraphKey {
     SweepWork sweep;
     PtDev pairs;
     const void *table, *state, *step_counts, *partial;
-    int64_t n;
+    int64_t n, pairs_items;
     int max_stage, sweep_grid;
 };
 
@@ -116,12 +116,14 @@ struct tbmd_ctx {
     // counter and the workspaces), and tables are rewritten after it on the host.
     cudaEvent_t ws_event = nullptr;
     cudaStream_t ws_stream = nullptr;
-    // no-cutoff forces of the mixed form as a product of pair tensors: the systems the plan was made
-    // for (their particle offsets), its tables on the device, panel, tile results
-    std::vector<int64_t> pt_off;
-    PtPlan pt;
-    PtDev pt_dev{};
-    DevBuf pt_tab, pt_panel, pt_slots;
+    // no-cutoff evaluations as a product of pair tensors, [0] forces, [1] the mixed form's adjoint: the systems
+    // the plan was made for (their particle offsets), its tables on the device, panels, tile results
+    struct PairState {
+        std::vector<int64_t> off;
+        PtPlan plan;
+        PtDev dev{};
+        DevBuf tab, panel, slots, panel2, slots2;
+    } pairs[2];
     int sms = 0;
 
     // P3BCA
@@ -348,42 +350,50 @@ static SweepWork single_sweep(tbmd_ctx *ctx, bool dual)
                      (const int32_t *)(t + 40), l.kseg};
 }
 
-// Whether the no-cutoff forces of a system (or the largest of a batch) go through the pair-tensor product
-// (tbmd_pairs.cu) instead of a sweep: the mixed form's forces.  At n = 128 both take about 50 us on the
-// device (46 against 54), from there on the product is faster (n = 1000: 0.21 against 0.94 ms, 8192: 71
-// against 240 ms for AUTA and 541 for NATA); above 65,536 its panel and tile results would pass 4 GB.
-constexpr int64_t kPairsMin = 128, kPairsMax = 65536;
+// Whether the no-cutoff evaluation of a system (or the largest of a batch) goes through the pair-tensor
+// product (tbmd_pairs.cu) instead of a sweep: the forces of both precisions, and the mixed adjoint.  Forces:
+// at n = 128 both take the same time on the device (mixed 46 and 54 us, FP64 34 and 34), from there on the
+// product is faster (n = 1000: mixed 0.21 against 0.94 ms, 8192: 71 against 240 ms for AUTA and 541 for NATA;
+// FP64 213 against 385 and 1021).  Mixed adjoint: n = 130 177 against 133 us, 300 187 against 200, 2500 6.1
+// against 19.4 ms.  Above 65,536 the panel and tile results would pass 4 GB.
+constexpr int64_t kPairsMin = 128, kPairsMinAdjoint = 300, kPairsMax = 65536;
 static bool use_pairs(const tbmd_ctx *ctx, int64_t n, bool dual)
 {
-    return !dual && n >= kPairsMin && n <= kPairsMax;
+    return (mixed(ctx) || !dual) && n >= (dual ? kPairsMinAdjoint : kPairsMin) && n <= kPairsMax;
 }
 
 // Plan, tables and workspaces of the pair-tensor product for systems at offsets off[0 .. nsys].  The
-// panel and the tile results of one launch stay within 1 GB (one range of k where that takes more).
-static tbmd_status ensure_pairs(tbmd_ctx *ctx, const int64_t *off, int nsys)
+// panel and the tile results of one launch stay within 1 GB (one range of k where that takes more), twice
+// that for the adjoint.
+static tbmd_status ensure_pairs(tbmd_ctx *ctx, const int64_t *off, int nsys, bool dual)
 {
-    if (ctx->pt_off.size() == (size_t)nsys + 1 && std::memcmp(ctx->pt_off.data(), off, sizeof(int64_t) * (nsys + 1)) == 0)
+    tbmd_ctx::PairState &s = ctx->pairs[dual ? 1 : 0];
+    if (s.off.size() == (size_t)nsys + 1 && std::memcmp(s.off.data(), off, sizeof(int64_t) * (nsys + 1)) == 0)
         return TBMD_OK;
     CK(ws_wait_host(ctx));  // a launch on a caller's stream may still read the old tables
-    ctx->pt_off.clear();
-    invalidate_graph(ctx);
+    s.off.clear();
     if (!ctx->sms) CK(cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device));
     CK(pt_init());
-    pt_plan(off, nsys, ctx->sms, (size_t)1 << 30, !mixed(ctx), ctx->pt);
-    const PtPlan &p = ctx->pt;
+    pt_plan(off, nsys, ctx->sms, (size_t)1 << 30, !mixed(ctx), dual, s.plan);
+    const PtPlan &p = s.plan;
     const size_t b_seg = sizeof(PtSeg) * p.segs.size(), b_sys = sizeof(PtSys) * p.sys.size(),
                  b_til = sizeof(unsigned int) * p.tiles.size();
-    CK(ctx->pt_tab.ensure(b_seg + b_sys + b_til));
-    CK(ctx->pt_panel.ensure(p.mem));
-    CK(ctx->pt_slots.ensure(p.slots * p.slot_bytes));
-    char *t = ctx->pt_tab.as<char>();
+    CK(s.tab.ensure(b_seg + b_sys + b_til));
+    CK(s.panel.ensure(p.mem));
+    CK(s.slots.ensure(p.slots * p.slot_bytes));
+    if (dual) {
+        CK(s.panel2.ensure(p.mem));
+        CK(s.slots2.ensure(p.slots * p.slot_bytes));
+    }
+    char *t = s.tab.as<char>();
     CK(cudaMemcpyAsync(t, p.segs.data(), b_seg, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(t + b_seg, p.sys.data(), b_sys, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(t + b_seg + b_sys, p.tiles.data(), b_til, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    ctx->pt_dev = PtDev{(const PtSeg *)t, (const PtSys *)(t + b_seg), (const unsigned int *)(t + b_seg + b_sys),
-                        ctx->pt_panel.as<unsigned char>(), ctx->pt_slots.as<double>(), pairs_err(ctx)};
-    ctx->pt_off.assign(off, off + nsys + 1);
+    s.dev = PtDev{(const PtSeg *)t, (const PtSys *)(t + b_seg), (const unsigned int *)(t + b_seg + b_sys),
+                  s.panel.as<unsigned char>(), s.slots.as<double>(), s.panel2.as<unsigned char>(), s.slots2.as<double>(),
+                  pairs_err(ctx)};
+    s.off.assign(off, off + nsys + 1);
     return TBMD_OK;
 }
 
@@ -549,7 +559,7 @@ static tbmd_status prepare(tbmd_ctx *ctx, int64_t n, bool dual, bool energy)
     if (is_p3bca_cut(ctx)) return ensure_cells(ctx, n, dual, energy);
     if (use_pairs(ctx, n, dual)) {
         const int64_t off[2] = {0, n};
-        return ensure_pairs(ctx, off, 1);
+        return ensure_pairs(ctx, off, 1, dual);
     }
     const int alg = dual ? TBMD_AUTA : (ctx->cfg.algorithm == TBMD_NATA ? TBMD_NATA : TBMD_AUTA);
     const int R = dual ? (mixed(ctx) ? 2 : 1) : sweep_R(ctx);
@@ -585,7 +595,8 @@ static tbmd_status enqueue_forces(tbmd_ctx *ctx, int64_t n, Pos pos, Out out, bo
     }
     phase_mark(ctx, st, PH_TRIPLETS, *nl);
     if (use_pairs(ctx, n, dual)) {
-        CK(launch_pairs(pos, out, ctx->pt, ctx->pt_dev, energy, nu, ctx->sms, st, nl));
+        const tbmd_ctx::PairState &s = ctx->pairs[dual ? 1 : 0];
+        CK(launch_pairs(dual, pos, out, s.plan, s.dev, energy, nu, ctx->sms, st, nl));
         phase_mark(ctx, st, PH_UPDATE, *nl);
         if (count) {
             k_add_u64<<<1, 1, 0, st>>>(count, choose3(n));
@@ -693,7 +704,8 @@ static void fill_graph_key(tbmd_ctx *ctx, GraphKey &k)
         k.table = ctx->ncell_tab.p;
         k.max_stage = ctx->max_stage;
     } else if (use_pairs(ctx, ctx->n, false)) {
-        k.pairs = ctx->pt_dev;
+        k.pairs = ctx->pairs[0].dev;
+        k.pairs_items = ctx->pairs[0].plan.groups.empty() ? 0 : ctx->pairs[0].plan.groups[0].items;
     } else {
         k.sweep = single_sweep(ctx, false);
         k.partial = ctx->partial.p;
@@ -842,8 +854,9 @@ void tbmd_destroy(tbmd_ctx *ctx)
     for (DevBuf *b : {&ctx->state, &ctx->snapshot, &ctx->scalars, &ctx->step_counts, &ctx->partial,
                       &ctx->cell_n, &ctx->cell_c, &ctx->nbr_buf, &ctx->dirs, &ctx->hvp, &ctx->gset_single,
                       &ctx->sweep[0].sys, &ctx->sweep[0].prefix, &ctx->sweep[1].sys, &ctx->sweep[1].prefix, &ctx->bpos, &ctx->bout, &ctx->bsys, &ctx->bprefix, &ctx->ncell_tab,
-                      &ctx->staging, &ctx->long_buf, &ctx->gen_buf, &ctx->bext, &ctx->pt_tab, &ctx->pt_panel,
-                      &ctx->pt_slots})
+                      &ctx->staging, &ctx->long_buf, &ctx->gen_buf, &ctx->bext, &ctx->pairs[0].tab, &ctx->pairs[0].panel,
+                      &ctx->pairs[0].slots, &ctx->pairs[1].tab, &ctx->pairs[1].panel, &ctx->pairs[1].slots,
+                      &ctx->pairs[1].panel2, &ctx->pairs[1].slots2})
         b->release();
     if (ctx->hpin) cudaFreeHost(ctx->hpin);
     if (ctx->copy_stream) {
@@ -1791,11 +1804,12 @@ static tbmd_status batch_eval(tbmd_ctx *ctx, int32_t nsys, const int64_t *offset
         CK(cudaMemcpyAsync(c.data(), CNT, sizeof(unsigned long long) * nsys, cudaMemcpyDeviceToHost, sm));
         CK(cudaStreamSynchronize(sm));
         for (int s = 0; s < nsys; ++s) res.counts[s] = c[s];
-    } else if (!dual && N >= kPairsMin && nmax <= kPairsMax) {
+    } else if ((mx || !dual) && N >= (dual ? kPairsMinAdjoint : kPairsMin) && nmax <= kPairsMax) {
         CK(reset_cap_flags(ctx, sm));
-        st = ensure_pairs(ctx, offsets, nsys);
+        st = ensure_pairs(ctx, offsets, nsys, dual);
         if (st != TBMD_OK) return st;
-        CK(launch_pairs(pos, out, ctx->pt, ctx->pt_dev, E, nu, ctx->sms, sm, &nl));
+        const tbmd_ctx::PairState &s = ctx->pairs[dual ? 1 : 0];
+        CK(launch_pairs(dual, pos, out, s.plan, s.dev, E, nu, ctx->sms, sm, &nl));
         CapSeen seen{};
         CK(read_cap_flags(ctx, sm, &seen));
         CK(cudaStreamSynchronize(sm));

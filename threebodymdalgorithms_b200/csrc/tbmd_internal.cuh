@@ -370,12 +370,14 @@ struct PtDev {
     const unsigned int *tiles;
     unsigned char *panel;
     double *slots;
+    unsigned char *panel2;  // adjoint: the tensors' rates
+    double *slots2;         // and the tiles' results for H d
     unsigned int *err;  // set by a launch that gave up waiting
 };
-void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, bool fp64, PtPlan &plan);
+void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, bool fp64, bool dual, PtPlan &plan);
 cudaError_t pt_init();
-// forces overwritten; energy (one accumulator per system, may be NULL) added to
-cudaError_t launch_pairs(Pos pos, Out out, const PtPlan &plan, const PtDev &d, double *energy,
+// dual (mixed form): also H d into out.h; forces overwritten; energy (one accumulator per system, may be NULL) added to
+cudaError_t launch_pairs(bool dual, Pos pos, Out out, const PtPlan &plan, const PtDev &d, double *energy,
                          double nu, int sms, cudaStream_t st, int *launches);
 
 // P3BCA pipeline

@@ -1,4 +1,5 @@
-// No-cutoff forces and energy of the mixed form as a matrix product on the tensor cores.
+// No-cutoff forces and energy as a matrix product: the mixed form (and its adjoint) on the tensor cores, the
+// FP64 form on the FP64 matrix instruction (second part of this file).
 //
 // With the pair tensors T_ij = (3 r r^T - r^2) / r^5 (r = x_j - x_i, symmetric, traceless, T_ii = 0) the
 // Axilrod-Teller energy of a triplet is -nu/3 tr(T_ij T_jk T_ki), so over all triplets
@@ -55,8 +56,10 @@ constexpr int PT_SLOT = pt_slot(PT_PART);
 
 struct PtShared {
     unsigned char stage[PT_STAGES][PT_STAGE_BYTES];
-    float4 geo[2][PT_GEO];  // (n_x n_x' n_y n_y') and (n_z n_z' r^-4 r'^-4) of particle i and two j
-    double xj[3][2 * PT_PART], xi[3][PT_PART];  // positions of the tile's particles
+    // (n_x n_x' n_y n_y') and (n_z n_z' r^-4 r'^-4) of particle i and two j; with the second-order terms for one
+    // column block at a time, its rates behind it
+    float4 geo[2][PT_GEO];
+    double xj[6][2 * PT_PART], xi[6][PT_PART];  // positions of the tile's particles, and their directions
     double fi[2][PT_ROWS][3];
     float fj[8][PT_ROWS];
     double e[8];
@@ -289,6 +292,7 @@ __device__ __forceinline__ void split3(double v, unsigned short &h, unsigned sho
 // i and 8 particles k: 24 columns of its three rows, three 16-byte chunks per row and split.  The stores
 // are 16-byte pieces that L2 merges; the panel is 0.4% of the product's time at n = 8192.
 constexpr int PT_PANEL_THREADS = 192;
+template <bool TANGENT>
 __global__ void __launch_bounds__(PT_PANEL_THREADS) k_pt_panel(Pos pos, const PtSeg *__restrict__ seg, int nseg,
                                                               unsigned char *__restrict__ panel)
 {
@@ -300,11 +304,16 @@ __global__ void __launch_bounds__(PT_PANEL_THREADS) k_pt_panel(Pos pos, const Pt
     if (il > PT_PART + 1) return;  // 42 and 43 are the two rows left over
     const int i = rb * PT_PART + il;
     const bool row_ok = il < PT_PART && i < s.n;
-    double xi = 0.0, yi = 0.0, zi = 0.0;
+    double xi = 0.0, yi = 0.0, zi = 0.0, ui = 0.0, vi = 0.0, wi = 0.0;
     if (row_ok) {
         xi = pos.x[s.part0 + i];
         yi = pos.y[s.part0 + i];
         zi = pos.z[s.part0 + i];
+        if (TANGENT) {
+            ui = pos.dx[s.part0 + i];
+            vi = pos.dy[s.part0 + i];
+            wi = pos.dz[s.part0 + i];
+        }
     }
     // packed bfloat16 pairs of the 24 columns: [split][row a][12 words]
     unsigned int w[3][3][12];
@@ -322,12 +331,23 @@ __global__ void __launch_bounds__(PT_PANEL_THREADS) k_pt_panel(Pos pos, const Pt
             const double x = pos.x[s.part0 + k] - xi, y = pos.y[s.part0 + k] - yi, z = pos.z[s.part0 + k] - zi;
             const double ri = rsqrt(fma(x, x, fma(y, y, z * z)));
             const double ri2 = ri * ri, i3 = ri * ri2, s5 = 3.0 * i3 * ri2;
-            t[0] = fma(s5 * x, x, -i3);
-            t[1] = s5 * x * y;
-            t[2] = s5 * x * z;
-            t[3] = fma(s5 * y, y, -i3);
-            t[4] = s5 * y * z;
-            t[5] = fma(s5 * z, z, -i3);
+            if (TANGENT) {  // dT along the directions: r' = (u v w)
+                const double u = pos.dx[s.part0 + k] - ui, v = pos.dy[s.part0 + k] - vi, w = pos.dz[s.part0 + k] - wi;
+                const double rr = fma(x, u, fma(y, v, z * w)), c = s5 * rr, e = -5.0 * c * ri2;
+                t[0] = fma(e * x, x, fma(2.0 * s5 * x, u, c));
+                t[1] = fma(e * x, y, s5 * fma(x, v, y * u));
+                t[2] = fma(e * x, z, s5 * fma(x, w, z * u));
+                t[3] = fma(e * y, y, fma(2.0 * s5 * y, v, c));
+                t[4] = fma(e * y, z, s5 * fma(y, w, z * v));
+                t[5] = fma(e * z, z, fma(2.0 * s5 * z, w, c));
+            } else {
+                t[0] = fma(s5 * x, x, -i3);
+                t[1] = s5 * x * y;
+                t[2] = s5 * x * z;
+                t[3] = fma(s5 * y, y, -i3);
+                t[4] = s5 * y * z;
+                t[5] = fma(s5 * z, z, -i3);
+            }
         }
         constexpr int at[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
 #pragma unroll
@@ -363,6 +383,29 @@ __global__ void __launch_bounds__(PT_PANEL_THREADS) k_pt_panel(Pos pos, const Pt
     }
 }
 
+// Sums of 18 values over the warp's lanes into dst[0 .. 17] (a butterfly that halves the values with the
+// lanes: 16, then the last two).
+__device__ __forceinline__ void warp_sums18(float *v, float *dst, int lane)
+{
+#pragma unroll
+    for (int o = 16, m = 8; o >= 2; o >>= 1, m >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (q < m) {
+                const float keep = up ? v[q + m] : v[q], send = up ? v[q] : v[q + m];
+                v[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+    }
+    const bool up = (lane & 16) != 0;
+    float w = (up ? v[17] : v[16]) + __shfl_xor_sync(0xffffffffu, up ? v[16] : v[17], 16);
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+#pragma unroll
+    for (int o = 8; o >= 1; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+    if ((lane & 1) == 0) dst[(lane >> 4 & 1) * 8 + (lane >> 3 & 1) * 4 + (lane >> 2 & 1) * 2 + (lane >> 1 & 1)] = v[0];
+    if ((lane & 15) == 0) dst[16 + (lane >> 4)] = w;
+}
+
 // One item of a cluster: row blocks 2 a and 2 a + 1 (one per block) and column blocks 2 b and 2 b + 1 of G
 // over one segment's k.
 struct PtItem {
@@ -379,14 +422,20 @@ __device__ __forceinline__ PtItem pt_item(const PtSeg *seg, int nseg, const unsi
     return it;
 }
 
-template <bool ENERGY>
+// MODE 0: forces (and energy).  The adjoint's H d, with T' and r' the rates of T and r along d, is
+//   sum_j (G'_ij : dT/dr + G_ij : d(dT/dr)/dr r'),  G' = T' T + T T'
+// MODE 1: forces, energy and the second term, from G; MODE 2: the first, from G', whose two products follow
+// one another into the same sums (panel2 holds T').
+template <int MODE, bool ENERGY>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
     k_pt_gemm(Pos pos, const PtSeg *__restrict__ seg, int nseg, int64_t items, const unsigned int *__restrict__ tiles,
-              const unsigned char *__restrict__ panel, double *__restrict__ slots, double nu, unsigned int *err)
+              const unsigned char *__restrict__ panel, const unsigned char *__restrict__ panel2,
+              double *__restrict__ slots, double *__restrict__ slots2, double nu, unsigned int *err)
 {
     extern __shared__ __align__(1024) unsigned char smraw[];
     PtShared &S = *(PtShared *)smraw;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto slabs_of = [](const PtItem &it) { return MODE == 2 ? 2 * it.s.nslab : it.s.nslab; };
     const int rank = blockIdx.x & 1, cluster = blockIdx.x >> 1, clusters = gridDim.x >> 1;
     if (threadIdx.x == 0) {
         for (int k = 0; k < PT_STAGES; ++k) {
@@ -422,15 +471,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
             for (int64_t w = cluster; w < items; w += clusters) {
                 const PtItem it = pt_item(seg, nseg, tiles, w);
                 const int64_t row = (int64_t)it.s.nslab * PT_BLOCK_BYTES;
-                const unsigned char *pa = panel + it.s.mem + (2 * it.a + rank) * row,
-                                    *pb = panel + it.s.mem + (2 * it.b + rank) * row;
-                for (int k = 0; k < it.s.nslab; ++k, ++n) {
+                const int64_t oa = it.s.mem + (2 * it.a + rank) * row, ob = it.s.mem + (2 * it.b + rank) * row;
+                for (int k = 0; k < slabs_of(it); ++k, ++n) {
                     const int st = n % PT_STAGES;
                     if (!bar_wait(&S.empty[st], ((n / PT_STAGES) & 1) ^ 1, S, err)) break;
+                    // MODE 2: T' T, then T T'
+                    const bool second = MODE == 2 && k >= it.s.nslab;
+                    const int64_t ko = (int64_t)(second ? k - it.s.nslab : k) * PT_BLOCK_BYTES;
                     unsigned char *dst = S.stage[st];
                     bar_expect(&S.full[st], PT_STAGE_BYTES);
-                    bulk_load(dst, pa + (int64_t)k * PT_BLOCK_BYTES, PT_BLOCK_BYTES, &S.full[st]);
-                    bulk_load(dst + PT_BLOCK_BYTES, pb + (int64_t)k * PT_BLOCK_BYTES, PT_BLOCK_BYTES, &S.full[st]);
+                    bulk_load(dst, (MODE == 2 && !second ? panel2 : panel) + oa + ko, PT_BLOCK_BYTES, &S.full[st]);
+                    bulk_load(dst + PT_BLOCK_BYTES, (second ? panel2 : panel) + ob + ko, PT_BLOCK_BYTES, &S.full[st]);
                 }
                 if (*(volatile int *)&S.dead) break;
             }
@@ -447,7 +498,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
             unsigned int n = 0;
             for (int64_t w = cluster; w < items; w += clusters) {
                 const PtItem it = pt_item(seg, nseg, tiles, w);
-                for (int k = 0; k < it.s.nslab; ++k, ++n) {
+                for (int k = 0; k < slabs_of(it); ++k, ++n) {
                     if (!bar_wait(&S.full[n % PT_STAGES], (n / PT_STAGES) & 1, S, err)) break;
                     bar_arrive_at(&S.full[n % PT_STAGES], 0);
                 }
@@ -459,7 +510,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
             bool ok = true;
             for (int64_t w = cluster; ok && w < items; w += clusters) {
                 const PtItem it = pt_item(seg, nseg, tiles, w);
-                for (int k = 0; k < it.s.nslab; ++k, ++n) {
+                for (int k = 0; k < slabs_of(it); ++k, ++n) {
                     const int st = n % PT_STAGES, buf = n & 1;
                     ok = bar_wait(&S.acc_empty[buf], ((n >> 1) & 1) ^ 1, S, err) &&
                          bar_wait(&S.full[st], (n / PT_STAGES) & 1, S, err);
@@ -500,6 +551,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
                     d[0] = pos.x[p];
                     d[step] = pos.y[p];
                     d[2 * step] = pos.z[p];
+                    if (MODE == 1) {
+                        d[3 * step] = pos.dx[p];
+                        d[4 * step] = pos.dy[p];
+                        d[5 * step] = pos.dz[p];
+                    }
                 }
                 __syncwarp();
                 if (lane == 0) bar_arrive(&S.geo_full);
@@ -519,7 +575,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
             f2 g2[64];  // columns 2 c and 2 c + 1
 #pragma unroll
             for (int c = 0; c < 64; ++c) g2[c] = 0ull;
-            for (int k = 0; k < it.s.nslab; ++k, ++n) {
+            for (int k = 0; k < slabs_of(it); ++k, ++n) {
                 const int buf = n & 1;
                 if (!bar_wait(&S.acc_full[buf], (n >> 1) & 1, S, err)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -542,6 +598,151 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
             // the operands' reads leave shared memory no room for it while the product runs.
             const int i0 = (2 * it.a + rank) * PT_PART, j0 = 2 * it.b * PT_PART;
             bar_wait(&S.geo_full, m & 1, S, err);
+            // this warp's sums for the i of its rows, for its energy, and the tile's results from all warps'
+            auto store_i = [&](double x, double y, double z) {
+                S.fi[half][row][0] = x;
+                S.fi[half][row][1] = y;
+                S.fi[half][row][2] = z;
+            };
+            auto store_e = [&](double e) {
+                if (!ENERGY) return;
+                e = warp_sum(e);
+                if (lane == 0) S.e[warp] = e;
+            };
+            auto write_slot = [&](double *to, bool with_energy) {
+                double *slot = to + (it.s.slot0 + (int64_t)it.b * (it.b + 1) + 2 * it.a + rank) * PT_SLOT;
+                const int t = threadIdx.x;
+                if ((t & 127) < 126) {
+                    double v = 0.0;
+                    for (int q = 0; q < 4; ++q) v += (double)S.fj[(t >> 7) * 4 + q][t & 127];
+                    const int c = t & 127;
+                    slot[126 + (t >> 7) * 126 + 3 * (2 * (c / 6) + (c & 1)) + (c % 6 >> 1)] = -nu * v;
+                }
+                if (t < 126) {
+                    const int p = t / 3, c = t - 3 * p;
+                    double v = 0.0;
+                    for (int h = 0; h < 2; ++h)
+                        for (int q = 0; q < 3; ++q) v += S.fi[h][pt_row(p, q)][c];
+                    slot[t] = nu * v;
+                }
+                if (with_energy && t == 255) {
+                    double v = 0.0;
+                    for (int q = 0; q < 8; ++q) v += S.e[q];
+                    slot[378] = -nu * v / 9.0;
+                }
+            };
+            const int go = (MODE == 1 ? 0 : half * (PT_PART / 2) * PT_PART) + (row < 3 * PT_PART ? ip : 0);
+            const float rv = row < 3 * PT_PART ? 1.f : 0.f;
+            double fx = 0.0, fy = 0.0, fz = 0.0, en = 0.0;
+            [[maybe_unused]] double hx = 0.0, hy = 0.0, hz = 0.0;
+            if constexpr (MODE == 1) {
+                // One column block after the other, since shared memory holds the geometry and its rates for
+                // one: all warps form them, the block's four contract.  The rates along d are m = n' (the part
+                // of r' across n, over r) and q = |r|' / |r|; with U = y e + n_al g + (g_al - 5 n_al y) n the
+                // contraction r^-4 U of the forces has the rate
+                //   r^-4 (y' e + m_al g - 5 (m_al y + n_al y') n + (g_al - 5 n_al y) m - 4 q U),  y' = g.m
+                constexpr int HALF = PT_GEO / 2;
+                float4 *gn = &S.geo[0][0], *gm = gn + 2 * HALF;
+                for (int h = 0; h < 2; ++h) {
+                    if (h) asm volatile("bar.sync 1, 256;" ::: "memory");  // the first block has been contracted
+                    for (int q = threadIdx.x; q < HALF; q += 256) {
+                        const int jp = q / PT_PART, il = q - jp * PT_PART, i = i0 + il, jl = h * PT_PART + 2 * jp;
+                        float v[2][8];
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            const int j = j0 + jl + u;
+                            const double x = S.xj[0][jl + u] - S.xi[0][il], y = S.xj[1][jl + u] - S.xi[1][il],
+                                         z = S.xj[2][jl + u] - S.xi[2][il];
+                            const double r2 = fma(x, x, fma(y, y, z * z)), t = (double)rsqrt_((float)r2);
+                            const double ri = fma(0.5 * fma(-r2, t * t, 1.0), t, t), ri2 = ri * ri;
+                            const double nx = x * ri, ny = y * ri, nz = z * ri;
+                            const double mx = (S.xj[3][jl + u] - S.xi[3][il]) * ri, my = (S.xj[4][jl + u] - S.xi[4][il]) * ri,
+                                         mz = (S.xj[5][jl + u] - S.xi[5][il]) * ri;
+                            const double qr = fma(nx, mx, fma(ny, my, nz * mz));
+                            const double w[8] = {nx,
+                                                 ny,
+                                                 nz,
+                                                 ri2 * ri2,
+                                                 fma(-qr, nx, mx),
+                                                 fma(-qr, ny, my),
+                                                 fma(-qr, nz, mz),
+                                                 -4.0 * qr};
+                            const bool ok = i < j && j < it.s.n;
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) v[u][k] = ok ? (float)w[k] : 0.f;
+                        }
+                        gn[q] = make_float4(v[0][0], v[1][0], v[0][1], v[1][1]);
+                        gn[HALF + q] = make_float4(v[0][2], v[1][2], v[0][3], v[1][3]);
+                        gm[q] = make_float4(v[0][4], v[1][4], v[0][5], v[1][5]);
+                        gm[HALF + q] = make_float4(v[0][6], v[1][6], v[0][7], v[1][7]);
+                    }
+                    asm volatile("bar.sync 1, 256;" ::: "memory");
+                    if (h == 1 && lane == 0) bar_arrive(&S.geo_empty);
+                    if (half != h) continue;
+#pragma unroll
+                    for (int p3 = 0; p3 < PT_PART / 2; p3 += 3) {
+                        f2 sx = 0ull, sy = 0ull, sz = 0ull, se = 0ull, tx = 0ull, ty = 0ull, tz = 0ull;
+                        float fv[18];  // on the j, in the order of the columns
+#pragma unroll
+                        for (int p = p3; p < p3 + 3; ++p) {
+                            const int q = p * PT_PART + go;
+                            const float4 A = gn[q], B = gn[HALF + q], C = gm[q], D = gm[HALF + q];
+                            const f2 nx = pack2(A.x, A.y), ny = pack2(A.z, A.w), nz = pack2(B.x, B.y);
+                            const f2 mx = pack2(C.x, C.y), my = pack2(C.z, C.w), mz = pack2(D.x, D.y), q4 = pack2(D.z, D.w);
+                            const f2 i4 = pack2(B.z * rv, B.w * rv);
+                            const f2 gx = g2[3 * p], gy = g2[3 * p + 1], gz = g2[3 * p + 2];
+                            const f2 y = dot2(gx, gy, gz, nx, ny, nz), yd = dot2(gx, gy, gz, mx, my, mz);
+                            const f2 na = al == 0 ? nx : al == 1 ? ny : nz, ga = al == 0 ? gx : al == 1 ? gy : gz,
+                                     ma = al == 0 ? mx : al == 1 ? my : mz;
+                            const f2 nay = mul2(na, y), sc = fma2(m5, nay, ga), dc = mul2(m5, fma2(ma, y, mul2(na, yd)));
+                            const f2 ux = fma2(ex, y, fma2(na, gx, mul2(sc, nx))), uy = fma2(ey, y, fma2(na, gy, mul2(sc, ny))),
+                                     uz = fma2(ez, y, fma2(na, gz, mul2(sc, nz)));
+                            const f2 vx = mul2(ux, i4), vy = mul2(uy, i4), vz = mul2(uz, i4);
+                            sx = add2(sx, vx);
+                            sy = add2(sy, vy);
+                            sz = add2(sz, vz);
+                            const int o = 6 * (p - p3);
+                            unpack2(vx, fv[o], fv[o + 1]);
+                            unpack2(vy, fv[o + 2], fv[o + 3]);
+                            unpack2(vz, fv[o + 4], fv[o + 5]);
+                            if (ENERGY) {
+                                const float q0 = rsqrt_(fmaxf(B.z, 1e-36f)), q1 = rsqrt_(fmaxf(B.w, 1e-36f));  // r^2
+                                se = fma2(mul2(i4, pack2(q0 * rsqrt_(q0), q1 * rsqrt_(q1))), fma2(c3, nay, mul2(m1, ga)), se);
+                            }
+                            g2[3 * p] = mul2(fma2(ex, yd, fma2(ma, gx, fma2(dc, nx, fma2(sc, mx, mul2(q4, ux))))), i4);
+                            g2[3 * p + 1] = mul2(fma2(ey, yd, fma2(ma, gy, fma2(dc, ny, fma2(sc, my, mul2(q4, uy))))), i4);
+                            g2[3 * p + 2] = mul2(fma2(ez, yd, fma2(ma, gz, fma2(dc, nz, fma2(sc, mz, mul2(q4, uz))))), i4);
+                            tx = add2(tx, g2[3 * p]);
+                            ty = add2(ty, g2[3 * p + 1]);
+                            tz = add2(tz, g2[3 * p + 2]);
+                        }
+                        warp_sums18(fv, &S.fj[warp][6 * p3], lane);
+                        float u0, u1;
+                        unpack2(sx, u0, u1);
+                        fx += (double)(u0 + u1);
+                        unpack2(sy, u0, u1);
+                        fy += (double)(u0 + u1);
+                        unpack2(sz, u0, u1);
+                        fz += (double)(u0 + u1);
+                        unpack2(se, u0, u1);
+                        if (ENERGY) en += (double)(u0 + u1);
+                        unpack2(tx, u0, u1);
+                        hx += (double)(u0 + u1);
+                        unpack2(ty, u0, u1);
+                        hy += (double)(u0 + u1);
+                        unpack2(tz, u0, u1);
+                        hz += (double)(u0 + u1);
+                    }
+                }
+                store_i(fx, fy, fz);
+                store_e(en);
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                write_slot(slots, ENERGY);
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                fx = hx;
+                fy = hy;
+                fz = hz;
+            } else {
             for (int q = threadIdx.x; q < PT_GEO; q += 256) {
                 const int jp = q / PT_PART, il = q - jp * PT_PART, i = i0 + il;
                 const double xi = S.xi[0][il], yi = S.xi[1][il], zi = S.xi[2][il];
@@ -566,9 +767,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
             // contraction: this thread's row (i, al) of G against dT_ij/dr for the 42 particles j of its
             // column block, two at a time; with g the row of G_ij, n = r / |r|, y = g.n and the unit vector e
             // of the row, its part of G_ij : dT/dr is 3 / r^4 (y e + n_al g + (g_al - 5 n_al y) n)
-            const int go = half * (PT_PART / 2) * PT_PART + (row < 3 * PT_PART ? ip : 0);
-            const float rv = row < 3 * PT_PART ? 1.f : 0.f;
-            double fx = 0.0, fy = 0.0, fz = 0.0, en = 0.0;
 #pragma unroll
             for (int p3 = 0; p3 < PT_PART / 2; p3 += 3) {
                 f2 sx = 0ull, sy = 0ull, sz = 0ull, se = 0ull;
@@ -605,6 +803,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
                 unpack2(se, u0, u1);
                 if (ENERGY) en += (double)(u0 + u1);
             }
+            }
             float g[128];
 #pragma unroll
             for (int c = 0; c < 63; ++c) unpack2(g2[c], g[2 * c], g[2 * c + 1]);
@@ -623,34 +822,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
             const int col = ((lane >> 4) & 1) * 64 + ((lane >> 3) & 1) * 32 + ((lane >> 2) & 1) * 16 +
                             ((lane >> 1) & 1) * 8 + (lane & 1) * 4;
             *(float4 *)&S.fj[warp][col] = make_float4(g[0], g[1], g[2], g[3]);
-            S.fi[half][row][0] = fx;
-            S.fi[half][row][1] = fy;
-            S.fi[half][row][2] = fz;
-            if (ENERGY) {
-                en = warp_sum(en);
-                if (lane == 0) S.e[warp] = en;
-            }
+            store_i(fx, fy, fz);
+            if (MODE == 0) store_e(en);
             asm volatile("bar.sync 1, 256;" ::: "memory");
-            double *slot = slots + (it.s.slot0 + (int64_t)it.b * (it.b + 1) + 2 * it.a + rank) * PT_SLOT;
-            const int t = threadIdx.x;
-            if ((t & 127) < 126) {
-                double v = 0.0;
-                for (int q = 0; q < 4; ++q) v += (double)S.fj[(t >> 7) * 4 + q][t & 127];
-                const int c = t & 127;
-                slot[126 + (t >> 7) * 126 + 3 * (2 * (c / 6) + (c & 1)) + (c % 6 >> 1)] = -nu * v;
-            }
-            if (t < 126) {
-                const int p = t / 3, c = t - 3 * p;
-                double v = 0.0;
-                for (int h = 0; h < 2; ++h)
-                    for (int q = 0; q < 3; ++q) v += S.fi[h][pt_row(p, q)][c];
-                slot[t] = nu * v;
-            }
-            if (ENERGY && t == 255) {
-                double v = 0.0;
-                for (int q = 0; q < 8; ++q) v += S.e[q];
-                slot[378] = -nu * v / 9.0;
-            }
+            write_slot(MODE == 0 ? slots : slots2, MODE == 0 && ENERGY);
             asm volatile("bar.sync 1, 256;" ::: "memory");
         }
     }
@@ -885,7 +1060,7 @@ __global__ void __launch_bounds__(256, 1)
 // launch that gave up gives NaN.
 template <int PART>
 __global__ void k_pt_reduce(int64_t p0, int64_t n, const PtSys *__restrict__ sys, int nsys, const double *__restrict__ slots, Out out,
-                            const unsigned int *__restrict__ err)
+                            bool more, const unsigned int *__restrict__ err)
 {
     const int64_t p = p0 + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
@@ -907,9 +1082,9 @@ __global__ void k_pt_reduce(int64_t p0, int64_t n, const PtSys *__restrict__ sys
     for (int c = 0; c < 3; ++c) f[c] = warp_sum(f[c]);
     if (lane == 0) {
         const double nan = __longlong_as_double(0x7ff8000000000000ll);
-        out.fx[p] = bad ? nan : (s.add ? out.fx[p] : 0.0) + f[0];
-        out.fy[p] = bad ? nan : (s.add ? out.fy[p] : 0.0) + f[1];
-        out.fz[p] = bad ? nan : (s.add ? out.fz[p] : 0.0) + f[2];
+        out.fx[p] = bad ? nan : (s.add || more ? out.fx[p] : 0.0) + f[0];
+        out.fy[p] = bad ? nan : (s.add || more ? out.fy[p] : 0.0) + f[1];
+        out.fz[p] = bad ? nan : (s.add || more ? out.fz[p] : 0.0) + f[2];
     }
 }
 
@@ -958,12 +1133,13 @@ static int pt_steps(int64_t k, bool fp64) { return fp64 ? (int)((k + P64_K - 1) 
 // a slab (what its product takes) and 14,000 an item, while the product pauses (geometry 5,800, contraction
 // 4,800, the rest sums over rows and set-up).  FP64: 3,072 cycles for 8 k, 6,000 an item.  512 at most, for the
 // accuracy of the mixed form's FP32 sums over a range, and for L2.
-static int pt_range(const int64_t *sys_off, int nsys, int sms, bool fp64)
+static int pt_range(const int64_t *sys_off, int nsys, int sms, bool fp64, int most)
 {
     const int units = fp64 ? sms : sms / 2;  // items in flight
-    int best = 512;
+    int best = most;
     double least = 0.0;
     for (int kp : {512, 384, 256, 192, 128, 96, 64, 32}) {
+        if (kp > most) continue;
         int64_t items = 0;
         double steps = 0.0;
         for (int s = 0; s < nsys; ++s) {
@@ -973,7 +1149,7 @@ static int pt_range(const int64_t *sys_off, int nsys, int sms, bool fp64)
         }
         const double t = (double)((items + units - 1) / units) *
                          (steps / (double)(items ? items : 1) * (fp64 ? 3072.0 : 1536.0) + (fp64 ? 6000.0 : 14000.0));
-        if (kp == 512 || t < 0.98 * least) {
+        if (kp == most || t < 0.98 * least) {
             least = t;
             best = kp;
         }
@@ -983,13 +1159,13 @@ static int pt_range(const int64_t *sys_off, int nsys, int sms, bool fp64)
 
 // Panels, tiles and results of all systems, in groups whose panel and results stay within `budget` bytes
 // (a group has at least one range); a system may go over several groups.
-void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, bool fp64, PtPlan &plan)
+void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, bool fp64, bool dual, PtPlan &plan)
 {
     static_assert(P64_BLOCK * sizeof(double) == PT_BLOCK_BYTES, "both forms' panels are planned alike");
     plan = PtPlan{};
     plan.fp64 = fp64;
     plan.slot_bytes = sizeof(double) * (size_t)(fp64 ? P64_SLOT : PT_SLOT);
-    const int kp = pt_range(sys_off, nsys, sms, fp64);
+    const int kp = pt_range(sys_off, nsys, sms, fp64, dual ? 256 : 512);  // G' sums a range twice
     PtGroup g{};
     for (int s = 0; s < nsys; ++s) {
         const int64_t n = sys_off[s + 1] - sys_off[s];
@@ -1038,7 +1214,7 @@ void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, bool fp64
 cudaError_t pt_init()
 {
     cudaError_t e;
-    for (auto k : {k_pt_gemm<false>, k_pt_gemm<true>})
+    for (auto k : {k_pt_gemm<0, false>, k_pt_gemm<0, true>, k_pt_gemm<1, false>, k_pt_gemm<1, true>, k_pt_gemm<2, false>})
         if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PtShared))) != cudaSuccess)
             return e;
     for (auto k : {k_p64_gemm<false>, k_p64_gemm<true>})
@@ -1047,7 +1223,7 @@ cudaError_t pt_init()
     return cudaSuccess;
 }
 
-cudaError_t launch_pairs(Pos pos, Out out, const PtPlan &plan, const PtDev &d, double *energy,
+cudaError_t launch_pairs(bool dual, Pos pos, Out out, const PtPlan &plan, const PtDev &d, double *energy,
                          double nu, int sms, cudaStream_t st, int *launches)
 {
     static_assert(sizeof(PtShared) <= 232448 && sizeof(P64Shared) <= 232448, "shared memory of one block");
@@ -1062,14 +1238,30 @@ cudaError_t launch_pairs(Pos pos, Out out, const PtPlan &plan, const PtDev &d, d
             auto gemm = energy ? k_p64_gemm<true> : k_p64_gemm<false>;
             gemm<<<(unsigned)std::min<int64_t>(g.items, sms), 256, sizeof(P64Shared), st>>>(
                 pos, seg, g.nsegs, g.items, d.tiles, (const double *)d.panel, d.slots, nu, d.err);
-            k_pt_reduce<P64_PART><<<reduce_blocks, 256, 0, st>>>(first.part0, np, sys, g.nsys, d.slots, out, d.err);
+            k_pt_reduce<P64_PART><<<reduce_blocks, 256, 0, st>>>(first.part0, np, sys, g.nsys, d.slots, out, false, d.err);
             if (energy) k_pt_energy<P64_PART><<<(unsigned)g.nsys, 512, 0, st>>>(sys, d.slots, energy);
         } else {
-            k_pt_panel<<<(unsigned)g.gen, PT_PANEL_THREADS, 0, st>>>(pos, seg, g.nsegs, d.panel);
-            auto gemm = energy ? k_pt_gemm<true> : k_pt_gemm<false>;
-            gemm<<<2 * (unsigned)std::min<int64_t>(g.items, sms / 2), PT_WARPS * 32, sizeof(PtShared), st>>>(
-                pos, seg, g.nsegs, g.items, d.tiles, d.panel, d.slots, nu, d.err);
-            k_pt_reduce<PT_PART><<<reduce_blocks, 256, 0, st>>>(first.part0, np, sys, g.nsys, d.slots, out, d.err);
+            const unsigned blocks = 2 * (unsigned)std::min<int64_t>(g.items, sms / 2);
+            auto gemm = [&](auto kern) {
+                kern<<<blocks, PT_WARPS * 32, sizeof(PtShared), st>>>(pos, seg, g.nsegs, g.items, d.tiles, d.panel, d.panel2,
+                                                                     d.slots, d.slots2, nu, d.err);
+            };
+            auto reduce = [&](const double *slots, Out to, bool more) {
+                k_pt_reduce<PT_PART><<<reduce_blocks, 256, 0, st>>>(first.part0, np, sys, g.nsys, slots, to, more, d.err);
+            };
+            k_pt_panel<false><<<(unsigned)g.gen, PT_PANEL_THREADS, 0, st>>>(pos, seg, g.nsegs, d.panel);
+            if (dual) {
+                const Out h{out.hx, out.hy, out.hz, nullptr, nullptr, nullptr};
+                k_pt_panel<true><<<(unsigned)g.gen, PT_PANEL_THREADS, 0, st>>>(pos, seg, g.nsegs, d.panel2);
+                gemm(energy ? k_pt_gemm<1, true> : k_pt_gemm<1, false>);
+                reduce(d.slots2, h, false);
+                gemm(k_pt_gemm<2, false>);
+                reduce(d.slots2, h, true);
+                *launches += 4;
+            } else {
+                gemm(energy ? k_pt_gemm<0, true> : k_pt_gemm<0, false>);
+            }
+            reduce(d.slots, out, false);
             if (energy) k_pt_energy<PT_PART><<<(unsigned)g.nsys, 512, 0, st>>>(sys, d.slots, energy);
         }
         *launches += energy ? 4 : 3;
