@@ -122,8 +122,9 @@ struct tbmd_ctx {
         std::vector<int64_t> off;
         PtPlan plan;
         PtDev dev{};
-        DevBuf tab, panel, slots, panel2, slots2;
+        DevBuf mem;  // tables, panels, tile results (one allocation: a context's first call waits for it)
     } pairs[2];
+    bool pairs_ready = false;  // pt_init has run
     int sms = 0;
 
     // P3BCA
@@ -363,8 +364,9 @@ static bool use_pairs(const tbmd_ctx *ctx, int64_t n, bool dual)
 }
 
 // Plan, tables and workspaces of the pair-tensor product for systems at offsets off[0 .. nsys].  The
-// panel and the tile results of one launch stay within 1 GB (one range of k where that takes more), twice
-// that for the adjoint.
+// panel and the tile results of one launch stay within 256 MB (mixed; n = 8192: 69 ms, 71 with 1 GB) or 1 GB
+// (FP64; n = 4001: 25.7 ms, 26.4 with 256 MB), or hold one range of k where that takes more; twice that
+// for the adjoint.
 static tbmd_status ensure_pairs(tbmd_ctx *ctx, const int64_t *off, int nsys, bool dual)
 {
     tbmd_ctx::PairState &s = ctx->pairs[dual ? 1 : 0];
@@ -373,26 +375,31 @@ static tbmd_status ensure_pairs(tbmd_ctx *ctx, const int64_t *off, int nsys, boo
     CK(ws_wait_host(ctx));  // a launch on a caller's stream may still read the old tables
     s.off.clear();
     if (!ctx->sms) CK(cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    CK(pt_init());
-    pt_plan(off, nsys, ctx->sms, (size_t)1 << 30, !mixed(ctx), dual, s.plan);
+    if (!ctx->pairs_ready) CK(pt_init());
+    ctx->pairs_ready = true;
+    pt_plan(off, nsys, ctx->sms, (size_t)1 << (mixed(ctx) ? 28 : 30), !mixed(ctx), dual, s.plan);
     const PtPlan &p = s.plan;
-    const size_t b_seg = sizeof(PtSeg) * p.segs.size(), b_sys = sizeof(PtSys) * p.sys.size(),
-                 b_til = sizeof(unsigned int) * p.tiles.size();
-    CK(s.tab.ensure(b_seg + b_sys + b_til));
-    CK(s.panel.ensure(p.mem));
-    CK(s.slots.ensure(p.slots * p.slot_bytes));
-    if (dual) {
-        CK(s.panel2.ensure(p.mem));
-        CK(s.slots2.ensure(p.slots * p.slot_bytes));
-    }
-    char *t = s.tab.as<char>();
-    CK(cudaMemcpyAsync(t, p.segs.data(), b_seg, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(t + b_seg, p.sys.data(), b_sys, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(t + b_seg + b_sys, p.tiles.data(), b_til, cudaMemcpyHostToDevice, ctx->stream));
+    size_t end = 0;
+    auto place = [&](size_t bytes) {
+        const size_t at = end;
+        end += (bytes + 255) / 256 * 256;
+        return at;
+    };
+    const size_t seg = place(sizeof(PtSeg) * p.segs.size()), sys = place(sizeof(PtSys) * p.sys.size()),
+                 til = place(sizeof(unsigned int) * p.tiles.size()), tables = end, panel = place(p.mem),
+                 slots = place(p.slots * p.slot_bytes), panel2 = dual ? place(p.mem) : panel,
+                 slots2 = dual ? place(p.slots * p.slot_bytes) : slots;
+    CK(s.mem.ensure(end));
+    std::vector<char> host(tables);
+    std::memcpy(host.data() + seg, p.segs.data(), sizeof(PtSeg) * p.segs.size());
+    std::memcpy(host.data() + sys, p.sys.data(), sizeof(PtSys) * p.sys.size());
+    std::memcpy(host.data() + til, p.tiles.data(), sizeof(unsigned int) * p.tiles.size());
+    char *t = s.mem.as<char>();
+    CK(cudaMemcpyAsync(t, host.data(), tables, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    s.dev = PtDev{(const PtSeg *)t, (const PtSys *)(t + b_seg), (const unsigned int *)(t + b_seg + b_sys),
-                  s.panel.as<unsigned char>(), s.slots.as<double>(), s.panel2.as<unsigned char>(), s.slots2.as<double>(),
-                  pairs_err(ctx)};
+    s.dev = PtDev{(const PtSeg *)(t + seg), (const PtSys *)(t + sys), (const unsigned int *)(t + til),
+                  (unsigned char *)(t + panel), (double *)(t + slots), (unsigned char *)(t + panel2),
+                  (double *)(t + slots2), pairs_err(ctx)};
     s.off.assign(off, off + nsys + 1);
     return TBMD_OK;
 }
@@ -854,9 +861,7 @@ void tbmd_destroy(tbmd_ctx *ctx)
     for (DevBuf *b : {&ctx->state, &ctx->snapshot, &ctx->scalars, &ctx->step_counts, &ctx->partial,
                       &ctx->cell_n, &ctx->cell_c, &ctx->nbr_buf, &ctx->dirs, &ctx->hvp, &ctx->gset_single,
                       &ctx->sweep[0].sys, &ctx->sweep[0].prefix, &ctx->sweep[1].sys, &ctx->sweep[1].prefix, &ctx->bpos, &ctx->bout, &ctx->bsys, &ctx->bprefix, &ctx->ncell_tab,
-                      &ctx->staging, &ctx->long_buf, &ctx->gen_buf, &ctx->bext, &ctx->pairs[0].tab, &ctx->pairs[0].panel,
-                      &ctx->pairs[0].slots, &ctx->pairs[1].tab, &ctx->pairs[1].panel, &ctx->pairs[1].slots,
-                      &ctx->pairs[1].panel2, &ctx->pairs[1].slots2})
+                      &ctx->staging, &ctx->long_buf, &ctx->gen_buf, &ctx->bext, &ctx->pairs[0].mem, &ctx->pairs[1].mem})
         b->release();
     if (ctx->hpin) cudaFreeHost(ctx->hpin);
     if (ctx->copy_stream) {
