@@ -205,6 +205,14 @@ def hbm_peak():
         return 6650.0, "fallback"
 
 
+def bf16_peak_tflops():
+    """(TFLOP/s, source): the sustained cuBLAS bf16 rate in MEASURED_PEAKS.json, else the fallback."""
+    try:
+        return float(json.loads((ROOT / "MEASURED_PEAKS.json").read_text())["bf16_tflops_sustained"]), "measured"
+    except (OSError, ValueError, KeyError):
+        return 1400.0, "fallback"
+
+
 def cell_build_roofline(phase, n):
     ms = phase["ms"] / max(phase["calls"], 1)
     peak, src = hbm_peak()
@@ -294,6 +302,12 @@ def run_ours(args, world, rank, local):
     fp64_peak = lib.tbmd_probe_fma_tflops(local, 1)
     peak = fp32_peak if args.precision == "mixed" else fp64_peak
     achieved = mean_trip * FLOP_PER_TRIPLET / (kern_ms * 1e-3) / 1e12
+    bound, peak_source = "fp32" if args.precision == "mixed" else "fp64", "tbmd_probe_fma_tflops"
+    pairs = w["cutoff"] <= 0 and 128 <= n <= 65536  # forces as a product of pair tensors
+    if pairs:  # the products' own operations over i < j: six bf16 splits of 27 n^3, or twelve FP64 sums of n^3
+        achieved = (162.0 if args.precision == "mixed" else 12.0) * n ** 3 / (kern_ms * 1e-3) / 1e12
+        if args.precision == "mixed":
+            bound, (peak, peak_source) = "bf16 tensor", bf16_peak_tflops()
     traffic = None
     tfile = ROOT / "profiles" / "traffic.json"
     if tfile.exists():
@@ -301,11 +315,15 @@ def run_ours(args, world, rank, local):
             traffic = json.loads(tfile.read_text()).get(f"{args.workload}:{args.precision}")
         except (ValueError, OSError):
             traffic = None
-    roofline = {"bound": "fp32" if args.precision == "mixed" else "fp64", "achieved": round(achieved, 3),
+    kernel = "k_p3bca" if w["algorithm"] == "p3bca" else f"k_{w['algorithm']}"
+    if pairs:
+        kernel = "k_pt_gemm" if args.precision == "mixed" else "k_p64_gemm"
+    roofline = {"bound": bound, "achieved": round(achieved, 3),
                 "peak": round(peak, 3), "unit": "TFLOP/s", "frac": round(achieved / peak, 4) if peak > 0 else None,
-                "traffic": traffic, "kernel": "k_p3bca" if w["algorithm"] == "p3bca" else f"k_{w['algorithm']}",
-                "kernel_ms": round(kern_ms, 5), "flop_per_triplet": FLOP_PER_TRIPLET,
-                "peak_source": "measured on this GPU by tbmd_probe_fma_tflops (FMA = 2 FLOP)",
+                "traffic": traffic, "kernel": kernel, "kernel_ms": round(kern_ms, 5),
+                "flop_per_triplet": None if pairs else FLOP_PER_TRIPLET,
+                "peak_source": "measured on this GPU by tbmd_probe_fma_tflops (FMA = 2 FLOP)"
+                if peak_source == "tbmd_probe_fma_tflops" else peak_source,
                 "phases_ms_per_step": {k: round(v["ms"] / max(v["calls"], 1), 5) for k, v in main["phases"].items()}}
     if w["algorithm"] == "p3bca" and w["cutoff"] > 0:
         roofline["cell_build"] = cell_build_roofline(main["phases"]["cells"], n)
