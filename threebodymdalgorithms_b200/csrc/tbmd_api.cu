@@ -354,7 +354,7 @@ static SweepWork single_sweep(tbmd_ctx *ctx, bool dual)
 // Whether the no-cutoff evaluation of a system (or the largest of a batch) goes through the pair-tensor
 // product (tbmd_pairs.cu) instead of a sweep: the forces of both precisions, and the mixed adjoint.  Forces:
 // at n = 128 both take the same time on the device (mixed 46 and 54 us, FP64 34 and 34), from there on the
-// product is faster (n = 1000: mixed 0.21 against 0.94 ms, 8192: 71 against 240 ms for AUTA and 541 for NATA;
+// product is faster (n = 1000: mixed 0.21 against 0.94 ms, 8192: 69 against 240 ms for AUTA and 541 for NATA;
 // FP64 213 against 385 and 1021).  Mixed adjoint: n = 130 177 against 133 us, 300 187 against 200, 2500 6.1
 // against 19.4 ms.  Above 65,536 the panel and tile results would pass 4 GB.
 constexpr int64_t kPairsMin = 128, kPairsMinAdjoint = 300, kPairsMax = 65536;

@@ -14,8 +14,8 @@
 //                same kernel
 //   k_pt_reduce  each particle's force from its tiles, in a fixed order (deterministic)
 //
-// Bound: the tensor cores, at the power cap for large n.  n = 8192: 9.4e13 FLOP of bf16 in 71 ms, 1.32
-// PFLOP/s of the 1.36 that cuBLAS sustains (AUTA's FP32 sweep took 240 ms, NATA's 541); n = 4096: 8.9 ms
+// Bound: the tensor cores, at the power cap for large n.  n = 8192: 9.4e13 FLOP of bf16 in 69 ms, 1.36
+// PFLOP/s, as much as cuBLAS sustains (AUTA's FP32 sweep took 240 ms, NATA's 541); n = 4096: 8.9 ms
 // (31.5 and 79).  A pair of SMs works on one tile of 256 x 256 (cta_group::2), which halves what each loads
 // of B: 48 KB a slab.  A block's 128 x 256 part is the largest whose FP32 sums fit the registers (128 a
 // thread in eight warps) beside two accumulators of 256 TMEM columns, one filling while the other is added
