@@ -290,7 +290,8 @@ __device__ __forceinline__ void split3(double v, unsigned short &h, unsigned sho
 
 // One block: a row block (42 particles) against 32 particles k (three slabs).  A thread holds one particle
 // i and 8 particles k: 24 columns of its three rows, three 16-byte chunks per row and split.  The stores
-// are 16-byte pieces that L2 merges; the panel is 0.4% of the product's time at n = 8192.
+// are 16-byte pieces that L2 merges: 70 us at n = 2048 (7% of the product's time; 2% at n = 8192).  Laying the
+// block's 72 KB out in shared memory and writing them with one bulk copy took 76.5 us.
 constexpr int PT_PANEL_THREADS = 192;
 template <bool TANGENT>
 __global__ void __launch_bounds__(PT_PANEL_THREADS) k_pt_panel(Pos pos, const PtSeg *__restrict__ seg, int nseg,
