@@ -131,3 +131,19 @@ def test_fits_that_do_not_wait(algo, precision, tol):
     for n, g, w in zip(sizes, got, want):
         for a, b in zip(g, w):
             assert float((a - b).detach().norm()) <= tol * max(float(b.detach().norm()), 1e-300), n
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+@pytest.mark.parametrize("n", [451, 577, 600, 801, 1025])
+def test_ranges_that_split_a_system_evenly(n, precision):
+    """Sizes whose ranges of k are an even split (160 to 416 particles) with a shorter last one; the tolerance
+    is that of the other ranges, as none is longer than 512."""
+    x, y, z = lattice(n, n)
+    ctx = Context("auta", precision, nu=1.3)
+    ctx.set_particles(x, y, z)
+    fx, fy, fz, e, c = ctx.forces()
+    ctx.close()
+    rx, ry, rz, rc = O.forces(x, y, z, 1.3, -1.0, nthreads=0)
+    assert c == rc
+    assert rel(np.stack([fx, fy, fz]), np.stack([rx, ry, rz])) <= TOL[precision]
+    assert abs(e - O.energy(x, y, z, 1.3, -1.0)) <= TOL[precision] * O.energy_abs(x, y, z, 1.3, -1.0)

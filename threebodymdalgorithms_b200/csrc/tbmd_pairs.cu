@@ -1130,27 +1130,57 @@ static int64_t pt_items(int64_t nb2, bool fp64) { return fp64 ? nb2 * (nb2 + 1) 
 // panel steps of a range of k: slabs of 32 columns (three per 32 particles), or 8 particles
 static int pt_steps(int64_t k, bool fp64) { return fp64 ? (int)((k + P64_K - 1) / P64_K) : (int)((k + 31) / 32 * 3); }
 
-// Particles k of one item: the range length with the least estimated time of all items.  Mixed: 1,536 cycles
-// a slab (what its product takes) and 14,000 an item, while the product pauses (geometry 5,800, contraction
-// 4,800, the rest sums over rows and set-up).  FP64: 3,072 cycles for 8 k, 6,000 an item.  512 at most, for the
-// accuracy of the mixed form's FP32 sums over a range, and for L2.
+// Time in cycles of a launch over ranges of kp particles: the most that one block is dealt (block b takes items
+// b, b + units, ... of all ranges in turn).  Mixed: 1,536 cycles a slab (what its product takes) and 14,000 an
+// item, while the product pauses (geometry 5,800, contraction 4,800, the rest sums over rows and set-up).  FP64:
+// 3,072 cycles for 8 k, 6,000 an item.  Above 32 items a block the average is as good and much cheaper.
+static double pt_cycles(const int64_t *sys_off, int nsys, int units, bool fp64, int kp)
+{
+    const double step = fp64 ? 3072.0 : 1536.0, item = fp64 ? 6000.0 : 14000.0;
+    int64_t items = 0;
+    double steps = 0.0;
+    for (int s = 0; s < nsys; ++s) {
+        const int64_t n = sys_off[s + 1] - sys_off[s], tiles = pt_items((n + pt_width(fp64) - 1) / pt_width(fp64), fp64);
+        items += tiles * ((n + kp - 1) / kp);
+        steps += (double)tiles * (double)pt_steps(n, fp64);
+    }
+    if (items > 32 * (int64_t)units)
+        return (double)((items + units - 1) / units) * (steps / (double)items * step + item);
+    std::vector<double> load((size_t)units, 0.0);
+    double every = 0.0;  // of the ranges' whole turns
+    int64_t at = 0;
+    for (int s = 0; s < nsys; ++s) {
+        const int64_t n = sys_off[s + 1] - sys_off[s], tiles = pt_items((n + pt_width(fp64) - 1) / pt_width(fp64), fp64);
+        for (int64_t k0 = 0; k0 < n; k0 += kp) {
+            const double t = pt_steps(std::min<int64_t>(kp, n - k0), fp64) * step + item;
+            every += (double)(tiles / units) * t;
+            for (int64_t q = 0; q < tiles % units; ++q) load[(size_t)((at + q) % units)] += t;
+            at = (at + tiles) % units;
+        }
+    }
+    return every + *std::max_element(load.begin(), load.end());
+}
+
+// Particles k of one item: the range length with the least time, of round lengths and of even splits of the
+// largest system, a longer one where it is within 2% (fewer results to store and add).  An estimate from the
+// average item does not see a short last range: it took 384 + 128 for n = 512 (all kernels of a call, FP64 121
+// us, with 256 + 256 93; mixed 77 and 67; n = 600: 177 and 156, 93 and 77.5).  512 at most, for the accuracy of
+// the mixed form's FP32 sums over a range, and for L2.
 static int pt_range(const int64_t *sys_off, int nsys, int sms, bool fp64, int most)
 {
-    const int units = fp64 ? sms : sms / 2;  // items in flight
-    int best = most;
+    const int units = std::max(1, fp64 ? sms : sms / 2);  // items in flight
+    int64_t nmax = 1;
+    for (int s = 0; s < nsys; ++s) nmax = std::max(nmax, sys_off[s + 1] - sys_off[s]);
+    std::vector<int> lengths{512, 384, 256, 192, 128, 96, 64, 32};
+    for (int64_t parts = 1; parts <= 8; ++parts)
+        lengths.push_back((int)std::min<int64_t>(most, ((nmax + parts - 1) / parts + 31) / 32 * 32));
+    std::sort(lengths.begin(), lengths.end(), [](int a, int b) { return a > b; });
+    int best = 0;
     double least = 0.0;
-    for (int kp : {512, 384, 256, 192, 128, 96, 64, 32}) {
-        if (kp > most) continue;
-        int64_t items = 0;
-        double steps = 0.0;
-        for (int s = 0; s < nsys; ++s) {
-            const int64_t n = sys_off[s + 1] - sys_off[s], nb2 = (n + pt_width(fp64) - 1) / pt_width(fp64);
-            items += pt_items(nb2, fp64) * ((n + kp - 1) / kp);
-            steps += (double)pt_items(nb2, fp64) * (double)pt_steps(n, fp64);
-        }
-        const double t = (double)((items + units - 1) / units) *
-                         (steps / (double)(items ? items : 1) * (fp64 ? 3072.0 : 1536.0) + (fp64 ? 6000.0 : 14000.0));
-        if (kp == most || t < 0.98 * least) {
+    for (int kp : lengths) {
+        if (kp > most || kp == best) continue;
+        const double t = pt_cycles(sys_off, nsys, units, fp64, kp);
+        if (!best || t < 0.98 * least) {
             least = t;
             best = kp;
         }
