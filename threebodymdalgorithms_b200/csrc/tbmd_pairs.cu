@@ -26,8 +26,8 @@
 // exact in FP32.  The tensor core adds into an FP32 accumulator that it truncates, so an accumulator only
 // lives for 32 columns of T: the ten small products go first, the two hh steps last, and the tile is then
 // added to FP32 registers with rounding.  After 512 particles at most the registers are contracted and the
-// forces go on in FP64.  Relative L2 error of the forces against FP64, thermal lattices of 512 .. 8192
-// particles: 1.5e-7 .. 2.3e-7 (the FP32 sweeps: 2.3e-7 .. 2.6e-7).  No step subtracts nearly equal
+// forces go on in FP64.  Relative L2 error of the forces against FP64, thermal lattices of 130 .. 8000
+// particles: 1.3e-7 .. 2.1e-7 (the FP32 sweeps: 2.2e-7 .. 2.4e-7 to 4000).  No step subtracts nearly equal
 // numbers: a pair's force needs no difference of large terms even where two of the three particles nearly
 // coincide.
 #include <cuda_bf16.h>
@@ -1254,10 +1254,17 @@ cudaError_t pt_init()
     return cudaSuccess;
 }
 
+// What the tensor core's truncation takes off a product on average.  A truncation loses half an ulp, which is
+// 2^-24 / (2 ln 2) = 4.3e-8 of a value with a log-uniform mantissa; a slab's sum is truncated twice at full size, by
+// the two hh steps, of which the first holds half of it.  The results' scale makes up for it.  Energies of thermal
+// lattices, 130 .. 4000 particles: -6.5e-8 .. -7.5e-8 in every one without (the FP32 sweeps: -2e-8 .. -5e-8).
+constexpr double PT_TRUNCATED = 1.5 * 5.9604644775390625e-08 * 0.72134752044448170;
+
 cudaError_t launch_pairs(bool dual, Pos pos, Out out, const PtPlan &plan, const PtDev &d, double *energy,
                          double nu, int sms, cudaStream_t st, int *launches)
 {
     static_assert(sizeof(PtShared) <= 232448 && sizeof(P64Shared) <= 232448, "shared memory of one block");
+    if (!plan.fp64) nu *= 1.0 + PT_TRUNCATED;
     for (const PtGroup &g : plan.groups) {
         const PtSeg *seg = d.segs + g.seg0;
         const PtSys *sys = d.sys + g.sys0;
