@@ -81,15 +81,26 @@ __device__ __forceinline__ void bar_expect(unsigned long long *b, unsigned int b
 {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
 }
-// arrive on the same barrier of block `rank` of the cluster.  Nothing is handed over in memory (a release at
-// cluster scope would wait for the thread's global stores, 1,000 cycles a slab): what the arrivals order is
-// TMEM reads (tcgen05.fence) and bulk copies that have signalled their own barrier.
-__device__ __forceinline__ void bar_arrive_at(unsigned long long *b, unsigned int rank)
+// Arrive on the same barrier of block `rank` of the cluster, after reads of TMEM (ordered by tcgen05.fence).
+// Nothing is handed over in memory, so the arrival is relaxed: a release at cluster scope waits for the
+// thread's global stores, 1,000 cycles a slab in the warps that write the tiles' results.
+__device__ __forceinline__ void bar_arrive_tmem(unsigned long long *b, unsigned int rank)
 {
     asm volatile(
         "{\n\t.reg .b32 a;\n\t"
         "mapa.shared::cluster.u32 a, %0, %1;\n\t"
         "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [a];\n\t}" ::"r"(smem_u32(b)),
+        "r"(rank)
+        : "memory");
+}
+// The same for a thread that has seen a bulk copy of its own block complete and passes that on: what the copy
+// wrote is ordered before the arrival, for a wait with bar_try_cluster.
+__device__ __forceinline__ void bar_relay_copy(unsigned long long *b, unsigned int rank)
+{
+    asm volatile(
+        "{\n\t.reg .b32 a;\n\t"
+        "mapa.shared::cluster.u32 a, %0, %1;\n\t"
+        "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [a];\n\t}" ::"r"(smem_u32(b)),
         "r"(rank)
         : "memory");
 }
@@ -109,15 +120,29 @@ __device__ __forceinline__ bool bar_try(unsigned long long *b, unsigned int pari
         : "memory");
     return ok != 0;
 }
+// for a phase that the other block's arrivals complete: acquires what they released
+__device__ __forceinline__ bool bar_try_cluster(unsigned long long *b, unsigned int parity)
+{
+    unsigned int ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(b)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 // Every wait ends: after four billion cycles (two seconds or more) it marks the block dead and the launch failed (*err); from then on
 // waits return at once, no copy or product is issued, and the loops run out.
-template <class Shared>
+template <bool CLUSTER = false, class Shared>
 __device__ __forceinline__ bool bar_wait(unsigned long long *b, unsigned int parity, Shared &S, unsigned int *err)
 {
-    if (bar_try(b, parity)) return true;
+    auto done = [&]() { return CLUSTER ? bar_try_cluster(b, parity) : bar_try(b, parity); };
+    if (done()) return true;
     const long long t0 = clock64();
     for (unsigned int n = 1;; ++n) {
-        if (bar_try(b, parity)) return true;
+        if (done()) return true;
         if ((n & 63u) == 0u) {
             if (*(volatile int *)&S.dead) return false;
             if (clock64() - t0 > 4000000000ll) {
@@ -501,7 +526,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
                 const PtItem it = pt_item(seg, nseg, tiles, w);
                 for (int k = 0; k < slabs_of(it); ++k, ++n) {
                     if (!bar_wait(&S.full[n % PT_STAGES], (n / PT_STAGES) & 1, S, err)) break;
-                    bar_arrive_at(&S.full[n % PT_STAGES], 0);
+                    bar_relay_copy(&S.full[n % PT_STAGES], 0);
                 }
                 if (*(volatile int *)&S.dead) break;
             }
@@ -514,7 +539,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
                 for (int k = 0; k < slabs_of(it); ++k, ++n) {
                     const int st = n % PT_STAGES, buf = n & 1;
                     ok = bar_wait(&S.acc_empty[buf], ((n >> 1) & 1) ^ 1, S, err) &&
-                         bar_wait(&S.full[st], (n / PT_STAGES) & 1, S, err);
+                         bar_wait<true>(&S.full[st], (n / PT_STAGES) & 1, S, err);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const unsigned int A = smem_u32(S.stage[st]), B = A + PT_BLOCK_BYTES, D = tmem + buf * 256;
@@ -587,7 +612,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
                     TM_WAIT64(t);
                     if (c == 1) {  // the accumulator is in registers: free for the next but one slab
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                        if (lane == 0) bar_arrive_at(&S.acc_empty[buf], 0);
+                        if (lane == 0) bar_arrive_tmem(&S.acc_empty[buf], 0);
                     }
 #pragma unroll
                     for (int q = 0; q < 32; ++q) g2[c * 32 + q] = add2(g2[c * 32 + q], pack2(t[2 * q], t[2 * q + 1]));
