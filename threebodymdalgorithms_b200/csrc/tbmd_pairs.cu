@@ -878,11 +878,40 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
 //
 // Bound: the FP64 rate, which the matrix instruction reaches with few warps (36.9 TFLOP/s with 8 on an SM) and
 // few shared-memory reads (half the wavefront slots): 192 registers of sums leave one block of 8 warps an SM.
+// n = 4001: 27.2 ms, 31 TFLOP/s of products (25.7 with sums over 512 k and T in plain operations, 2.6 times the
+// error).
+//
+// Accuracy.  The sums are folded into a second set after every 64 k, which waits in TMEM (the block uses no other
+// and has no registers left); T and the contraction use powers of r with their rounding errors carried along.
+// Relative L2 error of the forces against 80-bit arithmetic, lattices and uniform inputs of 300 .. 4001 particles:
+// 3.1e-16 .. 5.3e-16, where plain FP64 sums over triplets have 4.4e-16 .. 6.4e-16 (NATA's) and 8.5e-16 .. 1.4e-14
+// (AUTA's).  With sums over 512 k, and T in plain operations, 7.3e-16 .. 1.2e-15.
+//
 // Plain FMA on 2 x 4 pairs a thread, with three 16-byte reads for 8 FMA, reached 0.41 of the rate (n = 8192:
 // 477 ms).
 constexpr int P64_PART = 32, P64_K = 8, P64_F = 12, P64_STAGES = 3;
+constexpr int P64_CHUNK = 8;  // panel steps (64 k) of the matrix instruction's sums before they are folded
 constexpr int P64_BLOCK = P64_K * P64_F * P64_PART;  // doubles of one row block and 8 k: 24 KB
 constexpr int P64_SLOT = pt_slot(P64_PART);
+
+// 1 / r^2 and 1 / r^5 to about one rounding, and r^2: rsqrt with the rounding errors of r^2 and of the powers
+// carried along to first order.  In plain operations the power's error alone is 4e-16.
+struct P64Radius {
+    double r2, i2, i5;
+};
+__device__ __forceinline__ P64Radius p64_radius(double x, double y, double z)
+{
+    const double px = x * x, py = y * y, pz = z * z;
+    const double s = py + pz, t = s - py, es = (py - (s - t)) + (pz - t);
+    const double r2 = px + s, v = r2 - px, er = (px - (r2 - v)) + (s - v);
+    // what r^2 lacks
+    const double lo = (er + es) + (fma(x, x, -px) + (fma(y, y, -py) + fma(z, z, -pz)));
+    const double h = rsqrt(r2), p = r2 * h;
+    const double l = 0.5 * h * (fma(-p, h, 1.0) - fma(fma(r2, h, -p), h, lo * h * h));  // 1 / r = h + l
+    const double h2 = h * h, e2 = fma(h, h, -h2), h4 = h2 * h2, h5 = h4 * h;
+    const double c5 = fma(5.0 * h4, l, fma(h, fma(2.0 * h2, e2, fma(h2, h2, -h4)), fma(h4, h, -h5)));
+    return P64Radius{r2, h2 + fma(2.0 * h, l, e2), h5 + c5};
+}
 
 struct P64Shared {
     // row block i, two blocks j: [four k][pair of features][8 particles][particle, k][feature], so that the 32
@@ -890,6 +919,8 @@ struct P64Shared {
     double stage[P64_STAGES][3][P64_BLOCK];
     double fi[4][P64_PART][3], fj[2][2 * P64_PART][3], e[8];
     unsigned long long full[P64_STAGES];
+    PtItem item;  // in shared memory, since the sums leave few registers
+    unsigned int tmem;
     int dead;
 };
 
@@ -904,14 +935,13 @@ __global__ void __launch_bounds__(P64_K * P64_PART) k_p64_panel(Pos pos, const P
     if (i < s.n && k < s.n && i != k) {
         const double x = pos.x[s.part0 + k] - pos.x[s.part0 + i], y = pos.y[s.part0 + k] - pos.y[s.part0 + i],
                      z = pos.z[s.part0 + k] - pos.z[s.part0 + i];
-        const double ri = rsqrt(fma(x, x, fma(y, y, z * z)));
-        const double ri2 = ri * ri, i3 = ri * ri2, s5 = 3.0 * i3 * ri2;
-        xx = fma(s5 * x, x, -i3);
-        xy = s5 * x * y;
-        xz = s5 * x * z;
-        yy = fma(s5 * y, y, -i3);
-        yz = s5 * y * z;
-        zz = fma(s5 * z, z, -i3);
+        const double i5 = p64_radius(x, y, z).i5, s5 = 3.0 * i5;
+        xx = i5 * fma(2.0 * x, x, -fma(y, y, z * z));
+        xy = s5 * (x * y);
+        xz = s5 * (x * z);
+        yy = i5 * fma(2.0 * y, y, -fma(x, x, z * z));
+        yz = s5 * (y * z);
+        zz = i5 * fma(2.0 * z, z, -fma(x, x, y * y));
     }
     double *dst = panel + s.mem / 8 + ((int64_t)rb * s.nslab + kc) * P64_BLOCK +
                   ((kl >> 2) * (P64_F / 2) * 4 + (il >> 3)) * 64 + ((il & 7) * 4 + (kl & 3)) * 2;
@@ -929,6 +959,39 @@ __device__ __forceinline__ void mma_f64(double &d0, double &d1, double a, double
         : "d"(a), "d"(b));
 }
 
+// twelve doubles of each lane in 24 columns of TMEM
+__device__ __forceinline__ void tm_load12(double *v, unsigned int addr)
+{
+    int w[24];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%24];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16,%17,%18,%19,%20,%21,%22,%23}, [%25];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]), "=r"(w[8]),
+          "=r"(w[9]), "=r"(w[10]), "=r"(w[11]), "=r"(w[12]), "=r"(w[13]), "=r"(w[14]), "=r"(w[15]), "=r"(w[16]),
+          "=r"(w[17]), "=r"(w[18]), "=r"(w[19]), "=r"(w[20]), "=r"(w[21]), "=r"(w[22]), "=r"(w[23])
+        : "r"(addr), "r"(addr + 16)
+        : "memory");
+#pragma unroll
+    for (int q = 0; q < 12; ++q) v[q] = __hiloint2double(w[2 * q + 1], w[2 * q]);
+}
+__device__ __forceinline__ void tm_store12(const double *v, unsigned int addr)
+{
+    int w[24];
+#pragma unroll
+    for (int q = 0; q < 12; ++q) {
+        w[2 * q] = __double2loint(v[q]);
+        w[2 * q + 1] = __double2hiint(v[q]);
+    }
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%24], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};\n\t"
+        "tcgen05.st.sync.aligned.32x32b.x8.b32 [%25], {%16,%17,%18,%19,%20,%21,%22,%23};" ::"r"(w[0]),
+        "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "r"(w[8]), "r"(w[9]), "r"(w[10]),
+        "r"(w[11]), "r"(w[12]), "r"(w[13]), "r"(w[14]), "r"(w[15]), "r"(w[16]), "r"(w[17]), "r"(w[18]), "r"(w[19]),
+        "r"(w[20]), "r"(w[21]), "r"(w[22]), "r"(w[23]), "r"(addr), "r"(addr + 16)
+        : "memory");
+}
+
 template <bool ENERGY>
 __global__ void __launch_bounds__(256, 1)
     k_p64_gemm(Pos pos, const PtSeg *__restrict__ seg, int nseg, int64_t items, const unsigned int *__restrict__ tiles,
@@ -943,110 +1006,141 @@ __global__ void __launch_bounds__(256, 1)
         S.dead = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&S.tmem))
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // this warp's part of TMEM: its 32 lanes, half of the columns
+    const unsigned int tmem = S.tmem + ((unsigned int)((warp & 3) * 32) << 16) + (warp >> 2) * 256;
     // thread 0 loads, two steps of 8 k ahead of the products and across items
-    int64_t lw = blockIdx.x;  // item and step that is loaded next
-    int lk = 0;
+    int64_t lw = blockIdx.x;  // item that is loaded next, its steps left, its blocks i and j
+    int left = 0, nslab = 0, oj = 0;
     unsigned int ln = 0;
-    PtItem lit{};
-    auto load = [&]() {
-        if (lw >= items || *(volatile int *)&S.dead) return;
-        if (lk == 0) lit = pt_item(seg, nseg, tiles, lw);
-        const int st = ln % P64_STAGES;
-        const double *src = panel + lit.s.mem / 8 + (int64_t)lk * P64_BLOCK;
-        const int64_t row = (int64_t)lit.s.nslab * P64_BLOCK;
-        bar_expect(&S.full[st], 3 * P64_BLOCK * 8);
-        bulk_load(S.stage[st][0], src + lit.a * row, P64_BLOCK * 8, &S.full[st]);
-        bulk_load(S.stage[st][1], src + 2 * lit.b * row, P64_BLOCK * 8, &S.full[st]);
-        bulk_load(S.stage[st][2], src + (2 * lit.b + 1) * row, P64_BLOCK * 8, &S.full[st]);
-        ++ln;
-        if (++lk == lit.s.nslab) {
-            lk = 0;
+    const double *src = nullptr;
+    auto load = [&](unsigned int st) {
+        if (left == 0) {
+            if (lw >= items) return;
+            const PtItem q = pt_item(seg, nseg, tiles, lw);
+            left = nslab = q.s.nslab;
+            src = panel + q.s.mem / 8 + (int64_t)q.a * nslab * P64_BLOCK;
+            oj = (2 * q.b - q.a) * nslab;
             lw += gridDim.x;
         }
+        if (*(volatile int *)&S.dead) return;
+        bar_expect(&S.full[st], 3 * P64_BLOCK * 8);
+        bulk_load(S.stage[st][0], src, P64_BLOCK * 8, &S.full[st]);
+        bulk_load(S.stage[st][1], src + (int64_t)oj * P64_BLOCK, P64_BLOCK * 8, &S.full[st]);
+        bulk_load(S.stage[st][2], src + (int64_t)(oj + nslab) * P64_BLOCK, P64_BLOCK * 8, &S.full[st]);
+        ++ln;
+        src += P64_BLOCK;
+        --left;
     };
     if (threadIdx.x == 0)
-        for (int k = 0; k < P64_STAGES; ++k) load();
+        for (unsigned int k = 0; k < P64_STAGES; ++k) load(k);
     unsigned int n = 0;
     for (int64_t w = blockIdx.x; w < items; w += gridDim.x) {
-        const PtItem it = pt_item(seg, nseg, tiles, w);
-        double acc[P64_F][2][4];
+        if (threadIdx.x == 0) S.item = pt_item(seg, nseg, tiles, w);
+        __syncthreads();
+        const PtItem &it = S.item;
+        const int steps = it.s.nslab;
+        for (int k0 = 0; k0 < steps; k0 += P64_CHUNK) {
+            double acc[P64_F][2][4];
 #pragma unroll
-        for (int m = 0; m < P64_F; ++m)
+            for (int m = 0; m < P64_F; ++m)
 #pragma unroll
-            for (int q = 0; q < 8; ++q) acc[m][q >> 2][q & 3] = 0.0;
-        for (int kc = 0; kc < it.s.nslab; ++kc, ++n) {
-            const int st = n % P64_STAGES;
-            bar_wait(&S.full[st], (n / P64_STAGES) & 1, S, err);
-            const double2 *I = (const double2 *)S.stage[st][0] + iw * 64 + lane,
-                          *J = (const double2 *)S.stage[st][1 + (jw >> 1)] + (jw & 1) * 64 + lane;
+                for (int q = 0; q < 8; ++q) acc[m][q >> 2][q & 3] = 0.0;
+            const int k1 = min(k0 + P64_CHUNK, steps);
+            for (int kc = k0; kc < k1; ++kc, ++n) {
+                const unsigned int st = n % P64_STAGES;
+                bar_wait(&S.full[st], (n / P64_STAGES) & 1, S, err);
+                const double2 *I = (const double2 *)S.stage[st][0] + iw * 64 + lane,
+                              *J = (const double2 *)S.stage[st][1 + (jw >> 1)] + (jw & 1) * 64 + lane;
 #pragma unroll 1
-            for (int k = 0; k < P64_K / 4; ++k) {
+                for (int k = 0; k < P64_K / 4; ++k) {
 #pragma unroll
-                for (int m = 0; m < P64_F / 2; ++m) {
-                    const int o = (k * (P64_F / 2) + m) * 128;
-                    const double2 a[2] = {I[o], I[o + 32]}, b[2] = {J[o], J[o + 32]};
+                    for (int m = 0; m < P64_F / 2; ++m) {
+                        const int o = (k * (P64_F / 2) + m) * 128;
+                        const double2 a[2] = {I[o], I[o + 32]}, b[2] = {J[o], J[o + 32]};
 #pragma unroll
-                    for (int u = 0; u < 2; ++u)
+                        for (int u = 0; u < 2; ++u)
 #pragma unroll
-                        for (int v = 0; v < 2; ++v) {
-                            mma_f64(acc[2 * m][u][2 * v], acc[2 * m][u][2 * v + 1], a[u].x, b[v].x);
-                            mma_f64(acc[2 * m + 1][u][2 * v], acc[2 * m + 1][u][2 * v + 1], a[u].y, b[v].y);
-                        }
+                            for (int v = 0; v < 2; ++v) {
+                                mma_f64(acc[2 * m][u][2 * v], acc[2 * m][u][2 * v + 1], a[u].x, b[v].x);
+                                mma_f64(acc[2 * m + 1][u][2 * v], acc[2 * m + 1][u][2 * v + 1], a[u].y, b[v].y);
+                            }
+                    }
                 }
+                __syncthreads();  // the stage has been read
+                if (threadIdx.x == 0) load(st);
             }
-            __syncthreads();  // the stage has been read
-            if (threadIdx.x == 0) load();
+            __syncwarp();
+            // added to the earlier chunks' sums in TMEM, where the contraction finds them a pair at a time
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                double v[P64_F], old[P64_F] = {};
+                if (k0) tm_load12(old, tmem + 2 * P64_F * q);
+#pragma unroll
+                for (int m = 0; m < P64_F; ++m) v[m] = acc[m][q >> 2][q & 3] + old[m];
+                tm_store12(v, tmem + 2 * P64_F * q);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         }
-        // contraction of G with dT/dr: with n = r / |r|, q = n.G n
-        //   f_i += nu / r^4 (2 G n + (tr G - 5 q) n),  E -= nu / (9 r^3) (3 q - tr G)
+        // contraction of G with dT/dr: with h = 2 G r, q = r.h / 2
+        //   f_i += nu / r^5 (h + (tr G - 5 q / r^2) r),  E -= nu / (9 r^3) (3 q / r^2 - tr G)
         const int64_t P = it.s.part0;
         const int ia = it.a * P64_PART + iw * 16 + li, jb = 2 * it.b * P64_PART + jw * 16 + lj * 2;
-        double fi[2][3] = {}, fj[4][3] = {}, en = 0.0;
+        double fi[2][3] = {}, en = 0.0;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int u = q >> 2, v = q & 3, i = ia + u * 8, j = jb + (v >> 1) * 8 + (v & 1);
-            if (i < j && j < it.s.n) {
-                const double x = pos.x[P + j] - pos.x[P + i], y = pos.y[P + j] - pos.y[P + i],
-                             z = pos.z[P + j] - pos.z[P + i];
-                const double ri = rsqrt(fma(x, x, fma(y, y, z * z))), ri2 = ri * ri;
-                const double nx = x * ri, ny = y * ri, nz = z * ri;
-                const double dx = acc[0][u][v], dy = acc[1][u][v], dz = acc[2][u][v], sxy = acc[3][u][v], sxz = acc[4][u][v],
-                             syz = acc[5][u][v];
-                const double gxx = dx + sxy + sxz, gyy = dy + sxy + syz, gzz = dz + sxz + syz;
-                // twice the off-diagonal entries
-                const double gxy = (acc[7][u][v] - sxz - syz) - (acc[6][u][v] - sxy - dz);
-                const double gxz = (acc[9][u][v] - sxy - syz) - (acc[8][u][v] - sxz - dy);
-                const double gyz = (acc[11][u][v] - sxy - sxz) - (acc[10][u][v] - syz - dx);
-                const double hx = 2.0 * gxx * nx + gxy * ny + gxz * nz, hy = gxy * nx + 2.0 * gyy * ny + gyz * nz,
-                             hz = gxz * nx + gyz * ny + 2.0 * gzz * nz;
-                const double tr = gxx + gyy + gzz, qq = 0.5 * (hx * nx + hy * ny + hz * nz);
-                const double c = nu * ri2 * ri2, d = tr - 5.0 * qq;
-                const double vx = c * (hx + d * nx), vy = c * (hy + d * ny), vz = c * (hz + d * nz);
-                fi[u][0] += vx;
-                fi[u][1] += vy;
-                fi[u][2] += vz;
-                fj[v][0] -= vx;
-                fj[v][1] -= vy;
-                fj[v][2] -= vz;
-                if (ENERGY) en -= nu * ri * ri2 * (3.0 * qq - tr) / 9.0;
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
+        for (int v = 0; v < 4; ++v) {
+            const int j = jb + (v >> 1) * 8 + (v & 1);
+            double fj[3] = {};
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
-                double v = fi[u][c];
-                for (int o = 1; o < 4; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                if (lj == 0) S.fi[jw][iw * 16 + li + u * 8][c] = v;
+                const int i = ia + u * 8;
+                double g[P64_F];
+                tm_load12(g, tmem + 2 * P64_F * (4 * u + v));
+                if (i < j && j < it.s.n) {
+                    const double x = pos.x[P + j] - pos.x[P + i], y = pos.y[P + j] - pos.y[P + i],
+                                 z = pos.z[P + j] - pos.z[P + i];
+                    const P64Radius r = p64_radius(x, y, z);
+                    const double dx = g[0], dy = g[1], dz = g[2], sxy = g[3], sxz = g[4], syz = g[5];
+                    const double gxx = dx + sxy + sxz, gyy = dy + sxy + syz, gzz = dz + sxz + syz;
+                    // twice the off-diagonal entries
+                    const double gxy = (g[7] - sxz - syz) - (g[6] - sxy - dz);
+                    const double gxz = (g[9] - sxy - syz) - (g[8] - sxz - dy);
+                    const double gyz = (g[11] - sxy - sxz) - (g[10] - syz - dx);
+                    const double hx = fma(2.0 * gxx, x, fma(gxy, y, gxz * z)), hy = fma(gxy, x, fma(2.0 * gyy, y, gyz * z)),
+                                 hz = fma(gxz, x, fma(gyz, y, 2.0 * gzz * z));
+                    const double tr = gxx + gyy + gzz, qq = 0.5 * fma(hx, x, fma(hy, y, hz * z));
+                    const double c = nu * r.i5, d = fma(-5.0 * qq, r.i2, tr);
+                    const double vx = c * fma(d, x, hx), vy = c * fma(d, y, hy), vz = c * fma(d, z, hz);
+                    fi[u][0] += vx;
+                    fi[u][1] += vy;
+                    fi[u][2] += vz;
+                    fj[0] -= vx;
+                    fj[1] -= vy;
+                    fj[2] -= vz;
+                    if (ENERGY) en -= c * r.r2 * fma(3.0 * qq, r.i2, -tr);
+                }
+                __syncwarp();
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                double v = fj[u][c];
-                for (int o = 4; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                if (li == 0) S.fj[iw][jw * 16 + lj * 2 + (u >> 1) * 8 + (u & 1)][c] = v;
+            for (int c = 0; c < 3; ++c) {
+                for (int o = 4; o < 32; o <<= 1) fj[c] += __shfl_xor_sync(0xffffffffu, fj[c], o);
+                if (li == 0) S.fj[iw][jw * 16 + lj * 2 + (v >> 1) * 8 + (v & 1)][c] = fj[c];
             }
         }
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                for (int o = 1; o < 4; o <<= 1) fi[u][c] += __shfl_xor_sync(0xffffffffu, fi[u][c], o);
+                if (lj == 0) S.fi[jw][iw * 16 + li + u * 8][c] = fi[u][c];
+            }
         if (ENERGY) {
             en = warp_sum(en);
             if (lane == 0) S.e[warp] = en;
@@ -1067,7 +1161,7 @@ __global__ void __launch_bounds__(256, 1)
         if (ENERGY && threadIdx.x == 0) {
             double v = S.e[0];
             for (int q = 1; q < 8; ++q) v += S.e[q];
-            slot[9 * P64_PART] = v;
+            slot[9 * P64_PART] = v / 9.0;
         }
         __syncthreads();
     }
@@ -1078,6 +1172,9 @@ __global__ void __launch_bounds__(256, 1)
             while (!bar_try(&S.full[k % P64_STAGES], (k / P64_STAGES) & 1) && clock64() - t0 < 200000000ll) {
             }
         }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(S.tmem));
 }
 
 // Forces from the tiles' results: particle i of row block a sums the tiles (a, b) of its row and the tiles
@@ -1158,10 +1255,10 @@ static int pt_steps(int64_t k, bool fp64) { return fp64 ? (int)((k + P64_K - 1) 
 // Time in cycles of a launch over ranges of kp particles: the most that one block is dealt (block b takes items
 // b, b + units, ... of all ranges in turn).  Mixed: 1,536 cycles a slab (what its product takes) and 14,000 an
 // item, while the product pauses (geometry 5,800, contraction 4,800, the rest sums over rows and set-up).  FP64:
-// 3,072 cycles for 8 k, 6,000 an item.  Above 32 items a block the average is as good and much cheaper.
+// 3,200 cycles for 8 k (3,072 of products), 9,000 an item.  Above 32 items a block the average is as good and much cheaper.
 static double pt_cycles(const int64_t *sys_off, int nsys, int units, bool fp64, int kp)
 {
-    const double step = fp64 ? 3072.0 : 1536.0, item = fp64 ? 6000.0 : 14000.0;
+    const double step = fp64 ? 3200.0 : 1536.0, item = fp64 ? 9000.0 : 14000.0;
     int64_t items = 0;
     double steps = 0.0;
     for (int s = 0; s < nsys; ++s) {
