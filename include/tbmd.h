@@ -39,8 +39,9 @@ typedef enum {
     TBMD_NOT_READY = 3,       /* no particles set */
     TBMD_CAPACITY_RETRY = 4,  /* neighbour capacity still too small after the automatic retries */
     TBMD_CUDA_ERROR = 5,      /* a CUDA runtime call failed; see tbmd_last_error */
-    TBMD_TIMEOUT = 6,         /* a wait inside the pair-tensor kernel (mixed precision, no cutoff) ran out; the
-                                 forces are NaN.  No kernel waits on another kernel. */
+    TBMD_TIMEOUT = 6,         /* a wait inside a pair-tensor kernel (no cutoff, both precisions) ran out; forces,
+                                 gradients and energy are NaN (the *_device calls, which do not wait, only give
+                                 the NaN).  No kernel waits on another kernel. */
     TBMD_NO_DEVICE = 7,       /* no CUDA device, or not an sm_100 device */
     TBMD_TOO_LARGE = 8,       /* n above the limit of an allocation-free entry point */
     TBMD_RANK_LAYOUT = 9      /* the reference's run on that many MPI ranks would stop (tbmd_rank_layout_of) */

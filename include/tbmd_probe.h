@@ -4,11 +4,15 @@
  * The roofline of the triplet kernels is the FP32 pipe (mixed precision) or the FP64 pipe (FP64
  * drop-in), not a tensor core or HBM figure, so the benchmark measures those pipe peaks on the
  * device it runs on with a dependent-chain-free FMA loop.
+ *
+ * And a handle for tests on a limit that no run reaches.
  */
 #ifndef TBMD_PROBE_H
 #define TBMD_PROBE_H
 
 #include <stdint.h>
+
+#include "tbmd.h"
 
 #ifdef __cplusplus
 extern "C" {
@@ -18,6 +22,10 @@ extern "C" {
  * pipe, 1 for the FP64 pipe.  Runs about 0.1-0.3 s; returns a negative value on a CUDA error.  The
  * calling thread's current device is the same afterwards. */
 double tbmd_probe_fma_tflops(int32_t device, int32_t fp64);
+
+/* Waits inside the pair-tensor kernels (no cutoff) of this context give up after `cycles` clock cycles (4e9 in a
+ * new context); with 0 the first one does, and the evaluation ends with TBMD_TIMEOUT. */
+tbmd_status tbmd_probe_pair_waits(tbmd_ctx *ctx, int64_t cycles);
 
 #ifdef __cplusplus
 }

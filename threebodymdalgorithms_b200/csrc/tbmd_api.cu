@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "../../include/tbmd.h"
+#include "../../include/tbmd_probe.h"
 #include "tbmd_internal.cuh"
 
 using namespace tbmd;
@@ -125,6 +126,7 @@ struct tbmd_ctx {
         DevBuf mem;  // tables, panels, tile results (one allocation: a context's first call waits for it)
     } pairs[2];
     bool pairs_ready = false;  // pt_init has run
+    long long pairs_wait = PT_WAIT_LIMIT;
     int sms = 0;
 
     // P3BCA
@@ -399,7 +401,7 @@ static tbmd_status ensure_pairs(tbmd_ctx *ctx, const int64_t *off, int nsys, boo
     CK(cudaStreamSynchronize(ctx->stream));
     s.dev = PtDev{(const PtSeg *)(t + seg), (const PtSys *)(t + sys), (const unsigned int *)(t + til),
                   (unsigned char *)(t + panel), (double *)(t + slots), (unsigned char *)(t + panel2),
-                  (double *)(t + slots2), pairs_err(ctx)};
+                  (double *)(t + slots2), PtWait{pairs_err(ctx), ctx->pairs_wait}};
     s.off.assign(off, off + nsys + 1);
     return TBMD_OK;
 }
@@ -1418,7 +1420,10 @@ tbmd_status tbmd_adjoint(tbmd_ctx *ctx, const double *gfx, const double *gfy, co
         CK(cudaMemcpyAsync(f.data() + k * n, ctx->s[10 + k], sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(hv.data(), h, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(&e, energy_ptr(ctx), sizeof e, cudaMemcpyDeviceToHost, ctx->stream));
+    CapSeen seen{};
+    CK(read_cap_flags(ctx, ctx->stream, &seen));
     CK(cudaStreamSynchronize(ctx->stream));
+    if (seen.pairs_err) return fail(ctx, TBMD_TIMEOUT, "a wait inside the pair-tensor kernel ran out");
     const double scale = nu == 0.0 ? 0.0 : 1.0;  // with nu = 0 the true f, E and H are zero
     const double *g3[3] = {gfx, gfy, gfz};
     double *o3[3] = {gx, gy, gz};
@@ -1469,6 +1474,17 @@ tbmd_status tbmd_sync(tbmd_ctx *ctx)
 {
     if (!ctx) return TBMD_INVALID_ARG;
     CK(cudaStreamSynchronize(ctx->stream));
+    return TBMD_OK;
+}
+
+tbmd_status tbmd_probe_pair_waits(tbmd_ctx *ctx, int64_t cycles)
+{
+    if (!ctx || cycles < 0) return TBMD_INVALID_ARG;
+    tbmd_status st = check_device(ctx);
+    if (st != TBMD_OK) return st;
+    CK(ws_wait_host(ctx));
+    ctx->pairs_wait = cycles;
+    for (auto &s : ctx->pairs) s.dev.wait.limit = cycles;
     return TBMD_OK;
 }
 

@@ -364,6 +364,12 @@ struct PtPlan {
     size_t slot_bytes = 0;      // of one tile result
     bool fp64 = false;          // the FP64 form (panel steps of 8 k, row blocks of 32 particles)
 };
+// How long the kernels' waits last, and the flag that is set when one ran out.
+struct PtWait {
+    unsigned int *err;
+    long long limit;  // cycles
+};
+constexpr long long PT_WAIT_LIMIT = 4000000000ll;  // two seconds or more
 struct PtDev {
     const PtSeg *segs;
     const PtSys *sys;
@@ -372,7 +378,7 @@ struct PtDev {
     double *slots;
     unsigned char *panel2;  // adjoint: the tensors' rates
     double *slots2;         // and the tiles' results for H d
-    unsigned int *err;  // set by a launch that gave up waiting
+    PtWait wait;
 };
 void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, bool fp64, bool dual, PtPlan &plan);
 cudaError_t pt_init();

@@ -133,21 +133,26 @@ __device__ __forceinline__ bool bar_try_cluster(unsigned long long *b, unsigned 
         : "memory");
     return ok != 0;
 }
-// Every wait ends: after four billion cycles (two seconds or more) it marks the block dead and the launch failed (*err); from then on
-// waits return at once, no copy or product is issued, and the loops run out.
+// Every wait ends: after wt.limit cycles it marks the block dead and the launch failed (*wt.err); from then on
+// waits return at once, no copy or product is issued, and the loops run out.  A limit of zero gives up the first.
 template <bool CLUSTER = false, class Shared>
-__device__ __forceinline__ bool bar_wait(unsigned long long *b, unsigned int parity, Shared &S, unsigned int *err)
+__device__ __forceinline__ bool bar_wait(unsigned long long *b, unsigned int parity, Shared &S, const PtWait &wt)
 {
     auto done = [&]() { return CLUSTER ? bar_try_cluster(b, parity) : bar_try(b, parity); };
-    if (done()) return true;
+    if (wt.limit > 0 && done()) return true;
     const long long t0 = clock64();
+    if (wt.limit <= 0) {
+        *(volatile int *)&S.dead = 1;
+        atomicExch(wt.err, 1u);
+        return false;
+    }
     for (unsigned int n = 1;; ++n) {
         if (done()) return true;
         if ((n & 63u) == 0u) {
             if (*(volatile int *)&S.dead) return false;
-            if (clock64() - t0 > 4000000000ll) {
+            if (clock64() - t0 > wt.limit) {
                 *(volatile int *)&S.dead = 1;
-                atomicExch(err, 1u);
+                atomicExch(wt.err, 1u);
                 return false;
             }
         }
@@ -186,6 +191,11 @@ __device__ __forceinline__ void mma_commit(unsigned long long *b)
                      smem_u32(b)),
                  "h"((unsigned short)3)
                  : "memory");
+}
+// the same for this block's barrier alone
+__device__ __forceinline__ void mma_commit_local(unsigned long long *b)
+{
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(b)) : "memory");
 }
 // 64 columns of this warp's 32 TMEM lanes
 #define TM_LD64(v, addr)                                                                                       \
@@ -456,7 +466,7 @@ template <int MODE, bool ENERGY>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
     k_pt_gemm(Pos pos, const PtSeg *__restrict__ seg, int nseg, int64_t items, const unsigned int *__restrict__ tiles,
               const unsigned char *__restrict__ panel, const unsigned char *__restrict__ panel2,
-              double *__restrict__ slots, double *__restrict__ slots2, double nu, unsigned int *err)
+              double *__restrict__ slots, double *__restrict__ slots2, double nu, PtWait wt)
 {
     extern __shared__ __align__(1024) unsigned char smraw[];
     PtShared &S = *(PtShared *)smraw;
@@ -500,7 +510,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
                 const int64_t oa = it.s.mem + (2 * it.a + rank) * row, ob = it.s.mem + (2 * it.b + rank) * row;
                 for (int k = 0; k < slabs_of(it); ++k, ++n) {
                     const int st = n % PT_STAGES;
-                    if (!bar_wait(&S.empty[st], ((n / PT_STAGES) & 1) ^ 1, S, err)) break;
+                    if (!bar_wait(&S.empty[st], ((n / PT_STAGES) & 1) ^ 1, S, wt)) break;
                     // MODE 2: T' T, then T T'
                     const bool second = MODE == 2 && k >= it.s.nslab;
                     const int64_t ko = (int64_t)(second ? k - it.s.nslab : k) * PT_BLOCK_BYTES;
@@ -525,7 +535,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
             for (int64_t w = cluster; w < items; w += clusters) {
                 const PtItem it = pt_item(seg, nseg, tiles, w);
                 for (int k = 0; k < slabs_of(it); ++k, ++n) {
-                    if (!bar_wait(&S.full[n % PT_STAGES], (n / PT_STAGES) & 1, S, err)) break;
+                    if (!bar_wait(&S.full[n % PT_STAGES], (n / PT_STAGES) & 1, S, wt)) break;
                     bar_relay_copy(&S.full[n % PT_STAGES], 0);
                 }
                 if (*(volatile int *)&S.dead) break;
@@ -538,8 +548,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
                 const PtItem it = pt_item(seg, nseg, tiles, w);
                 for (int k = 0; k < slabs_of(it); ++k, ++n) {
                     const int st = n % PT_STAGES, buf = n & 1;
-                    ok = bar_wait(&S.acc_empty[buf], ((n >> 1) & 1) ^ 1, S, err) &&
-                         bar_wait<true>(&S.full[st], (n / PT_STAGES) & 1, S, err);
+                    ok = bar_wait(&S.acc_empty[buf], ((n >> 1) & 1) ^ 1, S, wt) &&
+                         bar_wait<true>(&S.full[st], (n / PT_STAGES) & 1, S, wt);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const unsigned int A = smem_u32(S.stage[st]), B = A + PT_BLOCK_BYTES, D = tmem + buf * 256;
@@ -556,7 +566,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
                 }
             }
             if (!ok) {  // products in flight end before the accumulators are given back
-                mma_commit(&S.drained);
+                mma_commit_local(&S.drained);
                 const long long t0 = clock64();
                 while (!bar_try(&S.drained, 0) && clock64() - t0 < 200000000ll) {
                 }
@@ -568,7 +578,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
             for (int64_t w = cluster; w < items; w += clusters, ++m) {
                 const PtItem it = pt_item(seg, nseg, tiles, w);
                 const int i0 = (2 * it.a + rank) * PT_PART, j0 = 2 * it.b * PT_PART;
-                bar_wait(&S.geo_empty, (m & 1) ^ 1, S, err);
+                bar_wait(&S.geo_empty, (m & 1) ^ 1, S, wt);
                 for (int q = (warp - 10) * 32 + lane; q < 3 * PT_PART; q += 64) {
                     const bool is_j = q < 2 * PT_PART;
                     const int64_t p = it.s.part0 + min(is_j ? j0 + q : i0 + q - 2 * PT_PART, it.s.n - 1);
@@ -603,7 +613,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
             for (int c = 0; c < 64; ++c) g2[c] = 0ull;
             for (int k = 0; k < slabs_of(it); ++k, ++n) {
                 const int buf = n & 1;
-                if (!bar_wait(&S.acc_full[buf], (n >> 1) & 1, S, err)) break;
+                if (!bar_wait(&S.acc_full[buf], (n >> 1) & 1, S, wt)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
@@ -623,7 +633,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
             // FP64 residual, t (1 + (1 - r^2 t^2) / 2): 2^-44.  Done here, in the pause of the product, since
             // the operands' reads leave shared memory no room for it while the product runs.
             const int i0 = (2 * it.a + rank) * PT_PART, j0 = 2 * it.b * PT_PART;
-            bar_wait(&S.geo_full, m & 1, S, err);
+            bar_wait(&S.geo_full, m & 1, S, wt);
             // this warp's sums for the i of its rows, for its energy, and the tile's results from all warps'
             auto store_i = [&](double x, double y, double z) {
                 S.fi[half][row][0] = x;
@@ -995,7 +1005,7 @@ __device__ __forceinline__ void tm_store12(const double *v, unsigned int addr)
 template <bool ENERGY>
 __global__ void __launch_bounds__(256, 1)
     k_p64_gemm(Pos pos, const PtSeg *__restrict__ seg, int nseg, int64_t items, const unsigned int *__restrict__ tiles,
-               const double *__restrict__ panel, double *__restrict__ slots, double nu, unsigned int *err)
+               const double *__restrict__ panel, double *__restrict__ slots, double nu, PtWait wt)
 {
     extern __shared__ __align__(1024) unsigned char smraw[];
     P64Shared &S = *(P64Shared *)smraw;
@@ -1056,7 +1066,7 @@ __global__ void __launch_bounds__(256, 1)
             const int k1 = min(k0 + P64_CHUNK, steps);
             for (int kc = k0; kc < k1; ++kc, ++n) {
                 const unsigned int st = n % P64_STAGES;
-                bar_wait(&S.full[st], (n / P64_STAGES) & 1, S, err);
+                bar_wait(&S.full[st], (n / P64_STAGES) & 1, S, wt);
                 const double2 *I = (const double2 *)S.stage[st][0] + iw * 64 + lane,
                               *J = (const double2 *)S.stage[st][1 + (jw >> 1)] + (jw & 1) * 64 + lane;
 #pragma unroll 1
@@ -1212,10 +1222,10 @@ __global__ void k_pt_reduce(int64_t p0, int64_t n, const PtSys *__restrict__ sys
 }
 
 // Energy of each system: its tiles' energies, a block per system, in a fixed order.  Adds to energy[s]
-// (the caller zeroes it).
+// (the caller zeroes it).  NaN after a launch that gave up, as the forces.
 template <int PART>
 __global__ void __launch_bounds__(512) k_pt_energy(const PtSys *__restrict__ sys, const double *__restrict__ slots,
-                                                   double *energy)
+                                                   double *energy, const unsigned int *__restrict__ err)
 {
     __shared__ double part[16];
     const PtSys s = sys[blockIdx.x];
@@ -1227,7 +1237,7 @@ __global__ void __launch_bounds__(512) k_pt_energy(const PtSys *__restrict__ sys
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int k = 1; k < 16; ++k) e += part[k];
-        energy[s.index] += e;
+        energy[s.index] = *err != 0u ? __longlong_as_double(0x7ff8000000000000ll) : energy[s.index] + e;
     }
 }
 
@@ -1397,17 +1407,17 @@ cudaError_t launch_pairs(bool dual, Pos pos, Out out, const PtPlan &plan, const 
             k_p64_panel<<<(unsigned)g.gen, P64_K * P64_PART, 0, st>>>(pos, seg, g.nsegs, (double *)d.panel);
             auto gemm = energy ? k_p64_gemm<true> : k_p64_gemm<false>;
             gemm<<<(unsigned)std::min<int64_t>(g.items, sms), 256, sizeof(P64Shared), st>>>(
-                pos, seg, g.nsegs, g.items, d.tiles, (const double *)d.panel, d.slots, nu, d.err);
-            k_pt_reduce<P64_PART><<<reduce_blocks, 256, 0, st>>>(first.part0, np, sys, g.nsys, d.slots, out, false, d.err);
-            if (energy) k_pt_energy<P64_PART><<<(unsigned)g.nsys, 512, 0, st>>>(sys, d.slots, energy);
+                pos, seg, g.nsegs, g.items, d.tiles, (const double *)d.panel, d.slots, nu, d.wait);
+            k_pt_reduce<P64_PART><<<reduce_blocks, 256, 0, st>>>(first.part0, np, sys, g.nsys, d.slots, out, false, d.wait.err);
+            if (energy) k_pt_energy<P64_PART><<<(unsigned)g.nsys, 512, 0, st>>>(sys, d.slots, energy, d.wait.err);
         } else {
             const unsigned blocks = 2 * (unsigned)std::min<int64_t>(g.items, sms / 2);
             auto gemm = [&](auto kern) {
                 kern<<<blocks, PT_WARPS * 32, sizeof(PtShared), st>>>(pos, seg, g.nsegs, g.items, d.tiles, d.panel, d.panel2,
-                                                                     d.slots, d.slots2, nu, d.err);
+                                                                     d.slots, d.slots2, nu, d.wait);
             };
             auto reduce = [&](const double *slots, Out to, bool more) {
-                k_pt_reduce<PT_PART><<<reduce_blocks, 256, 0, st>>>(first.part0, np, sys, g.nsys, slots, to, more, d.err);
+                k_pt_reduce<PT_PART><<<reduce_blocks, 256, 0, st>>>(first.part0, np, sys, g.nsys, slots, to, more, d.wait.err);
             };
             k_pt_panel<false><<<(unsigned)g.gen, PT_PANEL_THREADS, 0, st>>>(pos, seg, g.nsegs, d.panel);
             if (dual) {
@@ -1422,7 +1432,7 @@ cudaError_t launch_pairs(bool dual, Pos pos, Out out, const PtPlan &plan, const 
                 gemm(energy ? k_pt_gemm<0, true> : k_pt_gemm<0, false>);
             }
             reduce(d.slots, out, false);
-            if (energy) k_pt_energy<PT_PART><<<(unsigned)g.nsys, 512, 0, st>>>(sys, d.slots, energy);
+            if (energy) k_pt_energy<PT_PART><<<(unsigned)g.nsys, 512, 0, st>>>(sys, d.slots, energy, d.wait.err);
         }
         *launches += energy ? 4 : 3;
     }
