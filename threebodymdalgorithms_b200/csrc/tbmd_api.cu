@@ -353,8 +353,8 @@ static SweepWork single_sweep(tbmd_ctx *ctx, bool dual)
                      (const int32_t *)(t + 40), l.kseg};
 }
 
-// Whether the no-cutoff evaluation of a system (or the largest of a batch) goes through the pair-tensor
-// product (tbmd_pairs.cu) instead of a sweep: the forces of both precisions, and the mixed adjoint.  Forces:
+// Whether the no-cutoff evaluation of a system goes through the pair-tensor product (tbmd_pairs.cu) instead of a
+// sweep: the forces of both precisions, and the mixed adjoint.  Forces:
 // at n = 128 both take the same time on the device (mixed 46 and 54 us, FP64 34 and 34), from there on the
 // product is faster (n = 1000: mixed 0.21 against 0.94 ms, 8192: 69 against 240 ms for AUTA and 541 for NATA;
 // FP64 213 against 385 and 1021).  Mixed adjoint: n = 130 177 against 133 us, 300 187 against 200, 2500 6.1
@@ -363,6 +363,30 @@ constexpr int64_t kPairsMin = 128, kPairsMinAdjoint = 300, kPairsMax = 65536;
 static bool use_pairs(const tbmd_ctx *ctx, int64_t n, bool dual)
 {
     return (mixed(ctx) || !dual) && n >= (dual ? kPairsMinAdjoint : kPairsMin) && n <= kPairsMax;
+}
+
+// The same for a batch, by the two costs summed over its systems (microseconds of the whole GPU): a small system
+// pays for whole tiles of the product.  The sweep takes n ceil((n - 2) / 32) times 10.5 ns (mixed), 12.8 (FP64) or
+// 14.8 (mixed adjoint), and n^3 times 0.44, 0.9 or 1.24 ps where that is more; the product takes a time per tile and
+// one per panel step of the tile, 2.7 times that for the adjoint.  The lines lie where 2,000 equal systems take the
+// same time, at 23, 17 and 34 particles: of 8 they take 155 us of sweep and 450 of product (mixed), of 48 2,000 and 700.
+static bool use_pairs_batch(const tbmd_ctx *ctx, const int64_t *off, int nsys, bool dual)
+{
+    const bool fp64 = !mixed(ctx);
+    if ((fp64 && dual) || off[nsys] < (dual ? kPairsMinAdjoint : kPairsMin)) return false;
+    double sweep = 0.0, product = 0.0;
+    for (int s = 0; s < nsys; ++s) {
+        const int64_t n = off[s + 1] - off[s];
+        if (n > kPairsMax) return false;
+        if (n < 1) continue;
+        const double x = (double)n, tiles = fp64 ? std::ceil(x / 64) : std::ceil(x / 84);
+        if (n > 2)
+            sweep += std::max((fp64 ? 0.0128 : dual ? 0.0148 : 0.0105) * x * std::ceil((x - 2) / 32),
+                              (fp64 ? 9e-7 : dual ? 1.24e-6 : 4.4e-7) * x * x * x);
+        product += fp64 ? tiles * (tiles + 1) * (0.07 + 0.0165 * std::ceil(x / 8))
+                        : (dual ? 2.7 : 1.0) * 0.5 * tiles * (tiles + 1) * (0.19 + 0.055 * std::ceil(x / 32));
+    }
+    return product < sweep;
 }
 
 // Plan, tables and workspaces of the pair-tensor product for systems at offsets off[0 .. nsys].  The
@@ -1736,8 +1760,6 @@ static tbmd_status batch_eval(tbmd_ctx *ctx, int32_t nsys, const int64_t *offset
     const Out out{O, O + N, O + 2 * N, O + 3 * N, O + 4 * N, O + 5 * N};
     res.counts.assign(nsys, 0);
     int nl = 0;
-    int64_t nmax = 0;
-    for (int s = 0; s < nsys; ++s) nmax = std::max(nmax, offsets[s + 1] - offsets[s]);
 
     if (is_p3bca_cut(ctx)) {
         // per-system grids: the given box, or the reference's domain rule on that system's positions
@@ -1825,7 +1847,7 @@ static tbmd_status batch_eval(tbmd_ctx *ctx, int32_t nsys, const int64_t *offset
         CK(cudaMemcpyAsync(c.data(), CNT, sizeof(unsigned long long) * nsys, cudaMemcpyDeviceToHost, sm));
         CK(cudaStreamSynchronize(sm));
         for (int s = 0; s < nsys; ++s) res.counts[s] = c[s];
-    } else if ((mx || !dual) && N >= (dual ? kPairsMinAdjoint : kPairsMin) && nmax <= kPairsMax) {
+    } else if (use_pairs_batch(ctx, offsets, nsys, dual)) {
         CK(reset_cap_flags(ctx, sm));
         st = ensure_pairs(ctx, offsets, nsys, dual);
         if (st != TBMD_OK) return st;
