@@ -5,7 +5,7 @@
  * drop-in), not a tensor core or HBM figure, so the benchmark measures those pipe peaks on the
  * device it runs on with a dependent-chain-free FMA loop.
  *
- * And a handle for tests on a limit that no run reaches.
+ * And two handles for tests on limits that no run reaches.
  */
 #ifndef TBMD_PROBE_H
 #define TBMD_PROBE_H
@@ -26,6 +26,10 @@ double tbmd_probe_fma_tflops(int32_t device, int32_t fp64);
 /* Waits inside the pair-tensor kernels (no cutoff) of this context give up after `cycles` clock cycles (4e9 in a
  * new context); with 0 the first one does, and the evaluation ends with TBMD_TIMEOUT. */
 tbmd_status tbmd_probe_pair_waits(tbmd_ctx *ctx, int64_t cycles);
+
+/* A workspace of the pair-tensor product (no cutoff) that would take more than `bytes` is not to be had in this
+ * context, as if the device's memory were full; takes effect with the next sizes. */
+tbmd_status tbmd_probe_pair_workspace(tbmd_ctx *ctx, int64_t bytes);
 
 #ifdef __cplusplus
 }

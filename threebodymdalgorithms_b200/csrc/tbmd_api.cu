@@ -124,7 +124,9 @@ struct tbmd_ctx {
         PtPlan plan;
         PtDev dev{};
         DevBuf mem;  // tables, panels, tile results (one allocation: a context's first call waits for it)
+        bool no_room = false;  // the device had no memory for them: these systems are swept
     } pairs[2];
+    size_t pairs_most = SIZE_MAX;  // bytes that a workspace may take
     bool pairs_ready = false;  // pt_init has run
     long long pairs_wait = PT_WAIT_LIMIT;
     int sms = 0;
@@ -358,11 +360,17 @@ static SweepWork single_sweep(tbmd_ctx *ctx, bool dual)
 // at n = 128 both take the same time on the device (mixed 46 and 54 us, FP64 34 and 34), from there on the
 // product is faster (n = 1000: mixed 0.21 against 0.94 ms, 8192: 69 against 240 ms for AUTA and 541 for NATA;
 // FP64 213 against 385 and 1021).  Mixed adjoint: n = 130 177 against 133 us, 300 187 against 200, 2500 6.1
-// against 19.4 ms.  Above 65,536 the panel and tile results would pass 4 GB.
+// against 19.4 ms.  At 65,536 one range of k and its tile results take 3.7 GB (mixed), 5.6 GB (mixed adjoint) or
+// 5.7 GB (FP64), where the sweep takes next to nothing.
 constexpr int64_t kPairsMin = 128, kPairsMinAdjoint = 300, kPairsMax = 65536;
 static bool use_pairs(const tbmd_ctx *ctx, int64_t n, bool dual)
 {
     return (mixed(ctx) || !dual) && n >= (dual ? kPairsMinAdjoint : kPairsMin) && n <= kPairsMax;
+}
+// ... and its workspace could be had (after ensure_pairs)
+static bool on_pairs(const tbmd_ctx *ctx, int64_t n, bool dual)
+{
+    return use_pairs(ctx, n, dual) && !ctx->pairs[dual ? 1 : 0].no_room;
 }
 
 // The same for a batch, by the two costs summed over its systems (microseconds of the whole GPU): a small system
@@ -392,7 +400,7 @@ static bool use_pairs_batch(const tbmd_ctx *ctx, const int64_t *off, int nsys, b
 // Plan, tables and workspaces of the pair-tensor product for systems at offsets off[0 .. nsys].  The
 // panel and the tile results of one launch stay within 256 MB (mixed; n = 8192: 69 ms, 71 with 1 GB) or 1 GB
 // (FP64; n = 4001: 25.7 ms, 26.4 with 256 MB), or hold one range of k where that takes more; twice that
-// for the adjoint.
+// for the adjoint.  Where the device has no room for them the systems are swept, until other sizes come.
 static tbmd_status ensure_pairs(tbmd_ctx *ctx, const int64_t *off, int nsys, bool dual)
 {
     tbmd_ctx::PairState &s = ctx->pairs[dual ? 1 : 0];
@@ -400,6 +408,7 @@ static tbmd_status ensure_pairs(tbmd_ctx *ctx, const int64_t *off, int nsys, boo
         return TBMD_OK;
     CK(ws_wait_host(ctx));  // a launch on a caller's stream may still read the old tables
     s.off.clear();
+    s.no_room = false;
     if (!ctx->sms) CK(cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device));
     if (!ctx->pairs_ready) CK(pt_init());
     ctx->pairs_ready = true;
@@ -415,7 +424,14 @@ static tbmd_status ensure_pairs(tbmd_ctx *ctx, const int64_t *off, int nsys, boo
                  til = place(sizeof(unsigned int) * p.tiles.size()), tables = end, panel = place(p.mem),
                  slots = place(p.slots * p.slot_bytes), panel2 = dual ? place(p.mem) : panel,
                  slots2 = dual ? place(p.slots * p.slot_bytes) : slots;
-    CK(s.mem.ensure(end));
+    const cudaError_t room = end <= ctx->pairs_most ? s.mem.ensure(end) : cudaErrorMemoryAllocation;
+    if (room == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        s.no_room = true;
+        s.off.assign(off, off + nsys + 1);
+        return TBMD_OK;
+    }
+    CK(room);
     std::vector<char> host(tables);
     std::memcpy(host.data() + seg, p.segs.data(), sizeof(PtSeg) * p.segs.size());
     std::memcpy(host.data() + sys, p.sys.data(), sizeof(PtSys) * p.sys.size());
@@ -592,7 +608,8 @@ static tbmd_status prepare(tbmd_ctx *ctx, int64_t n, bool dual, bool energy)
     if (is_p3bca_cut(ctx)) return ensure_cells(ctx, n, dual, energy);
     if (use_pairs(ctx, n, dual)) {
         const int64_t off[2] = {0, n};
-        return ensure_pairs(ctx, off, 1, dual);
+        s = ensure_pairs(ctx, off, 1, dual);
+        if (s != TBMD_OK || on_pairs(ctx, n, dual)) return s;
     }
     const int alg = dual ? TBMD_AUTA : (ctx->cfg.algorithm == TBMD_NATA ? TBMD_NATA : TBMD_AUTA);
     const int R = dual ? (mixed(ctx) ? 2 : 1) : sweep_R(ctx);
@@ -627,7 +644,7 @@ static tbmd_status enqueue_forces(tbmd_ctx *ctx, int64_t n, Pos pos, Out out, bo
         return TBMD_OK;
     }
     phase_mark(ctx, st, PH_TRIPLETS, *nl);
-    if (use_pairs(ctx, n, dual)) {
+    if (on_pairs(ctx, n, dual)) {
         const tbmd_ctx::PairState &s = ctx->pairs[dual ? 1 : 0];
         CK(launch_pairs(dual, pos, out, s.plan, s.dev, energy, nu, ctx->sms, st, nl));
         phase_mark(ctx, st, PH_UPDATE, *nl);
@@ -736,7 +753,7 @@ static void fill_graph_key(tbmd_ctx *ctx, GraphKey &k)
         k.plan = ctx->plan;
         k.table = ctx->ncell_tab.p;
         k.max_stage = ctx->max_stage;
-    } else if (use_pairs(ctx, ctx->n, false)) {
+    } else if (on_pairs(ctx, ctx->n, false)) {
         k.pairs = ctx->pairs[0].dev;
         k.pairs_items = ctx->pairs[0].plan.groups.empty() ? 0 : ctx->pairs[0].plan.groups[0].items;
     } else {
@@ -1512,6 +1529,13 @@ tbmd_status tbmd_probe_pair_waits(tbmd_ctx *ctx, int64_t cycles)
     return TBMD_OK;
 }
 
+tbmd_status tbmd_probe_pair_workspace(tbmd_ctx *ctx, int64_t bytes)
+{
+    if (!ctx || bytes < 0) return TBMD_INVALID_ARG;
+    ctx->pairs_most = (size_t)bytes;
+    return TBMD_OK;
+}
+
 const char *tbmd_tuning(const tbmd_ctx *ctx) { return ctx ? ctx->tuning.c_str() : "{}"; }
 
 int32_t tbmd_bounds_report(int64_t *violations, int32_t *site, int64_t *index, int64_t *size)
@@ -1761,6 +1785,12 @@ static tbmd_status batch_eval(tbmd_ctx *ctx, int32_t nsys, const int64_t *offset
     res.counts.assign(nsys, 0);
     int nl = 0;
 
+    bool pairs = !is_p3bca_cut(ctx) && use_pairs_batch(ctx, offsets, nsys, dual);
+    if (pairs) {
+        st = ensure_pairs(ctx, offsets, nsys, dual);
+        if (st != TBMD_OK) return st;
+        pairs = !ctx->pairs[dual ? 1 : 0].no_room;
+    }
     if (is_p3bca_cut(ctx)) {
         // per-system grids: the given box, or the reference's domain rule on that system's positions
         std::vector<Grid> grids(nsys);
@@ -1847,10 +1877,8 @@ static tbmd_status batch_eval(tbmd_ctx *ctx, int32_t nsys, const int64_t *offset
         CK(cudaMemcpyAsync(c.data(), CNT, sizeof(unsigned long long) * nsys, cudaMemcpyDeviceToHost, sm));
         CK(cudaStreamSynchronize(sm));
         for (int s = 0; s < nsys; ++s) res.counts[s] = c[s];
-    } else if (use_pairs_batch(ctx, offsets, nsys, dual)) {
+    } else if (pairs) {
         CK(reset_cap_flags(ctx, sm));
-        st = ensure_pairs(ctx, offsets, nsys, dual);
-        if (st != TBMD_OK) return st;
         const tbmd_ctx::PairState &s = ctx->pairs[dual ? 1 : 0];
         CK(launch_pairs(dual, pos, out, s.plan, s.dev, E, nu, ctx->sms, sm, &nl));
         CapSeen seen{};
