@@ -112,11 +112,11 @@ struct tbmd_ctx {
     } sweep[2];
     DevBuf partial;
     int sweep_grid = 0;
-    // No-cutoff evaluations return without waiting, on the caller's stream: the event after the last one,
-    // and its stream.  The next one on another stream waits for it on the device (they share the work lists'
-    // counter and the workspaces), and tables are rewritten after it on the host.
+    // No-cutoff evaluations return without waiting, on the caller's stream: the event after the last one.
+    // The next one waits for it on the device (they share the work lists' counter and the workspaces), and
+    // tables are rewritten after it on the host.  Streams are not told apart by their handles, which can be
+    // those of a stream that was destroyed with work in flight, or another stream in each thread.
     cudaEvent_t ws_event = nullptr;
-    cudaStream_t ws_stream = nullptr;
     // no-cutoff evaluations as a product of pair tensors, [0] forces, [1] the mixed form's adjoint: the systems
     // the plan was made for (their particle offsets), its tables on the device, panels, tile results
     struct PairState {
@@ -280,7 +280,7 @@ static bool capturing(cudaStream_t st)
 }
 static cudaError_t ws_acquire(tbmd_ctx *ctx, cudaStream_t st)
 {
-    if (!ctx->ws_event || ctx->ws_stream == st || capturing(st)) return cudaSuccess;
+    if (!ctx->ws_event || capturing(st)) return cudaSuccess;
     return cudaStreamWaitEvent(st, ctx->ws_event, 0);
 }
 static cudaError_t ws_release(tbmd_ctx *ctx, cudaStream_t st)
@@ -290,7 +290,6 @@ static cudaError_t ws_release(tbmd_ctx *ctx, cudaStream_t st)
         const cudaError_t e = cudaEventCreateWithFlags(&ctx->ws_event, cudaEventDisableTiming);
         if (e != cudaSuccess) return e;
     }
-    ctx->ws_stream = st;
     return cudaEventRecord(ctx->ws_event, st);
 }
 static cudaError_t ws_wait_host(tbmd_ctx *ctx) { return ctx->ws_event ? cudaEventSynchronize(ctx->ws_event) : cudaSuccess; }
