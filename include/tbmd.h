@@ -77,6 +77,9 @@ void tbmd_config_init(tbmd_config *cfg);
 /* Simulation constructor + Init (Simulation.cpp:3-19). */
 tbmd_status tbmd_create(const tbmd_config *cfg, tbmd_ctx **out);
 void tbmd_destroy(tbmd_ctx *ctx);
+/* Destroyed contexts leave their no-cutoff workspaces of up to 64 MB for later ones (128 MB in all, and only while
+ * they are used again); this frees the device's. */
+tbmd_status tbmd_trim(int32_t device);
 const char *tbmd_last_error(const tbmd_ctx *ctx);
 const char *tbmd_status_string(tbmd_status s);
 int32_t tbmd_abi_version(void);

@@ -26,7 +26,7 @@ EXPORTS = ("tbmd_config_init", "tbmd_create", "tbmd_destroy", "tbmd_last_error",
            "tbmd_forces", "tbmd_adjoint", "tbmd_forces_device", "tbmd_adjoint_device", "tbmd_set_domain",
            "tbmd_cells", "tbmd_batch_forces", "tbmd_batch_adjoint", "tbmd_autotune", "tbmd_tuning", "tbmd_sync",
            "tbmd_kernel_launches", "tbmd_set_profiling", "tbmd_phase_times", "tbmd_nata_forces_noalloc",
-           "tbmd_bounds_report",
+           "tbmd_bounds_report", "tbmd_trim",
            "tbmd_generator_init", "tbmd_generate_particles", "tbmd_rank_layout_of", "tbmd_step_host")
 PHASES = ("predictor", "cells", "neighbors", "triplets", "update")
 
@@ -115,6 +115,7 @@ def load():
                                           i32]),
         "tbmd_step_host": (C.c_int, [vp, i64, pi32] + [d] * 10 + [i32, pu64, pi32] + [d] * 13),
         "tbmd_bounds_report": (i32, [pi64, pi32, pi64, pi64]),
+        "tbmd_trim": (C.c_int, [i32]),
     }
     for name, (res, args) in sig.items():
         f = getattr(lib, name)
@@ -342,6 +343,13 @@ class Context:
                                        launches.ctypes.data_as(C.POINTER(C.c_uint64)), k)
         return {PHASES[i]: {"ms": float(ms[i]), "calls": int(calls[i]), "launches": int(launches[i])}
                 for i in range(m)}
+
+
+def trim(device: int = 0):
+    """Free the workspaces that closed contexts left on the device for later ones (tbmd_trim)."""
+    st = load().tbmd_trim(int(device))
+    if st != 0:
+        raise TbmdError(st, "tbmd_trim failed")
 
 
 def rank_layout(algorithm: str, world_size: int, n: int, cutoff: float = 0.0, L=None, decomposition: str = "naive"):

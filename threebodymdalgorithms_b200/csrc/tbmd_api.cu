@@ -2,6 +2,7 @@
 // device-pointer variants.  Host code in C++; every device operation is enqueued on the context
 // stream.  Multi-step runs are captured once per configuration as a CUDA graph of one step and
 // replayed; per-step triplet counts are recorded on the device and read back once per call.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -12,6 +13,7 @@
 #include <cstddef>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <functional>
 #include <new>
 #include <string>
@@ -49,6 +51,121 @@ struct DevBuf {
     template <class T>
     T *as() const { return (T *)p; }
 };
+
+// Pair-tensor workspaces that destroyed contexts leave for later ones.  A context's first no-cutoff evaluation would
+// otherwise wait 350 us for its workspace (25 MB at n = 512 in FP64), as long as the sweep of 500 particles takes.  At most 64 MB a
+// block and 128 MB in all; a block that 16 later ones were given back without its being taken is freed, as are all when an
+// allocation fails and by tbmd_trim.  Blocks belong to a CUDA context, so those of a reset device are forgotten.
+// A block is idle when it is given: the device has been synchronised.
+class WorkspacePool {
+public:
+    // the smallest block of `bytes` to four times that, or null
+    void *take(size_t bytes, size_t *got)
+    {
+        const std::lock_guard<std::mutex> lock(m_);
+        const unsigned long long id = context_id();
+        size_t best = blocks_.size();
+        for (size_t k = 0; k < blocks_.size(); ++k)
+            if (blocks_[k].context == id && blocks_[k].bytes >= bytes && blocks_[k].bytes <= 4 * bytes &&
+                (best == blocks_.size() || blocks_[k].bytes < blocks_[best].bytes))
+                best = k;
+        if (!id || best == blocks_.size()) return nullptr;
+        void *p = blocks_[best].p;
+        *got = blocks_[best].bytes;
+        blocks_.erase(blocks_.begin() + (long)best);
+        return p;
+    }
+    void give(void *p, size_t bytes, int device)
+    {
+        if (!p) return;
+        const std::lock_guard<std::mutex> lock(m_);
+        const unsigned long long id = context_id();
+        ++given_;
+        forget(device, id);
+        size_t total = bytes;
+        for (const Block &b : blocks_) total += b.context == id ? b.bytes : 0;
+        for (size_t k = 0; k < blocks_.size();) {  // oldest first
+            if (blocks_[k].context == id && (given_ - blocks_[k].given > 16 || (bytes <= kBlock && total > kAll))) {
+                total -= blocks_[k].bytes;
+                cudaFree(blocks_[k].p);
+                blocks_.erase(blocks_.begin() + (long)k);
+            } else {
+                ++k;
+            }
+        }
+        if (!id || bytes > kBlock || cudaDeviceSynchronize() != cudaSuccess)
+            cudaFree(p);
+        else
+            blocks_.push_back(Block{p, bytes, id, device, given_});
+    }
+    bool empty()
+    {
+        const std::lock_guard<std::mutex> lock(m_);
+        return blocks_.empty();
+    }
+    // free the current device's blocks
+    bool trim(int device)
+    {
+        const std::lock_guard<std::mutex> lock(m_);
+        const unsigned long long id = context_id();
+        forget(device, id);
+        bool any = false;
+        for (size_t k = 0; k < blocks_.size();) {
+            if (blocks_[k].device == device) {
+                any = true;
+                cudaFree(blocks_[k].p);
+                blocks_.erase(blocks_.begin() + (long)k);
+            } else {
+                ++k;
+            }
+        }
+        return any;
+    }
+
+private:
+    static constexpr size_t kBlock = (size_t)64 << 20, kAll = (size_t)128 << 20;
+    struct Block {
+        void *p;
+        size_t bytes;
+        unsigned long long context;  // id of its CUDA context
+        int device;
+        unsigned long long given;
+    };
+    // blocks of an earlier CUDA context of the device went with it
+    void forget(int device, unsigned long long id)
+    {
+        for (size_t k = 0; k < blocks_.size();)
+            if (blocks_[k].device == device && blocks_[k].context != id)
+                blocks_.erase(blocks_.begin() + (long)k);
+            else
+                ++k;
+    }
+    // of the current device's CUDA context; 0 if the driver does not tell
+    static unsigned long long context_id()
+    {
+        using Get = CUresult (*)(CUcontext, unsigned long long *);
+        static const Get get = [] {
+            void *f = nullptr;
+            cudaDriverEntryPointQueryResult r = cudaDriverEntryPointSymbolNotFound;
+            if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &r) != cudaSuccess ||
+                r != cudaDriverEntryPointSuccess) {
+                cudaGetLastError();
+                f = nullptr;
+            }
+            return (Get)f;
+        }();
+        unsigned long long id = 0;
+        return get && get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+    }
+    std::mutex m_;
+    std::vector<Block> blocks_;
+    unsigned long long given_ = 0;
+};
+WorkspacePool &workspaces()
+{
+    static WorkspacePool *pool = new WorkspacePool;  // never destroyed: the driver may be gone at exit
+    return *pool;
+}
 
 // Everything that a step's launches take by value: a graph holds them as they were at its capture.
 // Zeroed before it is filled, since it is compared bytewise.
@@ -127,7 +244,7 @@ struct tbmd_ctx {
         bool no_room = false;  // the device had no memory for them: these systems are swept
     } pairs[2];
     size_t pairs_most = SIZE_MAX;  // bytes that a workspace may take
-    bool pairs_ready = false;  // pt_init has run
+    bool pairs_ready[2][2] = {};  // pt_init has run: forces or adjoint, without or with the energy
     long long pairs_wait = PT_WAIT_LIMIT;
     int sms = 0;
 
@@ -400,17 +517,18 @@ static bool use_pairs_batch(const tbmd_ctx *ctx, const int64_t *off, int nsys, b
 // panel and the tile results of one launch stay within 256 MB (mixed; n = 8192: 69 ms, 71 with 1 GB) or 1 GB
 // (FP64; n = 4001: 25.7 ms, 26.4 with 256 MB), or hold one range of k where that takes more; twice that
 // for the adjoint.  Where the device has no room for them the systems are swept, until other sizes come.
-static tbmd_status ensure_pairs(tbmd_ctx *ctx, const int64_t *off, int nsys, bool dual)
+static tbmd_status ensure_pairs(tbmd_ctx *ctx, const int64_t *off, int nsys, bool dual, bool energy)
 {
     tbmd_ctx::PairState &s = ctx->pairs[dual ? 1 : 0];
+    bool &ready = ctx->pairs_ready[dual ? 1 : 0][energy ? 1 : 0];
+    if (!ready) CK(pt_init(!mixed(ctx), dual, energy));
+    ready = true;
     if (s.off.size() == (size_t)nsys + 1 && std::memcmp(s.off.data(), off, sizeof(int64_t) * (nsys + 1)) == 0)
         return TBMD_OK;
     CK(ws_wait_host(ctx));  // a launch on a caller's stream may still read the old tables
     s.off.clear();
     s.no_room = false;
     if (!ctx->sms) CK(cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    if (!ctx->pairs_ready) CK(pt_init());
-    ctx->pairs_ready = true;
     pt_plan(off, nsys, ctx->sms, (size_t)1 << (mixed(ctx) ? 28 : 30), !mixed(ctx), dual, s.plan);
     const PtPlan &p = s.plan;
     size_t end = 0;
@@ -423,7 +541,16 @@ static tbmd_status ensure_pairs(tbmd_ctx *ctx, const int64_t *off, int nsys, boo
                  til = place(sizeof(unsigned int) * p.tiles.size()), tables = end, panel = place(p.mem),
                  slots = place(p.slots * p.slot_bytes), panel2 = dual ? place(p.mem) : panel,
                  slots2 = dual ? place(p.slots * p.slot_bytes) : slots;
-    const cudaError_t room = end <= ctx->pairs_most ? s.mem.ensure(end) : cudaErrorMemoryAllocation;
+    if (s.mem.bytes < end) {
+        workspaces().give(s.mem.p, s.mem.bytes, ctx->device);
+        s.mem.bytes = 0;
+        s.mem.p = end <= ctx->pairs_most ? workspaces().take(end, &s.mem.bytes) : nullptr;
+    }
+    cudaError_t room = end <= ctx->pairs_most ? s.mem.ensure(end) : cudaErrorMemoryAllocation;
+    if (room == cudaErrorMemoryAllocation && end <= ctx->pairs_most && workspaces().trim(ctx->device)) {
+        cudaGetLastError();
+        room = s.mem.ensure(end);
+    }
     if (room == cudaErrorMemoryAllocation) {
         cudaGetLastError();
         s.no_room = true;
@@ -607,7 +734,7 @@ static tbmd_status prepare(tbmd_ctx *ctx, int64_t n, bool dual, bool energy)
     if (is_p3bca_cut(ctx)) return ensure_cells(ctx, n, dual, energy);
     if (use_pairs(ctx, n, dual)) {
         const int64_t off[2] = {0, n};
-        s = ensure_pairs(ctx, off, 1, dual);
+        s = ensure_pairs(ctx, off, 1, dual, energy);
         if (s != TBMD_OK || on_pairs(ctx, n, dual)) return s;
     }
     const int alg = dual ? TBMD_AUTA : (ctx->cfg.algorithm == TBMD_NATA ? TBMD_NATA : TBMD_AUTA);
@@ -903,8 +1030,9 @@ void tbmd_destroy(tbmd_ctx *ctx)
     for (DevBuf *b : {&ctx->state, &ctx->snapshot, &ctx->scalars, &ctx->step_counts, &ctx->partial,
                       &ctx->cell_n, &ctx->cell_c, &ctx->nbr_buf, &ctx->dirs, &ctx->hvp, &ctx->gset_single,
                       &ctx->sweep[0].sys, &ctx->sweep[0].prefix, &ctx->sweep[1].sys, &ctx->sweep[1].prefix, &ctx->bpos, &ctx->bout, &ctx->bsys, &ctx->bprefix, &ctx->ncell_tab,
-                      &ctx->staging, &ctx->long_buf, &ctx->gen_buf, &ctx->bext, &ctx->pairs[0].mem, &ctx->pairs[1].mem})
+                      &ctx->staging, &ctx->long_buf, &ctx->gen_buf, &ctx->bext})
         b->release();
+    for (auto &s : ctx->pairs) workspaces().give(s.mem.p, s.mem.bytes, ctx->device);
     if (ctx->hpin) cudaFreeHost(ctx->hpin);
     if (ctx->copy_stream) {
         cudaStreamSynchronize(ctx->copy_stream);
@@ -915,6 +1043,16 @@ void tbmd_destroy(tbmd_ctx *ctx)
     if (ctx->ws_event) cudaEventDestroy(ctx->ws_event);
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
+}
+
+tbmd_status tbmd_trim(int32_t device)
+{
+    int prev = 0;
+    if (workspaces().empty()) return TBMD_OK;
+    if (cudaGetDevice(&prev) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) return TBMD_NO_DEVICE;
+    workspaces().trim(device);
+    cudaSetDevice(prev);
+    return TBMD_OK;
 }
 
 int64_t tbmd_num_particles(const tbmd_ctx *ctx) { return ctx ? ctx->n : 0; }
@@ -1786,7 +1924,7 @@ static tbmd_status batch_eval(tbmd_ctx *ctx, int32_t nsys, const int64_t *offset
 
     bool pairs = !is_p3bca_cut(ctx) && use_pairs_batch(ctx, offsets, nsys, dual);
     if (pairs) {
-        st = ensure_pairs(ctx, offsets, nsys, dual);
+        st = ensure_pairs(ctx, offsets, nsys, dual, true);
         if (st != TBMD_OK) return st;
         pairs = !ctx->pairs[dual ? 1 : 0].no_room;
     }

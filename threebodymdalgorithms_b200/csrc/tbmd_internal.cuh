@@ -381,7 +381,7 @@ struct PtDev {
     PtWait wait;
 };
 void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, bool fp64, bool dual, PtPlan &plan);
-cudaError_t pt_init();
+cudaError_t pt_init(bool fp64, bool dual, bool energy);
 // dual (mixed form): also H d into out.h; forces overwritten; energy (one accumulator per system, may be NULL) added to
 cudaError_t launch_pairs(bool dual, Pos pos, Out out, const PtPlan &plan, const PtDev &d, double *energy,
                          double nu, int sms, cudaStream_t st, int *launches);

@@ -1374,16 +1374,17 @@ void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, bool fp64
     }
 }
 
-cudaError_t pt_init()
+// Shared memory of the kernels of one form.  Only those that will run: setting it loads a kernel, half a
+// millisecond each in a new process.
+cudaError_t pt_init(bool fp64, bool dual, bool energy)
 {
-    cudaError_t e;
-    for (auto k : {k_pt_gemm<0, false>, k_pt_gemm<0, true>, k_pt_gemm<1, false>, k_pt_gemm<1, true>, k_pt_gemm<2, false>})
-        if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PtShared))) != cudaSuccess)
-            return e;
-    for (auto k : {k_p64_gemm<false>, k_p64_gemm<true>})
-        if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(P64Shared))) != cudaSuccess)
-            return e;
-    return cudaSuccess;
+    auto set = [](auto kern, size_t bytes) {
+        return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    };
+    if (fp64) return set(energy ? k_p64_gemm<true> : k_p64_gemm<false>, sizeof(P64Shared));
+    if (!dual) return set(energy ? k_pt_gemm<0, true> : k_pt_gemm<0, false>, sizeof(PtShared));
+    const cudaError_t e = set(energy ? k_pt_gemm<1, true> : k_pt_gemm<1, false>, sizeof(PtShared));
+    return e != cudaSuccess ? e : set(k_pt_gemm<2, false>, sizeof(PtShared));
 }
 
 // What the tensor core's truncation takes off a product on average.  A truncation loses half an ulp, which is
