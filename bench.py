@@ -283,6 +283,7 @@ def run_ours(args, world, rank, local):
         ctx.set_profiling(True)
         timed_steps(ctx, min(args.steps, 10), flush, torch, reset)
         result[prec]["phases"] = ctx.phase_times()
+        result[prec]["pairs"] = bool(load().tbmd_probe_pairs(ctx.handle))
         ctx.close()
 
     main = result[args.precision]
@@ -303,7 +304,7 @@ def run_ours(args, world, rank, local):
     peak = fp32_peak if args.precision == "mixed" else fp64_peak
     achieved = mean_trip * FLOP_PER_TRIPLET / (kern_ms * 1e-3) / 1e12
     bound, peak_source = "fp32" if args.precision == "mixed" else "fp64", "tbmd_probe_fma_tflops"
-    pairs = w["cutoff"] <= 0 and 128 <= n <= 65536  # forces as a product of pair tensors
+    pairs = main["pairs"]  # forces as a product of pair tensors
     if pairs:  # the products' own operations over i < j: six bf16 splits of 27 n^3, or twelve FP64 sums of n^3
         achieved = (162.0 if args.precision == "mixed" else 12.0) * n ** 3 / (kern_ms * 1e-3) / 1e12
         if args.precision == "mixed":

@@ -23,6 +23,10 @@ extern "C" {
  * calling thread's current device is the same afterwards. */
 double tbmd_probe_fma_tflops(int32_t device, int32_t fp64);
 
+/* 1 if the forces of the context's particles go through the pair-tensor product, 0 if they go through a sweep or
+ * the neighbour lists (after an evaluation: a workspace that was not to be had counts as the sweep). */
+int32_t tbmd_probe_pairs(const tbmd_ctx *ctx);
+
 /* Waits inside the pair-tensor kernels (no cutoff) of this context give up after `cycles` clock cycles (4e9 in a
  * new context); with 0 the first one does, and the evaluation ends with TBMD_TIMEOUT. */
 tbmd_status tbmd_probe_pair_waits(tbmd_ctx *ctx, int64_t cycles);

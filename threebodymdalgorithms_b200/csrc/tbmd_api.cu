@@ -1666,6 +1666,11 @@ tbmd_status tbmd_probe_pair_waits(tbmd_ctx *ctx, int64_t cycles)
     return TBMD_OK;
 }
 
+int32_t tbmd_probe_pairs(const tbmd_ctx *ctx)
+{
+    return ctx && !is_p3bca_cut(ctx) && on_pairs(ctx, ctx->n, false) ? 1 : 0;
+}
+
 tbmd_status tbmd_probe_pair_workspace(tbmd_ctx *ctx, int64_t bytes)
 {
     if (!ctx || bytes < 0) return TBMD_INVALID_ARG;
