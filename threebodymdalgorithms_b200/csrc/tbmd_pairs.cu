@@ -628,6 +628,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
                     for (int q = 0; q < 32; ++q) g2[c * 32 + q] = add2(g2[c * 32 + q], pack2(t[2 * q], t[2 * q + 1]));
                 }
             }
+            // G_ii has no part in the results, but T_ij of a pair closer than 4e-7 makes it infinite
+            if (it.a == it.b && half == rank) {
+                const f2 other = ip & 1 ? 0x00000000ffffffffull : 0xffffffff00000000ull;
+#pragma unroll
+                for (int p = 0; p < PT_PART / 2; ++p)
+                    if (ip >> 1 == p) {
+                        g2[3 * p] &= other;
+                        g2[3 * p + 1] &= other;
+                        g2[3 * p + 2] &= other;
+                    }
+            }
             // Geometry of the tile's pairs: n = r / |r| and r^-4, rounded once from FP64 (in FP32 their rounding
             // would count four times in the force).  1 / r is the FP32 approximation t with one step on its
             // FP64 residual, t (1 + (1 - r^2 t^2) / 2): 2^-44.  Done here, in the pause of the product, since
