@@ -1301,6 +1301,15 @@ struct CapSeen {
 };
 static_assert(sizeof(CapSeen) == 24, "scalars 28..52");
 
+// All scalars, for one copy where a call reads several.
+struct HostScalars {
+    double energy;
+    unsigned long long count;
+    uint32_t pad[3];
+    CapSeen cap;
+};
+static_assert(offsetof(HostScalars, cap) == 28, "scalars 0..52");
+
 static cudaError_t reset_cap_flags(tbmd_ctx *ctx, cudaStream_t st)
 {
     cudaError_t e = cudaMemsetAsync(ctx->scalars.as<char>() + 28, 0, 4, st);
@@ -1484,8 +1493,12 @@ static tbmd_status evaluate(tbmd_ctx *ctx, int64_t n, Pos pos, Out out, bool dua
         tbmd_status s = prepare(ctx, n, dual, energy != nullptr);
         if (s != TBMD_OK) return s;
         const bool cut = is_p3bca_cut(ctx);
-        if (!cut) CK(ws_acquire(ctx, st));
-        CK(reset_cap_flags(ctx, st));
+        if (cut) {
+            CK(reset_cap_flags(ctx, st));
+        } else {
+            CK(ws_acquire(ctx, st));
+            CK(cudaMemsetAsync(pairs_err(ctx), 0, sizeof(unsigned int), st));
+        }
         if (energy) CK(cudaMemsetAsync(energy, 0, sizeof(double), st));
         if (count) CK(cudaMemsetAsync(count, 0, sizeof(unsigned long long), st));
         int nl = 0;
@@ -1523,20 +1536,16 @@ tbmd_status tbmd_forces(tbmd_ctx *ctx, double *fx, double *fy, double *fz, doubl
     if (st != TBMD_OK) return st;
     st = evaluate(ctx, ctx->n, state_pos(ctx), state_out(ctx), false, energy_ptr(ctx), count_ptr(ctx), ctx->stream);
     if (st != TBMD_OK) return st;
-    double e = 0;
-    unsigned long long c = 0;
     const int64_t n = ctx->n;
     if (fx) CK(cudaMemcpyAsync(fx, ctx->s[10], sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
     if (fy) CK(cudaMemcpyAsync(fy, ctx->s[11], sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
     if (fz) CK(cudaMemcpyAsync(fz, ctx->s[12], sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(&e, energy_ptr(ctx), sizeof e, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(&c, count_ptr(ctx), sizeof c, cudaMemcpyDeviceToHost, ctx->stream));
-    CapSeen seen{};
-    CK(read_cap_flags(ctx, ctx->stream, &seen));
+    HostScalars seen{};
+    CK(cudaMemcpyAsync(&seen, ctx->scalars.p, sizeof seen, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    if (seen.pairs_err) return fail(ctx, TBMD_TIMEOUT, "a wait inside the pair-tensor kernel ran out");
-    if (energy) *energy = e;
-    if (triplets) *triplets = c;
+    if (seen.cap.pairs_err) return fail(ctx, TBMD_TIMEOUT, "a wait inside the pair-tensor kernel ran out");
+    if (energy) *energy = seen.energy;
+    if (triplets) *triplets = seen.count;
     return TBMD_OK;
 }
 
@@ -1593,16 +1602,14 @@ tbmd_status tbmd_adjoint(tbmd_ctx *ctx, const double *gfx, const double *gfy, co
     ctx->cfg.nu = nu;
     if (st != TBMD_OK) return st;
     std::vector<double> f(3 * n), hv(3 * n);
-    double e = 0;
     for (int k = 0; k < 3; ++k)
         CK(cudaMemcpyAsync(f.data() + k * n, ctx->s[10 + k], sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(hv.data(), h, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(&e, energy_ptr(ctx), sizeof e, cudaMemcpyDeviceToHost, ctx->stream));
-    CapSeen seen{};
-    CK(read_cap_flags(ctx, ctx->stream, &seen));
+    HostScalars seen{};
+    CK(cudaMemcpyAsync(&seen, ctx->scalars.p, sizeof seen, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    if (seen.pairs_err) return fail(ctx, TBMD_TIMEOUT, "a wait inside the pair-tensor kernel ran out");
-    const double scale = nu == 0.0 ? 0.0 : 1.0;  // with nu = 0 the true f, E and H are zero
+    if (seen.cap.pairs_err) return fail(ctx, TBMD_TIMEOUT, "a wait inside the pair-tensor kernel ran out");
+    const double e = seen.energy, scale = nu == 0.0 ? 0.0 : 1.0;  // with nu = 0 the true f, E and H are zero
     const double *g3[3] = {gfx, gfy, gfz};
     double *o3[3] = {gx, gy, gz};
     double dot = 0.0;
@@ -2020,13 +2027,9 @@ static tbmd_status batch_eval(tbmd_ctx *ctx, int32_t nsys, const int64_t *offset
         CK(cudaStreamSynchronize(sm));
         for (int s = 0; s < nsys; ++s) res.counts[s] = c[s];
     } else if (pairs) {
-        CK(reset_cap_flags(ctx, sm));
+        CK(cudaMemsetAsync(pairs_err(ctx), 0, sizeof(unsigned int), sm));
         const tbmd_ctx::PairState &s = ctx->pairs[dual ? 1 : 0];
         CK(launch_pairs(dual, pos, out, s.plan, s.dev, E, nu, ctx->sms, sm, &nl));
-        CapSeen seen{};
-        CK(read_cap_flags(ctx, sm, &seen));
-        CK(cudaStreamSynchronize(sm));
-        if (seen.pairs_err) return fail(ctx, TBMD_TIMEOUT, "a wait inside the pair-tensor kernel ran out");
         for (int s = 0; s < nsys; ++s) res.counts[s] = choose3(offsets[s + 1] - offsets[s]);
     } else {
         // one sweep over all systems (AUTA work items; NATA gives the same forces)
@@ -2073,7 +2076,10 @@ static tbmd_status batch_eval(tbmd_ctx *ctx, int32_t nsys, const int64_t *offset
     CK(cudaMemcpyAsync(res.f, O, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, sm));
     if (dual) CK(cudaMemcpyAsync(res.h, O + 3 * N, sizeof(double) * 3 * N, cudaMemcpyDeviceToHost, sm));
     CK(cudaMemcpyAsync(res.energy, E, sizeof(double) * nsys, cudaMemcpyDeviceToHost, sm));
+    CapSeen seen{};
+    if (pairs) CK(read_cap_flags(ctx, sm, &seen));
     CK(cudaStreamSynchronize(sm));
+    if (seen.pairs_err) return fail(ctx, TBMD_TIMEOUT, "a wait inside the pair-tensor kernel ran out");
     if (ctx->cfg.nu == 0.0) {  // the nu = 1 parts were evaluated; the true f, E and H vanish
         std::fill(res.f, res.f + 3 * N, 0.0);
         if (dual) std::fill(res.h, res.h + 3 * N, 0.0);
