@@ -61,3 +61,16 @@ def test_route_and_results(precision, adjoint, sizes, product):
         r = np.stack([c[a] for c in want[:3]]) if adjoint else \
             np.stack(O.forces(*np.ascontiguousarray(x[:, a]), 1.0, -1.0, nthreads=1)[:3])
         assert np.linalg.norm(got - r) <= TOL[precision] * np.linalg.norm(r)
+
+
+@pytest.mark.parametrize("precision,n,product", [("mixed", 24, False), ("mixed", 31, True), ("fp64", 17, False), ("fp64", 24, True)])
+def test_sizes_at_the_line(precision, n, product):
+    """Planning a product on the host costs a system as much as the product gains at 24 particles."""
+    off, x = batch([n] * 40)
+    ctx = Context("auta", precision)
+    count, out = launches(ctx, lambda: ctx.batch_forces(off, *x))
+    ctx.close()
+    assert (count > 2) == product
+    want = np.concatenate([np.stack(O.forces(*np.ascontiguousarray(x[:, a:a + n]), 1.0, -1.0, nthreads=1)[:3])
+                           for a in off[:-1]], 1)
+    assert np.linalg.norm(np.stack(out[:3]) - want) <= TOL[precision] * np.linalg.norm(want)

@@ -492,13 +492,15 @@ static bool on_pairs(const tbmd_ctx *ctx, int64_t n, bool dual)
 // The same for a batch, by the two costs summed over its systems (microseconds of the whole GPU): a small system
 // pays for whole tiles of the product.  The sweep takes n ceil((n - 2) / 32) times 10.5 ns (mixed), 12.8 (FP64) or
 // 14.8 (mixed adjoint), and n^3 times 0.44, 0.9 or 1.24 ps where that is more; the product takes a time per tile and
-// one per panel step of the tile, 2.7 times that for the adjoint.  The lines lie where 2,000 equal systems take the
-// same time, at 23, 17 and 34 particles: of 8 they take 155 us of sweep and 450 of product (mixed), of 48 2,000 and 700.
+// one per panel step of the tile, 2.7 times that for the adjoint, and 50 ns a system to plan it on the host when the
+// sizes are new.  The lines lie at equal systems of 28, 22 and 34 particles: 2,000 of 8 take 155 us of sweep and 450 of
+// product (mixed), of 24 a call takes 880 us with the sweep, 840 with the product and 945 with new sizes each time, and
+// of 48 2,000 us are sweep and 700 product.
 static bool use_pairs_batch(const tbmd_ctx *ctx, const int64_t *off, int nsys, bool dual)
 {
     const bool fp64 = !mixed(ctx);
     if ((fp64 && dual) || off[nsys] < (dual ? kPairsMinAdjoint : kPairsMin)) return false;
-    double sweep = 0.0, product = 0.0;
+    double sweep = 0.0, product = 0.05 * nsys;
     for (int s = 0; s < nsys; ++s) {
         const int64_t n = off[s + 1] - off[s];
         if (n > kPairsMax) return false;
