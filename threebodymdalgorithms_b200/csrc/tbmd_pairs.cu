@@ -628,17 +628,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
                     for (int q = 0; q < 32; ++q) g2[c * 32 + q] = add2(g2[c * 32 + q], pack2(t[2 * q], t[2 * q + 1]));
                 }
             }
-            // G_ii has no part in the results, but T_ij of a pair closer than 4e-7 makes it infinite
-            if (it.a == it.b && half == rank) {
-                const f2 other = ip & 1 ? 0x00000000ffffffffull : 0xffffffff00000000ull;
-#pragma unroll
-                for (int p = 0; p < PT_PART / 2; ++p)
-                    if (ip >> 1 == p) {
-                        g2[3 * p] &= other;
-                        g2[3 * p + 1] &= other;
-                        g2[3 * p + 2] &= other;
-                    }
-            }
+            // G_ii has no part in the results, but T_ij of a pair closer than 4e-7 makes it infinite: the column of the
+            // row's own particle is left out as the contraction reads it (in place, ahead of it, the sums' register
+            // pairs came apart: 265 M instructions at n = 2048 for 197 M)
+            const int self = it.a == it.b && half == rank ? ip : -1;
+            auto kept = [&](f2 g, int p) {
+                return g & ((f2)(self == 2 * p + 1 ? 0u : ~0u) << 32 | (self == 2 * p ? 0u : ~0u));
+            };
             // Geometry of the tile's pairs: n = r / |r| and r^-4, rounded once from FP64 (in FP32 their rounding
             // would count four times in the force).  1 / r is the FP32 approximation t with one step on its
             // FP64 residual, t (1 + (1 - r^2 t^2) / 2): 2^-44.  Done here, in the pause of the product, since
@@ -737,7 +733,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
                             const f2 nx = pack2(A.x, A.y), ny = pack2(A.z, A.w), nz = pack2(B.x, B.y);
                             const f2 mx = pack2(C.x, C.y), my = pack2(C.z, C.w), mz = pack2(D.x, D.y), q4 = pack2(D.z, D.w);
                             const f2 i4 = pack2(B.z * rv, B.w * rv);
-                            const f2 gx = g2[3 * p], gy = g2[3 * p + 1], gz = g2[3 * p + 2];
+                            const f2 gx = kept(g2[3 * p], p), gy = kept(g2[3 * p + 1], p), gz = kept(g2[3 * p + 2], p);
                             const f2 y = dot2(gx, gy, gz, nx, ny, nz), yd = dot2(gx, gy, gz, mx, my, mz);
                             const f2 na = al == 0 ? nx : al == 1 ? ny : nz, ga = al == 0 ? gx : al == 1 ? gy : gz,
                                      ma = al == 0 ? mx : al == 1 ? my : mz;
@@ -822,7 +818,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
                     const float4 A = S.geo[0][go + p * PT_PART], B = S.geo[1][go + p * PT_PART];
                     const f2 nx = pack2(A.x, A.y), ny = pack2(A.z, A.w), nz = pack2(B.x, B.y);
                     const f2 i4 = pack2(B.z * rv, B.w * rv);
-                    const f2 gx = g2[3 * p], gy = g2[3 * p + 1], gz = g2[3 * p + 2];
+                    const f2 gx = kept(g2[3 * p], p), gy = kept(g2[3 * p + 1], p), gz = kept(g2[3 * p + 2], p);
                     const f2 y = dot2(gx, gy, gz, nx, ny, nz);
                     const f2 na = al == 0 ? nx : al == 1 ? ny : nz, ga = al == 0 ? gx : al == 1 ? gy : gz;
                     const f2 nay = mul2(na, y), sc = fma2(m5, nay, ga);
