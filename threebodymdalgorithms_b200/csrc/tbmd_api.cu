@@ -475,7 +475,7 @@ static SweepWork single_sweep(tbmd_ctx *ctx, bool dual)
 // sweep: the forces of both precisions, and the mixed adjoint.  Forces:
 // at n = 128 both take the same time on the device (mixed 46 and 54 us, FP64 34 and 34), from there on the
 // product is faster (n = 1000: mixed 0.21 against 0.94 ms, 8192: 69 against 240 ms for AUTA and 541 for NATA;
-// FP64 213 against 385 and 1021).  Mixed adjoint: n = 130 177 against 133 us, 300 187 against 200, 2500 6.1
+// FP64 225 against 385 and 1021).  Mixed adjoint: n = 130 177 against 133 us, 300 187 against 200, 2500 6.1
 // against 19.4 ms.  At 65,536 one range of k and its tile results take 3.7 GB (mixed), 5.6 GB (mixed adjoint) or
 // 5.7 GB (FP64), where the sweep takes next to nothing.
 constexpr int64_t kPairsMin = 128, kPairsMinAdjoint = 300, kPairsMax = 65536;
@@ -517,7 +517,7 @@ static bool use_pairs_batch(const tbmd_ctx *ctx, const int64_t *off, int nsys, b
 
 // Plan, tables and workspaces of the pair-tensor product for systems at offsets off[0 .. nsys].  The
 // panel and the tile results of one launch stay within 256 MB (mixed; n = 8192: 69 ms, 71 with 1 GB) or 1 GB
-// (FP64; n = 4001: 25.7 ms, 26.4 with 256 MB), or hold one range of k where that takes more; twice that
+// (FP64; n = 4001, before its sums were folded: 25.7 ms, 26.4 with 256 MB; 27.2 now), or hold one range of k where that takes more; twice that
 // for the adjoint.  Where the device has no room for them the systems are swept, until other sizes come.
 static tbmd_status ensure_pairs(tbmd_ctx *ctx, const int64_t *off, int nsys, bool dual, bool energy)
 {
