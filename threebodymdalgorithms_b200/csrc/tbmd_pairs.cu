@@ -30,6 +30,14 @@
 // particles: 1.3e-7 .. 2.1e-7 (the FP32 sweeps: 2.2e-7 .. 2.4e-7 to 4000).  No step subtracts nearly equal
 // numbers: a pair's force needs no difference of large terms even where two of the three particles nearly
 // coincide.
+//
+// Three modules come from this source: 0 the mixed forces and the host's part, 1 the kernels of the mixed adjoint
+// (tbmd_pairs_adjoint.cu), 2 those of the FP64 form (tbmd_pairs_fp64.cu).  The first launch of a kernel in a process loads
+// its whole module, 1.24 ms for all in one, 0.44 + 0.72 and 0.36 as they are.
+#ifndef TBMD_PAIRS_MODULE
+#define TBMD_PAIRS_MODULE 0
+#endif
+
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -37,6 +45,13 @@
 #include "tbmd_internal.cuh"
 
 namespace tbmd {
+
+// One group's kernels of module 1 (T' and the second-order terms, then G') and of module 2, and their set-up.
+cudaError_t pt_init_adjoint(bool energy);
+void pt_launch_adjoint(bool second, Pos pos, const PtGroup &g, const PtDev &d, bool energy, double nu, int sms, cudaStream_t st);
+cudaError_t pt_init_fp64(bool energy);
+void pt_launch_fp64(Pos pos, Out out, const PtPlan &plan, const PtGroup &g, const PtDev &d, double *energy, double nu,
+                    int sms, cudaStream_t st);
 
 // A row block holds 42 particles in 126 of its 128 rows, two particles side by side in six rows (x x' y y'
 // z z'), so that the columns of a tile come in pairs that packed FP32 operations take at once.
@@ -907,7 +922,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT_WARPS * 32, 1)
 // Plain FMA on 2 x 4 pairs a thread, with three 16-byte reads for 8 FMA, reached 0.41 of the rate (n = 8192:
 // 477 ms).
 constexpr int P64_PART = 32, P64_K = 8, P64_F = 12, P64_STAGES = 3;
-constexpr int P64_CHUNK = 8;  // panel steps (64 k) of the matrix instruction's sums before they are folded
+[[maybe_unused]] constexpr int P64_CHUNK = 8;  // panel steps (64 k) of the matrix instruction's sums before they are folded
 constexpr int P64_BLOCK = P64_K * P64_F * P64_PART;  // doubles of one row block and 8 k: 24 KB
 constexpr int P64_SLOT = pt_slot(P64_PART);
 
@@ -941,6 +956,7 @@ struct P64Shared {
     int dead;
 };
 
+#if TBMD_PAIRS_MODULE == 2
 __global__ void __launch_bounds__(P64_K * P64_PART) k_p64_panel(Pos pos, const PtSeg *__restrict__ seg, int nseg,
                                                               double *__restrict__ panel)
 {
@@ -966,6 +982,7 @@ __global__ void __launch_bounds__(P64_K * P64_PART) k_p64_panel(Pos pos, const P
 #pragma unroll
     for (int m = 0; m < P64_F / 2; ++m) *(double2 *)(dst + m * 256) = make_double2(f[2 * m], f[2 * m + 1]);
 }
+#endif
 
 // D += A B, A 8 x 4 (lane: row lane / 4, column lane % 4), B 4 x 8 (lane: row lane % 4, column lane / 4), D 8 x 8
 // (lane: row lane / 4, columns 2 (lane % 4) and + 1)
@@ -1248,6 +1265,59 @@ __global__ void __launch_bounds__(512) k_pt_energy(const PtSys *__restrict__ sys
     }
 }
 
+template <class K>
+static cudaError_t pt_shared(K kern, size_t bytes)
+{
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+static int64_t pt_particles(const PtPlan &plan, const PtGroup &g)
+{
+    const PtSys &first = plan.sys[g.sys0], &last = plan.sys[g.sys0 + g.nsys - 1];
+    return last.part0 + last.n - first.part0;
+}
+template <int PART>
+static void pt_reduce(const PtPlan &plan, const PtGroup &g, const PtDev &d, const double *slots, Out to, bool more, cudaStream_t st)
+{
+    const int64_t np = pt_particles(plan, g);
+    k_pt_reduce<PART><<<(unsigned)((np + 7) / 8), 256, 0, st>>>(plan.sys[g.sys0].part0, np, d.sys + g.sys0, g.nsys, slots, to,
+                                                               more, d.wait.err);
+}
+template <class K>
+static void pt_gemm(K kern, Pos pos, const PtGroup &g, const PtDev &d, double nu, int sms, cudaStream_t st)
+{
+    const unsigned blocks = 2 * (unsigned)std::min<int64_t>(g.items, sms / 2);
+    kern<<<blocks, PT_WARPS * 32, sizeof(PtShared), st>>>(pos, d.segs + g.seg0, g.nsegs, g.items, d.tiles, d.panel, d.panel2,
+                                                         d.slots, d.slots2, nu, d.wait);
+}
+
+#if TBMD_PAIRS_MODULE == 1
+cudaError_t pt_init_adjoint(bool energy)
+{
+    const cudaError_t e = pt_shared(energy ? k_pt_gemm<1, true> : k_pt_gemm<1, false>, sizeof(PtShared));
+    return e != cudaSuccess ? e : pt_shared(k_pt_gemm<2, false>, sizeof(PtShared));
+}
+
+void pt_launch_adjoint(bool second, Pos pos, const PtGroup &g, const PtDev &d, bool energy, double nu, int sms, cudaStream_t st)
+{
+    if (second) return pt_gemm(k_pt_gemm<2, false>, pos, g, d, nu, sms, st);
+    k_pt_panel<true><<<(unsigned)g.gen, PT_PANEL_THREADS, 0, st>>>(pos, d.segs + g.seg0, g.nsegs, d.panel2);
+    pt_gemm(energy ? k_pt_gemm<1, true> : k_pt_gemm<1, false>, pos, g, d, nu, sms, st);
+}
+#elif TBMD_PAIRS_MODULE == 2
+cudaError_t pt_init_fp64(bool energy) { return pt_shared(energy ? k_p64_gemm<true> : k_p64_gemm<false>, sizeof(P64Shared)); }
+
+void pt_launch_fp64(Pos pos, Out out, const PtPlan &plan, const PtGroup &g, const PtDev &d, double *energy, double nu,
+                    int sms, cudaStream_t st)
+{
+    const PtSeg *seg = d.segs + g.seg0;
+    k_p64_panel<<<(unsigned)g.gen, P64_K * P64_PART, 0, st>>>(pos, seg, g.nsegs, (double *)d.panel);
+    auto gemm = energy ? k_p64_gemm<true> : k_p64_gemm<false>;
+    gemm<<<(unsigned)std::min<int64_t>(g.items, sms), 256, sizeof(P64Shared), st>>>(
+        pos, seg, g.nsegs, g.items, d.tiles, (const double *)d.panel, d.slots, nu, d.wait);
+    pt_reduce<P64_PART>(plan, g, d, d.slots, out, false, st);
+    if (energy) k_pt_energy<P64_PART><<<(unsigned)g.nsys, 512, 0, st>>>(d.sys + g.sys0, d.slots, energy, d.wait.err);
+}
+#else
 // ---------------------------------------------------------------------------------------------
 // Work lists (host)
 
@@ -1384,17 +1454,12 @@ void pt_plan(const int64_t *sys_off, int nsys, int sms, size_t budget, bool fp64
     }
 }
 
-// Shared memory of the kernels of one form.  Only those that will run: setting it loads a kernel, half a
-// millisecond each in a new process.
+// Shared memory of the kernels of one form.  Only those that will run: setting it loads a kernel.
 cudaError_t pt_init(bool fp64, bool dual, bool energy)
 {
-    auto set = [](auto kern, size_t bytes) {
-        return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    };
-    if (fp64) return set(energy ? k_p64_gemm<true> : k_p64_gemm<false>, sizeof(P64Shared));
-    if (!dual) return set(energy ? k_pt_gemm<0, true> : k_pt_gemm<0, false>, sizeof(PtShared));
-    const cudaError_t e = set(energy ? k_pt_gemm<1, true> : k_pt_gemm<1, false>, sizeof(PtShared));
-    return e != cudaSuccess ? e : set(k_pt_gemm<2, false>, sizeof(PtShared));
+    if (fp64) return pt_init_fp64(energy);
+    if (dual) return pt_init_adjoint(energy);
+    return pt_shared(energy ? k_pt_gemm<0, true> : k_pt_gemm<0, false>, sizeof(PtShared));
 }
 
 // What the tensor core's truncation takes off a product on average.  A truncation loses half an ulp, which is
@@ -1408,46 +1473,28 @@ cudaError_t launch_pairs(bool dual, Pos pos, Out out, const PtPlan &plan, const 
 {
     static_assert(sizeof(PtShared) <= 232448 && sizeof(P64Shared) <= 232448, "shared memory of one block");
     if (!plan.fp64) nu *= 1.0 + PT_TRUNCATED;
+    const Out h{out.hx, out.hy, out.hz, nullptr, nullptr, nullptr};
     for (const PtGroup &g : plan.groups) {
-        const PtSeg *seg = d.segs + g.seg0;
-        const PtSys *sys = d.sys + g.sys0;
-        const PtSys &first = plan.sys[g.sys0], &last = plan.sys[g.sys0 + g.nsys - 1];
-        const int64_t np = last.part0 + last.n - first.part0;
-        const unsigned reduce_blocks = (unsigned)((np + 7) / 8);
-        if (plan.fp64) {
-            k_p64_panel<<<(unsigned)g.gen, P64_K * P64_PART, 0, st>>>(pos, seg, g.nsegs, (double *)d.panel);
-            auto gemm = energy ? k_p64_gemm<true> : k_p64_gemm<false>;
-            gemm<<<(unsigned)std::min<int64_t>(g.items, sms), 256, sizeof(P64Shared), st>>>(
-                pos, seg, g.nsegs, g.items, d.tiles, (const double *)d.panel, d.slots, nu, d.wait);
-            k_pt_reduce<P64_PART><<<reduce_blocks, 256, 0, st>>>(first.part0, np, sys, g.nsys, d.slots, out, false, d.wait.err);
-            if (energy) k_pt_energy<P64_PART><<<(unsigned)g.nsys, 512, 0, st>>>(sys, d.slots, energy, d.wait.err);
-        } else {
-            const unsigned blocks = 2 * (unsigned)std::min<int64_t>(g.items, sms / 2);
-            auto gemm = [&](auto kern) {
-                kern<<<blocks, PT_WARPS * 32, sizeof(PtShared), st>>>(pos, seg, g.nsegs, g.items, d.tiles, d.panel, d.panel2,
-                                                                     d.slots, d.slots2, nu, d.wait);
-            };
-            auto reduce = [&](const double *slots, Out to, bool more) {
-                k_pt_reduce<PT_PART><<<reduce_blocks, 256, 0, st>>>(first.part0, np, sys, g.nsys, slots, to, more, d.wait.err);
-            };
-            k_pt_panel<false><<<(unsigned)g.gen, PT_PANEL_THREADS, 0, st>>>(pos, seg, g.nsegs, d.panel);
-            if (dual) {
-                const Out h{out.hx, out.hy, out.hz, nullptr, nullptr, nullptr};
-                k_pt_panel<true><<<(unsigned)g.gen, PT_PANEL_THREADS, 0, st>>>(pos, seg, g.nsegs, d.panel2);
-                gemm(energy ? k_pt_gemm<1, true> : k_pt_gemm<1, false>);
-                reduce(d.slots2, h, false);
-                gemm(k_pt_gemm<2, false>);
-                reduce(d.slots2, h, true);
-                *launches += 4;
-            } else {
-                gemm(energy ? k_pt_gemm<0, true> : k_pt_gemm<0, false>);
-            }
-            reduce(d.slots, out, false);
-            if (energy) k_pt_energy<PT_PART><<<(unsigned)g.nsys, 512, 0, st>>>(sys, d.slots, energy, d.wait.err);
-        }
         *launches += energy ? 4 : 3;
+        if (plan.fp64) {
+            pt_launch_fp64(pos, out, plan, g, d, energy, nu, sms, st);
+            continue;
+        }
+        k_pt_panel<false><<<(unsigned)g.gen, PT_PANEL_THREADS, 0, st>>>(pos, d.segs + g.seg0, g.nsegs, d.panel);
+        if (dual) {
+            pt_launch_adjoint(false, pos, g, d, energy != nullptr, nu, sms, st);
+            pt_reduce<PT_PART>(plan, g, d, d.slots2, h, false, st);
+            pt_launch_adjoint(true, pos, g, d, energy != nullptr, nu, sms, st);
+            pt_reduce<PT_PART>(plan, g, d, d.slots2, h, true, st);
+            *launches += 4;
+        } else {
+            pt_gemm(energy ? k_pt_gemm<0, true> : k_pt_gemm<0, false>, pos, g, d, nu, sms, st);
+        }
+        pt_reduce<PT_PART>(plan, g, d, d.slots, out, false, st);
+        if (energy) k_pt_energy<PT_PART><<<(unsigned)g.nsys, 512, 0, st>>>(d.sys + g.sys0, d.slots, energy, d.wait.err);
     }
     return cudaGetLastError();
 }
+#endif
 
 }  // namespace tbmd
