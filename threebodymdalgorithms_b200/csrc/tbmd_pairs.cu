@@ -14,7 +14,7 @@
 //                same kernel
 //   k_pt_reduce  each particle's force from its tiles, in a fixed order (deterministic)
 //
-// Bound: the tensor cores, at the power cap for large n.  n = 8192: 9.4e13 FLOP of bf16 in 69 ms, 1.36
+// Bound: the tensor cores, at the power cap for large n.  n = 8192: 9.4e13 FLOP of bf16 in 70 ms, 1.35
 // PFLOP/s, as much as cuBLAS sustains (AUTA's FP32 sweep took 240 ms, NATA's 541); n = 4096: 8.9 ms
 // (31.5 and 79).  A pair of SMs works on one tile of 256 x 256 (cta_group::2), which halves what each loads
 // of B: 48 KB a slab.  A block's 128 x 256 part is the largest whose FP32 sums fit the registers (128 a
@@ -26,10 +26,11 @@
 // exact in FP32.  The tensor core adds into an FP32 accumulator that it truncates, so an accumulator only
 // lives for 32 columns of T: the ten small products go first, the two hh steps last, and the tile is then
 // added to FP32 registers with rounding.  After 512 particles at most the registers are contracted and the
-// forces go on in FP64.  Relative L2 error of the forces against FP64, thermal lattices of 130 .. 8000
-// particles: 1.3e-7 .. 2.1e-7 (the FP32 sweeps: 2.2e-7 .. 2.4e-7 to 4000).  No step subtracts nearly equal
-// numbers: a pair's force needs no difference of large terms even where two of the three particles nearly
-// coincide.
+// forces go on in FP64.  Relative L2 errors against FP64, product and FP32 sweep on the same inputs of 200 .. 4096
+// particles: thermal lattices, forces 1.3e-7 .. 2.3e-7 (sweeps 2.0e-7 .. 2.8e-7), H d 1.5e-7 .. 2.6e-7 (3.2e-7 ..
+// 4.8e-7); uniform inputs, which hang on one or two close pairs, forces 3.8e-8 .. 4.1e-7 (3.3e-8 .. 7.8e-7), H d
+// 7.2e-8 .. 3.8e-7 (4.7e-8 .. 1.4e-6).  No step subtracts nearly equal numbers: a pair's force needs no difference of
+// large terms even where two of the three particles nearly coincide.
 //
 // Three modules come from this source: 0 the mixed forces and the host's part, 1 the kernels of the mixed adjoint
 // (tbmd_pairs_adjoint.cu), 2 those of the FP64 form (tbmd_pairs_fp64.cu).  The first launch of a kernel in a process loads
