@@ -255,7 +255,7 @@ struct tbmd_ctx {
     GridSet gset{};       // device tables of the systems being evaluated
     DevBuf gset_single;   // Grid[1] + cell_off[2] + sys_off[2] of the single-system case
     alignas(8) unsigned char gset_host[256] = {};  // host copy of what gset_single holds
-    DevBuf ncell_tab;     // neighbour-cell table of the cells being evaluated (27 runs per cell)
+    DevBuf ncell_tab;     // neighbour-cell table of the cells being evaluated (NB_RUNS runs per cell)
     int ncell_dims[3] = {0, 0, 0};  // cells per axis the single-system table was built for
     bool ncell_single = false;
     std::vector<int32_t> ncell_batch_key;  // per-system dims the batched table was built for
@@ -709,7 +709,7 @@ static tbmd_status ensure_cells(tbmd_ctx *ctx, int64_t n, bool dual, bool energy
                         (const int64_t *)(base + offsetof(decltype(tab), sys_off)), 1};
     ctx->max_stage = neighbor_stage_cap(ctx->grid, n);
     if (!ctx->ncell_single || std::memcmp(ctx->ncell_dims, ctx->grid.dims, sizeof ctx->ncell_dims) != 0) {
-        CK(ctx->ncell_tab.ensure(sizeof(int2) * 27 * (size_t)ctx->grid.ncells));
+        CK(ctx->ncell_tab.ensure(sizeof(int2) * NB_RUNS * (size_t)ctx->grid.ncells));
         CK(launch_neighbor_table(ctx->grid, ctx->gset, ctx->ncell_tab.as<int2>(), ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));  // the lists may be built on another stream
         ctx->launches += 1;
@@ -1990,7 +1990,7 @@ static tbmd_status batch_eval(tbmd_ctx *ctx, int32_t nsys, const int64_t *offset
         Grid all = grids[0];
         all.ncells = cell_off[nsys];
         if (new_table) {
-            CK(ctx->ncell_tab.ensure(sizeof(int2) * 27 * (size_t)cell_off[nsys]));
+            CK(ctx->ncell_tab.ensure(sizeof(int2) * NB_RUNS * (size_t)cell_off[nsys]));
             const GridSet gs{(const Grid *)tb, (const int64_t *)(tb + gbytes), (const int64_t *)(tb + gbytes + obytes), nsys};
             CK(launch_neighbor_table(all, gs, ctx->ncell_tab.as<int2>(), sm));
             nl += 1;

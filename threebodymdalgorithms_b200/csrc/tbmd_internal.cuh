@@ -431,7 +431,9 @@ cudaError_t launch_unsort_update(int64_t n, const CellBufs &cb, double *const st
 cudaError_t launch_neighbors(int64_t n, const Grid &g, const GridSet &set, const int2 *nbr_runs, int max_stage,
                              CellBufs &cb, cudaStream_t st);
 int neighbor_stage_cap(const Grid &g, int64_t n);
-// neighbour-cell table: 27 runs of cells per cell; depends only on the systems' cells per axis
+// Neighbour-cell table: up to NB_RUNS runs of cells per cell; depends only on the systems' cells per axis.  14 is the most
+// that any cell has, of low-face cells with at least 4 cells per axis (112 bytes a cell, where 27 cell ids took 108).
+constexpr int NB_RUNS = 14;
 cudaError_t launch_neighbor_table(const Grid &g, const GridSet &set, int2 *out, cudaStream_t st);
 // Launch shape of the P3BCA triplet kernel for a list capacity; computed outside graph capture.
 struct P3Plan {

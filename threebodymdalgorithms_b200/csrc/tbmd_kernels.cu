@@ -881,7 +881,7 @@ __global__ void __launch_bounds__(NB_THREADS, 10) k_neighbors(int64_t n, const _
         const float sq_lo = (float)G.sqcut - G.band, sq_hi = (float)G.sqcut + G.band;
         if (warp == 0) {
             // this lane's run of neighbour cells and its particles, which are consecutive
-            int2 run = lane < 27 ? nbr_runs[c * 27 + lane] : make_int2(0, 0);
+            int2 run = lane < NB_RUNS ? nbr_runs[c * NB_RUNS + lane] : make_int2(0, 0);
             if (run.x < 0) run = make_int2(0, 0);
             if (run.y > run.x) run.x = (int)TBMD_IX(run.x, g.ncells, BS_NBR_CELL);
             const int cs = cell_start[run.x], len = cell_start[run.y] - cs;
@@ -917,7 +917,7 @@ __global__ void __launch_bounds__(NB_THREADS, 10) k_neighbors(int64_t n, const _
             int k = 0;
 #pragma unroll
             for (int step = 16; step > 0; step >>= 1)
-                if (k + step < 27 && cpre[k + step] <= q) k += step;
+                if (k + step < NB_RUNS && cpre[k + step] <= q) k += step;
             return k;
         };
         // read before the barrier below: warp 0 rewrites raw_cell for its next cell once past it
@@ -1057,7 +1057,7 @@ static int neighbor_split(int64_t n, int64_t ncells, int sms)
 }
 
 // Per cell, its neighbour cells with id >= its own in increasing order, as runs of consecutive ids
-// [first, end) padded with (-1, -1) to 27: an interior cell has five (its own row and the next one, and
+// [first, end) padded with (-1, -1) to NB_RUNS: an interior cell has five (its own row and the next one, and
 // three rows of the layer above).
 __global__ void k_neighbor_table(const __grid_constant__ Grid g, GridSet set, int2 *__restrict__ out)
 {
@@ -1087,13 +1087,13 @@ __global__ void k_neighbor_table(const __grid_constant__ Grid g, GridSet set, in
                 ids[q] = (int)nc;
             }
     int r = 0;
-    for (int k = 0; k < K;) {
+    for (int k = 0; k < K && r < NB_RUNS;) {
         int e = k + 1;
         while (e < K && ids[e] == ids[e - 1] + 1) ++e;
-        out[c * 27 + r++] = make_int2((int)cell0 + ids[k], (int)cell0 + ids[e - 1] + 1);
+        out[c * NB_RUNS + r++] = make_int2((int)cell0 + ids[k], (int)cell0 + ids[e - 1] + 1);
         k = e;
     }
-    for (; r < 27; ++r) out[c * 27 + r] = make_int2(-1, -1);
+    for (; r < NB_RUNS; ++r) out[c * NB_RUNS + r] = make_int2(-1, -1);
 }
 
 cudaError_t launch_neighbor_table(const Grid &g, const GridSet &set, int2 *out, cudaStream_t st)
